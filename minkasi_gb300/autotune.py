@@ -177,7 +177,7 @@ def choose_dct_engines(op, shapes: Sequence[Tuple[int, int]]) -> Dict[Tuple[int,
     gpu = torch.cuda.get_device_name(op.device)
     out, todo = {}, []
     for s in shapes:
-        hit = _lookup(f"dct2|{gpu}|{s[0]}x{s[1]}")
+        hit = _lookup(f"dct3|{gpu}|{s[0]}x{s[1]}")
         if isinstance(hit, list) and len(hit) == 2:
             out[s] = (int(hit[0]), int(hit[1]))
         else:
@@ -204,7 +204,7 @@ def choose_dct_engines(op, shapes: Sequence[Tuple[int, int]]) -> Dict[Tuple[int,
             del plan
         best = min(times, key=times.get)
         out[s] = best
-        _store(f"dct2|{gpu}|{nd}x{n}", list(best))
+        _store(f"dct3|{gpu}|{nd}x{n}", list(best))
         del x, y
     del ws
     return out

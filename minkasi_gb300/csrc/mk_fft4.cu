@@ -135,10 +135,10 @@ bool radices(int Ls, int *r, int *nr, int rmax) {
 size_t al(size_t x) { return (x + 255) / 256 * 256; }
 
 struct TableLayout {
-  size_t stw1, stw2, iperm1, iperm2, tlane, tblk, chirp, bhat, tlane2, tblk2, total;
+  size_t stw1, stw2, iperm1, iperm2, perm1, tlane, tblk, chirp, bhat, tlane2, tblk2, total;
 };
 
-size_t csz(const Fft4Dev &d);
+size_t csz(const Fft4Dev &d) { return d.f64 ? sizeof(double2) : sizeof(float2); }
 
 TableLayout layout(const Fft4Dev &d) {
   TableLayout t;
@@ -151,12 +151,14 @@ TableLayout layout(const Fft4Dev &d) {
   o += al((size_t)d.L1 * sizeof(int));
   t.iperm2 = o;
   o += al((size_t)d.L2 * sizeof(int));
+  t.perm1 = o;
+  o += d.blue ? al((size_t)d.L1 * sizeof(int)) : 0;
   t.tlane = o;
-  o += al((size_t)d.L1 * 32 * csz(d));
+  o += al((size_t)d.H1 * 32 * csz(d));
   t.tblk = o;
-  o += al((size_t)d.L1 * d.nb32 * csz(d));
+  o += al((size_t)d.H1 * d.nb32 * csz(d));
   t.chirp = o;
-  o += d.blue ? al((size_t)(d.m + 1) * csz(d)) : 0;
+  o += d.blue ? al((size_t)(d.m + 2) * csz(d)) : 0;
   t.bhat = o;
   o += d.blue ? al((size_t)d.L * csz(d)) : 0;
   t.tlane2 = o;
@@ -185,8 +187,6 @@ void put(char *base, size_t off, int64_t i, Cd v, bool f64) {
     reinterpret_cast<float2 *>(base + off)[i] = make_float2((float)v.x, (float)v.y);
   }
 }
-
-size_t csz(const Fft4Dev &d) { return d.f64 ? sizeof(double2) : csz(d); }
 
 void digit_rev(int Ls, const int *r, int nr, int *P) {
   std::vector<int> d(nr > 0 ? nr : 1);
@@ -247,7 +247,13 @@ static bool split_len(int64_t L, Fft4Dev *t) {
   t->L2 = (int)(L / best);
   const int rmax = t->f64 ? MK_FFT4_RMAX64 : MK_FFT4_RMAX;
   if (!radices(t->L1, t->r1, &t->nr1, rmax) || !radices(t->L2, t->r2, &t->nr2, rmax)) return false;
-  t->nb32 = (t->L2 + 31) / 32;
+  t->H1 = t->L1 / 2 + 1;
+  t->H2 = t->L2 / 2 + 1;
+  t->nb32 = (t->H2 + 31) / 32;
+  t->P = (2 * t->H2 + 15) / 16 * 16;
+  t->PV = (t->L1 + 15) / 16 * 16;
+  t->tsz = (int64_t)t->H1 * t->P;
+  t->vsz = (int64_t)t->L2 * t->PV;
   for (int pass = 0; pass < 2; pass++) {
     const int nr = pass ? t->nr2 : t->nr1;
     const int *r = pass ? t->r2 : t->r1;
@@ -298,9 +304,6 @@ bool fft4_shape(int64_t n, Fft4Dev *d, bool bluestein, bool f64) {
   if (!ok) return false;
   t.fba = fb_for(t.L2, f64);
   t.fbb = fb_for(t.L1, f64);
-  // MINKASI_GB300_FFT4_BLUE3=0 makes new Bluestein plans keep the four-pass form
-  const char *e4 = getenv("MINKASI_GB300_FFT4_BLUE3");
-  t.blue4 = t.blue && e4 && std::string(e4) == "0";
   *d = t;
   return true;
 }
@@ -308,17 +311,17 @@ bool fft4_shape(int64_t n, Fft4Dev *d, bool bluestein, bool f64) {
 size_t fft4_table_bytes(const Fft4Dev &d) { return layout(d).total; }
 
 size_t fft4_t_bytes(const Fft4Dev &d, int64_t nrow) {
-  return (d.blue ? 2 : 1) * (size_t)((nrow + 1) / 2) * (size_t)d.L * csz(d);
+  return (size_t)((nrow + 1) / 2) * (size_t)(d.tsz + (d.blue ? d.vsz : 0)) * csz(d);
 }
 
-// B^ = DFT_M(b) / M with b_t = conj(c_t) at t mod M for t in [-m, 2m - 1]
-// (M >= 3m keeps those positions distinct), in double precision through a
+// B^ = DFT_M(b) / M with b_t = conj(c_t) at t mod M for t in [-m, 2m]
+// (M > 3m keeps those positions distinct), in double precision through a
 // cuFFT Z2Z transform, rounded to the plan's precision
 static int bluestein_bhat(const Fft4Dev &d, char *base, size_t off) {
   const int64_t M = d.L, Lx = d.Lx, m = d.m;
   std::vector<cufftDoubleComplex> b((size_t)M);
   for (auto &v : b) v.x = v.y = 0.0;
-  for (int64_t t = 0; t < 2 * m; t++) {
+  for (int64_t t = 0; t <= 2 * m; t++) {
     const double a = M_PI * (double)((t * t) % (2 * Lx)) / (double)Lx;  // conj(c_t) = exp(+i a)
     b[(size_t)t].x = std::cos(a);
     b[(size_t)t].y = std::sin(a);
@@ -364,9 +367,10 @@ int fft4_init(Fft4Plan *p, int64_t n, void *dev_tables, bool bluestein, bool f64
     digit_rev(d.L2, d.r2, d.nr2, P2.data());
     int *I1 = (int *)(h.data() + t.iperm1), *I2 = (int *)(h.data() + t.iperm2);
     for (int j = 0; j < d.L1; j++) I1[P1[j]] = j;
+    if (d.blue) std::copy(P1.begin(), P1.end(), (int *)(h.data() + t.perm1));
     for (int j = 0; j < d.L2; j++) I2[P2[j]] = j;
   }
-  for (int64_t j1 = 0; j1 < d.L1; j1++) {
+  for (int64_t j1 = 0; j1 < d.H1; j1++) {
     for (int l = 0; l < 32; l++) put(h.data(), t.tlane, 32 * j1 + l, unit((double)(j1 * l % d.L), (double)d.L), d.f64);
     for (int i = 0; i < d.nb32; i++)
       put(h.data(), t.tblk, j1 * d.nb32 + i, unit((double)(j1 * 32 * i % d.L), (double)d.L), d.f64);
@@ -374,6 +378,11 @@ int fft4_init(Fft4Plan *p, int64_t n, void *dev_tables, bool bluestein, bool f64
   if (d.blue) {
     for (int64_t j = 0; j <= d.m; j++)
       put(h.data(), t.chirp, j, unit((double)((j * j) % (2 * d.Lx)), 2.0 * (double)d.Lx), d.f64);
+    Cd cm = unit((double)((d.m * d.m) % (2 * d.Lx)), 2.0 * (double)d.Lx);
+    put(h.data(), t.chirp, d.m + 1, cm, d.f64);
+    cm.x *= 0.5;
+    cm.y *= 0.5;
+    put(h.data(), t.chirp, d.m, cm, d.f64);
     const int rc = bluestein_bhat(d, h.data(), t.bhat);
     if (rc) return rc;
     d.nb32b = (d.L1 + 31) / 32;
@@ -390,6 +399,7 @@ int fft4_init(Fft4Plan *p, int64_t n, void *dev_tables, bool bluestein, bool f64
   d.stw2 = (const void *)(b + t.stw2);
   d.iperm1 = (const int *)(b + t.iperm1);
   d.iperm2 = (const int *)(b + t.iperm2);
+  d.perm1 = d.blue ? (const int *)(b + t.perm1) : nullptr;
   d.tlane = (const void *)(b + t.tlane);
   d.tblk = (const void *)(b + t.tblk);
   d.chirp = d.blue ? (const void *)(b + t.chirp) : nullptr;

@@ -6,14 +6,28 @@
 // DCT(x_r)_k = Re F_k and DCT(x_{r+1})_k = Im F_k, k = 0..m.
 //
 // With L = L1 L2 (both <= FFT4_LMAX, factors in {2,3,5,7,11}), j = j1 + L1 j2
-// and k = k2 + L2 k1:
-//   pass A: for each j1, T[j1][k2] = W_L^{j1 k2} sum_j2 e_{j1 + L1 j2} W_L2^{j2 k2}
-//   pass B: for each k2, F[k2 + L2 k1] = sum_j1 T[j1][k2] W_L1^{j1 k1}
+// and k = k2 + L2 k1, a four-step FFT has
+//   pass A: for each j1, A_j1[k2] = sum_j2 e_{j1 + L1 j2} W_L2^{j2 k2}
+//   pass B: for each k2, F[k2 + L2 k1] = sum_j1 W_L^{j1 k2} A_j1[k2] W_L1^{j1 k1}
+// e and F are even, which halves both passes and what goes between them:
+//   * column L1 - j1 of e is column j1 reversed, so
+//     A_{L1-j1}[k2] = W_L2^{-k2} A_j1[L2 - k2] and
+//     W_L^{(L1-j1) k2} A_{L1-j1}[k2] = W_L^{-j1 k2} A_j1[L2 - k2]:
+//     pass A runs the H1 = L1 / 2 + 1 columns j1 <= L1 / 2 only, and stores per
+//     column and k <= L2 / 2 the two values W_L^{j1 k} A_j1[k] (entry k of row
+//     j1 of T) and W_L^{-j1 k} A_j1[L2 - k] (entry P - 1 - k), of which pass B
+//     reads one for j1 and the other for L1 - j1;
+//   * F_{L-k} = F_k, and L - (k2 + L2 k1) lies in column L2 - k2, so pass B
+//     runs the H2 = L2 / 2 + 1 columns k2 <= L2 / 2 only and writes each
+//     output to k or L - k, whichever is <= m.
+// One DCT-I of 256 x 130,978 takes 0.193 ms in FP32 and 3.06 ms in FP64 this
+// way, against 0.307 and 5.63 ms with all columns; Bluestein (below) on
+// 256 x 144,278 0.829 and 15.3 ms against 0.953 and 20.1 ms.
 // Each CTA runs 8 or 16 (FP64: 4 or 8) transforms of one pass in shared memory (mixed-radix
 // decimation in time, butterflies in place), interleaved over its threads.
 // The first stage of each pass reads its inputs straight from global memory
 // (pass A forms the even extension there); pass A's last stage twiddles its
-// outputs and stores them to T; pass B's last stage writes only k <= m
+// outputs and stores them to T; pass B's last stage writes k <= m
 // straight to the rows with the epilogue (plain, times the inverse-spectrum
 // weights, or with columns 0 and m halved).  Twiddles come from tables computed in
 // double precision on the host.
@@ -22,17 +36,18 @@
 // some) go through Bluestein's algorithm on the same passes.  With the chirp
 // c_t = exp(-i pi t^2 / 2m) (even in t), W^{jk} = c_j c_k conj(c_{k-j}) for
 // W = exp(-i pi / m), and the extension is periodic in j with period 2m, so
-//   F_k = c_k sum_{j=-m+1}^{m} (e_j c_j) conj(c_{k-j}),   e_{-j} = e_j = z_{|j|}.
-// Only k = 0..m are needed, so the lags k - j cover [-m, 2m - 1]: 3m values.
-// F is then a circular convolution a (*) b of a smooth length M >= 3m, with
-// a at positions j mod M (z_{|j|} c_{|j|}, zero elsewhere) and b_t = conj(c_t)
-// at t mod M for t in [-m, 2m - 1] (one quarter shorter than the M >= 4m - 1
-// of taking j, k over a whole period).  Pass A forms a from the rows; a
-// middle pass finishes DFT(a) column by column, multiplies by
-// B^ = DFT_M(b) / M, conjugates (U = conj(DFT(a) B^)) and runs the first
-// step of DFT(U) on the same column in shared memory; pass B on the
-// transposed shape finishes DFT(U) and writes c_k conj(DFT(U)_k) for k <= m
-// with the usual epilogue (three passes; four when L1 takes one stage).
+//   F_k = c_k sum_{j=-m}^{m} (e'_j c_j) conj(c_{k-j}),   e'_{-j} = e'_j = z_{|j|},
+// with e' halved at the two ends j = +-m (the same point of the period, split
+// between them so that e' c is even).  Only k = 0..m are needed, so the lags
+// k - j cover [-m, 2m].  F is then a circular convolution a (*) b of a smooth
+// length M > 3m, with a at positions j mod M and b_t = conj(c_t) at t mod M.
+// (M = 3m never occurs: then 2m would be smooth.)  a and DFT(a) are even, so
+// pass A and the first half of the middle pass run half of their columns as
+// above; the middle pass finishes DFT(a) for the columns k2 and L2 - k2
+// together, multiplies by B^ = DFT_M(b) / M, conjugates (U = conj(DFT(a) B^))
+// and runs the first step of DFT(U) on both columns in shared memory; pass B
+// on the transposed shape finishes DFT(U), which has no symmetry, and writes
+// c_k conj(DFT(U)_k) for k <= m with the usual epilogue.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -55,8 +70,11 @@ struct Fft4Dev {
   int64_t Lx;       // even-extension length 2m
   bool blue;        // Bluestein: L = M, chirp and bhat set
   bool f64;         // FP64 plan: tables of double2, FP64 kernels
-  bool blue4;       // Bluestein in four passes (U written out) instead of three
-  int L1, L2, nb32;  // nb32 = ceil(L2 / 32)
+  int L1, L2;
+  int H1, H2;        // L1 / 2 + 1, L2 / 2 + 1: the columns an even transform needs
+  int P, PV;         // row pitch of T (2 H2) and of V (L1), rounded up to 16
+  int64_t tsz, vsz;  // elements of T and of V per row pair
+  int nb32;          // blocks of 32 covering 0 .. L2 / 2
   int fba, fbb;      // transforms per CTA of pass A (length L2) and pass B (length L1): 8 or 16
   int nr1, nr2;
   int r1[FFT4_MAXR], r2[FFT4_MAXR];
@@ -67,9 +85,10 @@ struct Fft4Dev {
   // stage twiddles W_{Ns R}^{r k} at [to + (r - 1) Ns + k]
   const void *stw1, *stw2;
   const int *iperm1, *iperm2;  // natural index at each digit-reversed (DIT input) position
-  // four-step twiddle W_L^{j1 k2} = tblk[j1 nb32 + k2 / 32] * tlane[32 j1 + k2 % 32]
+  const int *perm1;            // Bluestein: digit-reversed position of each natural index (length L1)
+  // four-step twiddle W_L^{j1 k} = tblk[j1 nb32 + k / 32] * tlane[32 j1 + k % 32], j1 < H1, k < H2
   const void *tlane, *tblk;
-  const void *chirp;  // Bluestein: c_t, t <= m
+  const void *chirp;  // Bluestein: c_t for t < m, c_m / 2 at m, c_m at m + 1
   const void *bhat;   // Bluestein: DFT_M(b) / M
   // Bluestein's middle pass: W_M^{k2 o1} = tblk2[k2 nb32b + o1 / 32] * tlane2[32 k2 + o1 % 32]
   const void *tlane2, *tblk2;
@@ -94,7 +113,7 @@ void fft4_set_split_rank(int r);
 int fft4_split_rank();
 // bytes of the device tables for that shape
 size_t fft4_table_bytes(const Fft4Dev &d);
-// bytes of the scratch (T, and U for Bluestein) for nrow rows
+// bytes of the scratch (T, and V for Bluestein) for nrow rows
 size_t fft4_t_bytes(const Fft4Dev &d, int64_t nrow);
 // computes the tables on the host (B^ with a double-precision cuFFT
 // transform) and uploads them to `dev_tables`

@@ -15,7 +15,6 @@
 #include <cstdlib>
 #include <utility>
 
-#include "mk_async.cuh"
 #include "mk_common.cuh"
 #include "mk_fft4.cuh"
 
@@ -215,17 +214,6 @@ struct Dft<14> : DftPfa<2, 7> {};
 template <>
 struct Dft<15> : DftPfa<3, 5> {};
 
-// one-element (4 or 8 byte) asynchronous global -> shared copy; !valid
-// zero-fills (src must still be a mapped address)
-__device__ __forceinline__ void cp4(void *dst, const void *src, bool valid) {
-  if (sizeof(RT) == 4)
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(valid ? 4 : 0)
-                 : "memory");
-  else
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(valid ? 8 : 0)
-                 : "memory");
-}
-
 struct WrTable {
   C w[WRN];
 };
@@ -239,18 +227,19 @@ __device__ __forceinline__ const C *tab(const void *t) { return static_cast<cons
 // the product (checked exhaustively for all q, Ns < 2048).
 
 // ---- pass A ------------------------------------------------------------
-// A CTA runs FB transforms (FB consecutive j1) with Cfg<FB>::NT threads.  The
+// A CTA runs FB transforms (FB consecutive j1 of the H1 = L1 / 2 + 1 that the
+// evenness of the input leaves) with Cfg<FB>::NT threads.  The
 // stages interleave them over the threads (row b = bf % FB), so the first
 // stage reads its inputs straight from the detector rows (FB lanes read FB
 // consecutive samples), forming the even extension, and the middle stages
 // run in shared memory with CTA barriers.  The last stage maps the threads
 // row by row instead (32 consecutive butterflies of one row per warp): it
 // reads shared memory without conflicts (its span is the whole row), twiddles
-// its outputs k2 (natural order) by W_L^{j1 k2} and stores them straight to
-// T, one contiguous span per instruction.
-// what pass A's first stage reads: the rows' even extension (DCT), the same
-// times the Bluestein chirp (zero past 2m), or a complex sequence (U)
-enum { AM_DCT = 0, AM_BLUE = 1, AM_CPLX = 2 };
+// its outputs k2 (natural order) and stores them straight to T, one contiguous
+// span per instruction (put_t).
+// what pass A's first stage reads: the rows' even extension (DCT), or the
+// same times the Bluestein chirp (zero past m, the ends at +-m halved)
+enum { AM_DCT = 0, AM_BLUE = 1 };
 
 // threads per CTA by transforms per CTA (FB_HI on passes short enough for
 // two such CTAs per SM, FB_LO on longer ones), and the CTAs per SM the
@@ -263,23 +252,34 @@ struct Cfg {
 
 struct PassA {
   const RT *x1, *x2;
-  const C *U;  // AM_CPLX: this pair's sequence
   const C *chirp;
   bool has2;
-  int L1, j1_0, nb, m, Lx, M;
+  int L1, j1_0, nb, m, L;
   const int *iperm;
 };
 
-// input at position j: the even extension e_j (AM_DCT, j < 2m); for
-// Bluestein, z_{|i|} c_{|i|} at the position j = i mod M of i in [-m + 1, m]
-// and zero in between; or the sequence U
+// input at position j of the circle of length L: the even extension e_j; for
+// Bluestein z_{|i|} c_{|i|} at j = i mod L, |i| <= m (entry m of the chirp
+// table carries the factor 1/2 of the two ends), and zero in between
 template <int AM>
 __device__ __forceinline__ C a_input(const PassA &pa, int j) {
-  if (AM == AM_CPLX) return pa.U[j];
-  if (AM == AM_BLUE && j > pa.m && j <= pa.M - pa.m) return mkc((RT)0, (RT)0);
-  const int jj = j <= pa.m ? j : (AM == AM_BLUE ? pa.M : pa.Lx) - j;
+  if (AM == AM_BLUE && j > pa.m && j < pa.L - pa.m) return mkc((RT)0, (RT)0);
+  const int jj = j <= pa.m ? j : pa.L - j;
   const C z = mkc(__ldg(pa.x1 + jj), pa.has2 ? __ldg(pa.x2 + jj) : (RT)0);
   return AM == AM_BLUE ? cmul(z, __ldg(pa.chirp + jj)) : z;
+}
+
+// output k2 of column j1, twiddled, into its row of T: with k = min(k2, L2 - k2)
+// the entry k (k2 <= L2 / 2) holds W_L^{j1 k} A and the entry P - 1 - k
+// (k2 >= L2 / 2, and k2 = 0) holds W_L^{-j1 k} A, which are what pass B reads
+// for the rows j1 and L1 - j1 of its column k
+__device__ __forceinline__ void put_t(C *row, int k2, C v, const C *tl, const C *tb, const Fft4Dev &p) {
+  const bool neg = 2 * k2 > p.L2;
+  const int k = neg ? p.L2 - k2 : k2;
+  C w = cmul(__ldg(tb + (k >> 5)), __ldg(tl + (k & 31)));
+  if (neg) w.y = -w.y;
+  row[neg ? p.P - 1 - k : k] = cmul(v, w);
+  if (k2 == 0 || 2 * k2 == p.L2) row[p.P - 1 - k] = cmul(v, mkc(w.x, -w.y));
 }
 
 template <int R, bool FIRST, int AM, int FB>
@@ -341,8 +341,8 @@ __device__ __forceinline__ void astage_r(int R, C *sbuf, int pitch, int Ls, int 
 }
 
 // the last stage of pass A (Ns R = L2, so every butterfly has g = 0): rows
-// mapped warp by warp, outputs k2 = q + r Ns twiddled by W_L^{j1 k2} and
-// stored to this pair's T (row j1 = j1_0 + b)
+// mapped warp by warp, outputs k2 = q + r Ns twiddled and stored to this
+// pair's T (row j1 = j1_0 + b)
 template <int R, int FB>
 __device__ __forceinline__ void astage_last(const C *sbuf, int pitch, int Ns, const C *stw,
                                             const C *wr, const PassA &pa, const Fft4Dev &p,
@@ -359,12 +359,9 @@ __device__ __forceinline__ void astage_last(const C *sbuf, int pitch, int Ns, co
     Dft<R>::run(v, wr);
     const int j1 = pa.j1_0 + b;
     const C *tl = tab(p.tlane) + 32 * j1, *tb = tab(p.tblk) + j1 * p.nb32;
-    C *row = Tp + (int64_t)j1 * p.L2;
+    C *row = Tp + (int64_t)j1 * p.P;
 #pragma unroll
-    for (int r = 0; r < R; r++) {
-      const int k2 = q + r * Ns;
-      row[k2] = cmul(v[r], cmul(__ldg(tb + (k2 >> 5)), __ldg(tl + (k2 & 31))));
-    }
+    for (int r = 0; r < R; r++) put_t(row, q + r * Ns, v[r], tl, tb, p);
   }
 }
 
@@ -401,30 +398,27 @@ __device__ __forceinline__ void astage_last_r(int R, const C *sbuf, int pitch, i
 // rows fall in distinct shared-memory banks
 __host__ __device__ __forceinline__ int pitch_odd(int Ls) { return Ls | 1; }
 
-// pass A: rows (2 pair, 2 pair + 1) of x (or the pair's U) -> T[pair]
-// (L1 x L2, twiddled)
+// pass A: rows (2 pair, 2 pair + 1) of x -> T[pair] (H1 x P, twiddled)
 template <int AM, int FB>
 __global__ void __launch_bounds__(Cfg<FB>::NT, Cfg<FB>::MINB) k_fft4_a(const RT *__restrict__ x, int64_t ldx,
-                                                    const C *__restrict__ U, int64_t nrow,
-                                                    C *__restrict__ T, const Fft4Dev p, const WrTable wt) {
+                                                    int64_t nrow, C *__restrict__ T, const Fft4Dev p,
+                                                    const WrTable wt) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C *const sbuf = reinterpret_cast<C *>(smem_raw);
   const int L1 = p.L1, L2 = p.L2, pitch = pitch_odd(L2), tid = threadIdx.x;
   const int64_t pair = blockIdx.y, r0 = 2 * pair;
   PassA pa;
   pa.has2 = r0 + 1 < nrow;
-  pa.x1 = AM == AM_CPLX ? nullptr : x + r0 * ldx;
-  pa.x2 = AM == AM_CPLX ? nullptr : pa.has2 ? pa.x1 + ldx : pa.x1;
-  pa.U = AM == AM_CPLX ? U + pair * p.L : nullptr;
+  pa.x1 = x + r0 * ldx;
+  pa.x2 = pa.has2 ? pa.x1 + ldx : pa.x1;
   pa.chirp = tab(p.chirp);
   pa.L1 = L1;
   pa.j1_0 = blockIdx.x * FB;
-  pa.nb = min(FB, L1 - pa.j1_0);
+  pa.nb = min(FB, p.H1 - pa.j1_0);
   pa.m = (int)p.m;
-  pa.Lx = (int)p.Lx;
-  pa.M = (int)p.L;
+  pa.L = (int)p.L;
   pa.iperm = p.iperm2;
-  C *Tp = T + pair * p.L;
+  C *Tp = T + pair * p.tsz;
   const int S = p.nr2;
   if (S >= 2) {
     astage_r<true, AM, FB>(p.r2[0], sbuf, pitch, L2, 1, 1.0f, tab(p.stw2), wt.w, pa);
@@ -437,7 +431,7 @@ __global__ void __launch_bounds__(Cfg<FB>::NT, Cfg<FB>::MINB) k_fft4_a(const RT 
     return;
   }
   // one stage at most (L2 <= 16): into shared memory, then each warp
-  // twiddles rows b by W_L^{j1 k2} and stores them
+  // twiddles and stores rows b
   if (S == 0) {  // L2 == 1: the column is its own transform
     if (tid < pa.nb) sbuf[tid * pitch] = a_input<AM>(pa, pa.j1_0 + tid);
   } else {
@@ -446,41 +440,45 @@ __global__ void __launch_bounds__(Cfg<FB>::NT, Cfg<FB>::MINB) k_fft4_a(const RT 
   __syncthreads();
   const int lane = tid & 31;
   for (int b = tid >> 5; b < pa.nb; b += Cfg<FB>::NT / 32) {
-    const C *row = sbuf + b * pitch;
     const int j1 = pa.j1_0 + b;
-    const C tl = __ldg(tab(p.tlane) + 32 * j1 + lane);
-    const C *tb = tab(p.tblk) + j1 * p.nb32;
-    for (int i = 0; i < p.nb32; i++) {
-      const int k2 = 32 * i + lane;
-      if (k2 < L2) Tp[(int64_t)j1 * L2 + k2] = cmul(row[k2], cmul(__ldg(tb + i), tl));
-    }
+    if (lane < L2)
+      put_t(Tp + (int64_t)j1 * p.P, lane, sbuf[b * pitch + lane], tab(p.tlane) + 32 * j1, tab(p.tblk) + j1 * p.nb32,
+            p);
   }
 }
 
 // ---- pass B ------------------------------------------------------------
-// The CTA's FB transforms (FB consecutive k2) are interleaved over its
+// The CTA's FB transforms (FB consecutive columns) are interleaved over its
 // Cfg<FB>::NT threads: butterfly bf of a stage belongs to row b = bf % FB, so the
 // FB lanes of a row group read or write FB consecutive columns of T / of the
 // output.  The first stage reads its inputs straight from T (natural order:
 // position g R0 + r of the digit-reversed layout holds index
 // iperm[g R0] + (L1 / R0) r), and the last stage writes its outputs straight
 // to the DCT rows with the epilogue.
-// what pass B's last stage writes: DCT rows (k <= m, epilogue), the
-// Bluestein product U = conj(F B^) (all k), or the Bluestein result
-// c_k conj(F_k) as DCT rows
-enum { BM_DCT = 0, BM_MUL = 1, BM_BLUE = 2 };
+// BM_DCT: the H2 columns k2 <= L2 / 2 of the even transform.  Input j1 is
+// T[j1][k2] for j1 <= L1 / 2 and the entry P - 1 - k2 of row L1 - j1 beyond
+// it; output kk = k2 + L2 k1 is the DCT's value kk, or L - kk when kk > m (the
+// column L2 - k2, which is not computed).
+// BM_BLUE: every column of V; output kk <= m is c_kk conj(F_kk).
+enum { BM_DCT = 0, BM_BLUE = 1 };
 
 struct PassB {
-  const C *Tp;  // this pair's T (L1 x L2)
-  C *U;         // BM_MUL: this pair's output sequence
-  const C *bhat, *chirp;
-  int L2, k2_0, nb, m, epi;
+  const C *Tp;  // this pair's T or V
+  const C *chirp;
+  int L1, L2, L, P, k2_0, nb, m, epi;
   bool has2;
   RT *o1, *o2;
-  const RT *sw;        // prefetched weights, [k1][b][row], or null
-  const RT *w1, *w2;      // else the weight rows, read in the last stage
+  const RT *w1, *w2;      // the weight rows, read in the last stage
   const int *iperm;
 };
+
+// element j1 of column k2
+template <int BM>
+__device__ __forceinline__ C b_input(const PassB &pb, int j1, int k2) {
+  if (BM == BM_BLUE) return pb.Tp[j1 * pb.P + k2];
+  const bool mir = 2 * j1 > pb.L1;
+  return pb.Tp[mir ? (pb.L1 - j1 + 1) * pb.P - 1 - k2 : j1 * pb.P + k2];
+}
 
 template <int R, bool FIRST, bool LAST, int BM, int FB>
 __device__ __forceinline__ void bstage(C *sbuf, int pitch, int Ls, int Ns, float invNs, const C *stw,
@@ -495,7 +493,7 @@ __device__ __forceinline__ void bstage(C *sbuf, int pitch, int Ls, int Ns, float
     if (FIRST) {  // Ns == 1: g == q, k == 0
       const int jg = __ldg(pb.iperm + q * R);
 #pragma unroll
-      for (int r = 0; r < R; r++) v[r] = pb.Tp[(jg + (Ls / R) * r) * pb.L2 + pb.k2_0 + b];
+      for (int r = 0; r < R; r++) v[r] = b_input<BM>(pb, jg + (Ls / R) * r, pb.k2_0 + b);
     } else {
       const C *a = sbuf + b * pitch + g * Ns * R + k;
 #pragma unroll
@@ -509,24 +507,18 @@ __device__ __forceinline__ void bstage(C *sbuf, int pitch, int Ls, int Ns, float
     if (LAST) {
 #pragma unroll
       for (int r = 0; r < R; r++) {
-        const int k1 = g * Ns * R + k + r * Ns;
-        const int kk = pb.k2_0 + b + pb.L2 * k1;
-        if (BM == BM_MUL) {
-          const C f = cmul(v[r], __ldg(pb.bhat + kk));
-          pb.U[kk] = mkc(f.x, -f.y);
-          continue;
+        const int k2 = pb.k2_0 + b;
+        int kk = k2 + pb.L2 * (g * Ns * R + k + r * Ns);
+        if (kk > pb.m) {
+          // the self-mirrored columns hold both values of a pair
+          if (BM == BM_BLUE || k2 == 0 || 2 * k2 == pb.L2) continue;
+          kk = pb.L - kk;
         }
-        if (kk > pb.m) continue;
-        if (BM == BM_BLUE) v[r] = cmul(mkc(v[r].x, -v[r].y), __ldg(pb.chirp + kk));
+        if (BM == BM_BLUE) v[r] = cmul(mkc(v[r].x, -v[r].y), __ldg(pb.chirp + (kk == pb.m ? kk + 1 : kk)));
         RT a = v[r].x, c = v[r].y;
         if (pb.epi == FFT4_FILTER) {
-          if (pb.sw) {
-            a *= pb.sw[2 * (k1 * FB + b)];
-            c *= pb.sw[2 * (k1 * FB + b) + 1];
-          } else {
-            a *= __ldg(pb.w1 + kk);
-            if (pb.has2) c *= __ldg(pb.w2 + kk);
-          }
+          a *= __ldg(pb.w1 + kk);
+          if (pb.has2) c *= __ldg(pb.w2 + kk);
         } else if (pb.epi == FFT4_HALVE && (kk == 0 || kk == pb.m)) {
           a *= (RT)0.5;
           c *= (RT)0.5;
@@ -571,57 +563,38 @@ __device__ __forceinline__ void bstage_r(int R, C *sbuf, int pitch, int Ls, int 
   }
 }
 
-// pass B: T[pair] -> DCT rows 2 pair, 2 pair + 1 of out (k <= m) with the
-// epilogue, or (BM_MUL) -> the pair's U
+// pass B: T[pair] (BM_DCT) or V[pair] (BM_BLUE) -> DCT rows 2 pair, 2 pair + 1
+// of out (k <= m) with the epilogue
 template <int BM, int FB>
 __global__ void __launch_bounds__(Cfg<FB>::NT, Cfg<FB>::MINB) k_fft4_b(const C *__restrict__ T, int64_t nrow,
-                                                    RT *__restrict__ out, int64_t ldo, C *__restrict__ U,
-                                                    const RT *__restrict__ w, int64_t ldw, int epi,
-                                                    int wpre, const Fft4Dev p, const WrTable wt) {
+                                                    RT *__restrict__ out, int64_t ldo, const RT *__restrict__ w,
+                                                    int64_t ldw, int epi, const Fft4Dev p, const WrTable wt) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C *const sbuf = reinterpret_cast<C *>(smem_raw);
-  const int L1 = p.L1, L2 = p.L2, pitch = pitch_odd(L1), tid = threadIdx.x;
+  const int L1 = p.L1, L2 = p.L2, pitch = pitch_odd(L1);
   const int64_t pair = blockIdx.y, r0 = 2 * pair;
   PassB pb;
   pb.has2 = r0 + 1 < nrow;
   pb.k2_0 = blockIdx.x * FB;
-  pb.nb = min(FB, L2 - pb.k2_0);
-  pb.Tp = T + pair * p.L;
-  pb.U = BM == BM_MUL ? U + pair * p.L : nullptr;
-  pb.bhat = tab(p.bhat);
+  pb.nb = min(FB, (BM == BM_DCT ? p.H2 : L2) - pb.k2_0);
+  pb.Tp = T + pair * (BM == BM_DCT ? p.tsz : p.vsz);
   pb.chirp = tab(p.chirp);
+  pb.L1 = L1;
   pb.L2 = L2;
+  pb.L = (int)p.L;
+  pb.P = BM == BM_DCT ? p.P : p.PV;
   pb.m = (int)p.m;
   pb.epi = epi;
-  pb.o1 = BM == BM_MUL ? nullptr : out + r0 * ldo;
-  pb.o2 = BM == BM_MUL ? nullptr : pb.o1 + ldo;
+  pb.o1 = out + r0 * ldo;
+  pb.o2 = pb.o1 + ldo;
   pb.iperm = p.iperm1;
-  pb.sw = nullptr;
   pb.w1 = pb.w2 = nullptr;
-  if (BM != BM_MUL && epi == FFT4_FILTER) {
-    const RT *w1 = w + r0 * ldw;
-    const RT *w2 = pb.has2 ? w1 + ldw : w1;
-    pb.w1 = w1;
-    pb.w2 = w2;
-    if (wpre) {
-      // the weights of this tile's outputs, [k1][b][row], prefetched during
-      // the first stages (when two CTAs still fit an SM with them)
-      RT *sw = reinterpret_cast<RT *>(sbuf + FB * pitch);
-      pb.sw = sw;
-#pragma unroll 4
-      for (int idx = tid; idx < FB * L1; idx += Cfg<FB>::NT) {
-        const int b = idx % FB, k1 = idx / FB;
-        const int k = pb.k2_0 + b + L2 * k1;
-        const bool ok = b < pb.nb && k <= pb.m;
-        cp4(sw + 2 * idx, ok ? w1 + k : w1, ok);
-        cp4(sw + 2 * idx + 1, ok ? w2 + k : w1, ok && pb.has2);
-      }
-    }
+  if (epi == FFT4_FILTER) {
+    pb.w1 = w + r0 * ldw;
+    pb.w2 = pb.has2 ? pb.w1 + ldw : pb.w1;
   }
   const int S = p.nr1;
   if (S == 1) {
-    cp_async_wait_all();
-    __syncthreads();
     bstage_r<true, true, BM, FB>(p.r1[0], sbuf, pitch, L1, 1, 1.0f, tab(p.stw1), wt.w, pb);
     return;
   }
@@ -631,8 +604,6 @@ __global__ void __launch_bounds__(Cfg<FB>::NT, Cfg<FB>::MINB) k_fft4_b(const C *
     bstage_r<false, false, BM, FB>(p.r1[s], sbuf, pitch, L1, p.ns1[s], p.inv1[s], tab(p.stw1) + p.to1[s], wt.w, pb);
     __syncthreads();
   }
-  cp_async_wait_all();
-  __syncthreads();
   bstage_r<false, true, BM, FB>(p.r1[S - 1], sbuf, pitch, L1, p.ns1[S - 1], p.inv1[S - 1],
                                 tab(p.stw1) + p.to1[S - 1], wt.w, pb);
 }
@@ -653,24 +624,47 @@ __global__ void __launch_bounds__(Cfg<FB>::NT, Cfg<FB>::MINB) k_fft4_b(const C *
 // product in between.  The last stage stores V[k2][o1] = W_M^{k2 o1} (.)
 // row by row (o1 contiguous), and pass B over the transposed shape (length
 // L2 over i2 -> o2, rows o1) finishes with the chirp and the epilogue.
+//
+// a is even, so DFT(a) is even: F[(L2 - k2) + L2 (L1 - 1 - k1)] = F[k2 + L2 k1],
+// and one first-transform column serves both columns k2 and L2 - k2 of the
+// second transform (B^ is not even, so that one needs them all).  A CTA takes
+// FB / 2 column pairs: the first transform runs on slots 0 .. FB / 2 - 1, the
+// shared butterfly pass writes column k2 back into its slot and column
+// L2 - k2 into slot FB / 2 + b, and the second transform runs on all slots.
 struct PassC {
-  const C *Tp;  // this pair's T (L1 x L2)
-  C *Vp;        // this pair's V (L2 x L1)
+  const C *Tp;  // this pair's T
+  C *Vp;        // this pair's V (L2 x PV)
   const C *bhat;
-  int L1, L2, k2_0, nb;
+  int L1, L2, P, PV, k2_0, nh;  // nh: column pairs of this CTA
 };
+
+// the column in slot b (pairs' first columns, then their partners), or -1
+template <int FB>
+__device__ __forceinline__ int c_col(const PassC &pc, int b) {
+  constexpr int H = FB / 2;
+  if (b < H) return b < pc.nh ? pc.k2_0 + b : -1;
+  const int k2 = pc.k2_0 + b - H;
+  return b - H < pc.nh && k2 != 0 && 2 * k2 != pc.L2 ? pc.L2 - k2 : -1;
+}
+
+// element j1 of column k2 <= L2 / 2 of T (as pass B's BM_DCT input)
+__device__ __forceinline__ C c_input(const PassC &pc, int j1, int k2) {
+  const bool mir = 2 * j1 > pc.L1;
+  return pc.Tp[mir ? (pc.L1 - j1 + 1) * pc.P - 1 - k2 : j1 * pc.P + k2];
+}
 
 // the first decimation-in-frequency stage (span Ns = L1 / R): natural-order
 // inputs k + r Ns from T's column, butterfly, twiddle after it
 template <int R, int FB>
 __device__ __forceinline__ void cstage_first(C *sbuf, int pitch, int Ns, const C *stw, const C *wr,
                                              const PassC &pc) {
-  for (int bf = threadIdx.x; bf < FB * Ns; bf += Cfg<FB>::NT) {
-    const int b = bf % FB, q = bf / FB;
-    if (b >= pc.nb) continue;
+  constexpr int H = FB / 2;
+  for (int bf = threadIdx.x; bf < H * Ns; bf += Cfg<FB>::NT) {
+    const int b = bf % H, q = bf / H;
+    if (b >= pc.nh) continue;
     C v[R];
 #pragma unroll
-    for (int r = 0; r < R; r++) v[r] = pc.Tp[(int64_t)(q + r * Ns) * pc.L2 + pc.k2_0 + b];
+    for (int r = 0; r < R; r++) v[r] = c_input(pc, q + r * Ns, pc.k2_0 + b);
     Dft<R>::run(v, wr);
 #pragma unroll
     for (int r = 1; r < R; r++) v[r] = cmul(v[r], __ldg(stw + (r - 1) * Ns + q));
@@ -684,11 +678,12 @@ __device__ __forceinline__ void cstage_first(C *sbuf, int pitch, int Ns, const C
 // butterfly), same butterfly indexing as the decimation-in-time stages
 template <int R, int FB>
 __device__ __forceinline__ void cstage_dif(C *sbuf, int pitch, int Ls, int Ns, float invNs, const C *stw,
-                                           const C *wr, int nb) {
+                                           const C *wr, int nh) {
+  constexpr int H = FB / 2;
   const int nq = Ls / R;
-  for (int bf = threadIdx.x; bf < FB * nq; bf += Cfg<FB>::NT) {
-    const int b = bf % FB, q = bf / FB;
-    if (b >= nb) continue;
+  for (int bf = threadIdx.x; bf < H * nq; bf += Cfg<FB>::NT) {
+    const int b = bf % H, q = bf / H;
+    if (b >= nh) continue;
     const int g = __float2int_rz(((float)q + 0.5f) * invNs);
     const int k = q - g * Ns;
     C *a = sbuf + b * pitch + g * Ns * R + k;
@@ -704,24 +699,47 @@ __device__ __forceinline__ void cstage_dif(C *sbuf, int pitch, int Ls, int Ns, f
 }
 
 // stage 0 of both transforms: the last DIF butterflies give F at k1 =
-// iperm[q R] + (L1 / R) r; U = conj(F B^) there; then the first DIT
-// butterflies of the second transform on the same R values
-template <int R, int FB>
-__device__ __forceinline__ void cstage_mid(C *sbuf, int pitch, int L1, const int *iperm, const C *wr,
-                                           const PassC &pc) {
+// iperm[q R] + (L1 / R) r; U = conj(F B^) there, for the column and, with k1
+// mirrored to L1 - 1 - k1 (another butterfly, its legs reversed), for its
+// partner; then the first DIT butterflies of the second transform on each.
+// F goes through shared memory in between, so that one set of R values is
+// live at a time.  LOAD (one-stage passes): the inputs come straight from T.
+template <int R, int FB, bool LOAD>
+__device__ __forceinline__ void cstage_mid(C *sbuf, int pitch, int L1, const int *iperm, const int *perm,
+                                           const C *wr, const PassC &pc) {
+  constexpr int H = FB / 2;
   const int nq = L1 / R;
-  for (int bf = threadIdx.x; bf < FB * nq; bf += Cfg<FB>::NT) {
-    const int b = bf % FB, q = bf / FB;
-    if (b >= pc.nb) continue;
+  for (int bf = threadIdx.x; bf < H * nq; bf += Cfg<FB>::NT) {
+    const int b = bf % H, q = bf / H;
+    if (b >= pc.nh) continue;
+    const int k2 = pc.k2_0 + b;
+    const int kq = __ldg(iperm + q * R);
     C *a = sbuf + b * pitch + q * R;
     C v[R];
 #pragma unroll
-    for (int r = 0; r < R; r++) v[r] = a[r];
+    for (int r = 0; r < R; r++) v[r] = LOAD ? c_input(pc, r, k2) : a[r];
     Dft<R>::run(v, wr);
-    const int k1 = __ldg(iperm + q * R);
+    const int kp = c_col<FB>(pc, H + b);
+    if (kp >= 0) {
+#pragma unroll
+      for (int r = 0; r < R; r++) a[r] = v[r];
+      C u[R];
+#pragma unroll
+      for (int r = 0; r < R; r++) {
+        const C f = cmul(v[r], __ldg(pc.bhat + kp + (int64_t)pc.L2 * (L1 - 1 - kq - nq * r)));
+        u[R - 1 - r] = mkc(f.x, -f.y);
+      }
+      Dft<R>::run(u, wr);
+      C *ap = sbuf + (H + b) * pitch + __ldg(perm + (nq - 1 - kq));
+#pragma unroll
+      for (int r = 0; r < R; r++) ap[r] = u[r];
+      asm volatile("" ::: "memory");
+#pragma unroll
+      for (int r = 0; r < R; r++) v[r] = a[r];
+    }
 #pragma unroll
     for (int r = 0; r < R; r++) {
-      const C f = cmul(v[r], __ldg(pc.bhat + pc.k2_0 + b + (int64_t)pc.L2 * (k1 + (L1 / R) * r)));
+      const C f = cmul(v[r], __ldg(pc.bhat + k2 + (int64_t)pc.L2 * (kq + nq * r)));
       v[r] = mkc(f.x, -f.y);
     }
     Dft<R>::run(v, wr);
@@ -731,13 +749,14 @@ __device__ __forceinline__ void cstage_mid(C *sbuf, int pitch, int L1, const int
 }
 
 // a decimation-in-time stage in shared memory (twiddles before the butterfly)
+// on all slots
 template <int R, int FB>
 __device__ __forceinline__ void cstage_dit(C *sbuf, int pitch, int Ls, int Ns, float invNs, const C *stw,
-                                           const C *wr, int nb) {
+                                           const C *wr, const PassC &pc) {
   const int nq = Ls / R;
   for (int bf = threadIdx.x; bf < FB * nq; bf += Cfg<FB>::NT) {
     const int b = bf % FB, q = bf / FB;
-    if (b >= nb) continue;
+    if (c_col<FB>(pc, b) < 0) continue;
     const int g = __float2int_rz(((float)q + 0.5f) * invNs);
     const int k = q - g * Ns;
     C *a = sbuf + b * pitch + g * Ns * R + k;
@@ -752,14 +771,21 @@ __device__ __forceinline__ void cstage_dit(C *sbuf, int pitch, int Ls, int Ns, f
   }
 }
 
+// element o1 of column k2, twiddled by W_M^{k2 o1}, into row k2 of V
+__device__ __forceinline__ void put_v(const PassC &pc, const Fft4Dev &p, int k2, int o1, C v) {
+  const C *tl = tab(p.tlane2) + 32 * k2, *tb = tab(p.tblk2) + k2 * p.nb32b;
+  pc.Vp[(int64_t)k2 * pc.PV + o1] = cmul(v, cmul(__ldg(tb + (o1 >> 5)), __ldg(tl + (o1 & 31))));
+}
+
 // the last DIT stage (Ns R = L1): rows warp by warp, outputs o1 = q + r Ns
-// twiddled by W_M^{k2 o1} and stored to V row k2
+// twiddled and stored to V
 template <int R, int FB>
 __device__ __forceinline__ void cstage_last(const C *sbuf, int pitch, int Ns, const C *stw,
                                             const C *wr, const PassC &pc, const Fft4Dev &p) {
   for (int bf = threadIdx.x; bf < FB * Ns; bf += Cfg<FB>::NT) {
     const int b = bf / Ns, q = bf - b * Ns;
-    if (b >= pc.nb) break;
+    const int k2 = c_col<FB>(pc, b);
+    if (k2 < 0) continue;
     const C *a = sbuf + b * pitch + q;
     C v[R];
 #pragma unroll
@@ -767,14 +793,8 @@ __device__ __forceinline__ void cstage_last(const C *sbuf, int pitch, int Ns, co
 #pragma unroll
     for (int r = 1; r < R; r++) v[r] = cmul(v[r], __ldg(stw + (r - 1) * Ns + q));
     Dft<R>::run(v, wr);
-    const int k2 = pc.k2_0 + b;
-    const C *tl = tab(p.tlane2) + 32 * k2, *tb = tab(p.tblk2) + k2 * p.nb32b;
-    C *row = pc.Vp + (int64_t)k2 * pc.L1;
 #pragma unroll
-    for (int r = 0; r < R; r++) {
-      const int o1 = q + r * Ns;
-      row[o1] = cmul(v[r], cmul(__ldg(tb + (o1 >> 5)), __ldg(tl + (o1 & 31))));
-    }
+    for (int r = 0; r < R; r++) put_v(pc, p, k2, q + r * Ns, v[r]);
   }
 }
 
@@ -816,8 +836,7 @@ __device__ __forceinline__ void cstage_last(const C *sbuf, int pitch, int Ns, co
     default: { constexpr int RR = 11; CALL; } break; \
   }
 
-// T[pair] (L1 x L2, from pass A on the chirped rows) -> V[pair] (L2 x L1);
-// needs nr1 >= 2
+// T[pair] (from pass A on the chirped rows) -> V[pair] (L2 x PV)
 template <int FB>
 __global__ void __launch_bounds__(Cfg<FB>::NT, Cfg<FB>::MINB) k_fft4_conv(const C *__restrict__ T, C *__restrict__ V,
                                                      const Fft4Dev p, const WrTable wt) {
@@ -826,25 +845,36 @@ __global__ void __launch_bounds__(Cfg<FB>::NT, Cfg<FB>::MINB) k_fft4_conv(const 
   const int L1 = p.L1, pitch = pitch_odd(L1), S = p.nr1;
   const int64_t pair = blockIdx.y;
   PassC pc;
-  pc.Tp = T + pair * p.L;
-  pc.Vp = V + pair * p.L;
+  pc.Tp = T + pair * p.tsz;
+  pc.Vp = V + pair * p.vsz;
   pc.bhat = tab(p.bhat);
   pc.L1 = L1;
   pc.L2 = p.L2;
-  pc.k2_0 = blockIdx.x * FB;
-  pc.nb = min(FB, p.L2 - pc.k2_0);
+  pc.P = p.P;
+  pc.PV = p.PV;
+  pc.k2_0 = blockIdx.x * (FB / 2);
+  pc.nh = min(FB / 2, p.H2 - pc.k2_0);
+  if (S == 1) {  // L1 <= 16: the shared butterfly pass alone, then the rows
+    MK_RADIX_SWITCH(p.r1[0], (cstage_mid<RR, FB, true>(sbuf, pitch, L1, p.iperm1, p.perm1, wt.w, pc)));
+    __syncthreads();
+    for (int e = threadIdx.x; e < FB * L1; e += Cfg<FB>::NT) {
+      const int b = e / L1, o1 = e - b * L1, k2 = c_col<FB>(pc, b);
+      if (k2 >= 0) put_v(pc, p, k2, o1, sbuf[b * pitch + o1]);
+    }
+    return;
+  }
   MK_RADIX_SWITCH(p.r1[S - 1], (cstage_first<RR, FB>(sbuf, pitch, p.ns1[S - 1], tab(p.stw1) + p.to1[S - 1], wt.w, pc)));
   __syncthreads();
   for (int s = S - 2; s >= 1; s--) {
     MK_RADIX_SWITCH(p.r1[s], (cstage_dif<RR, FB>(sbuf, pitch, L1, p.ns1[s], p.inv1[s], tab(p.stw1) + p.to1[s], wt.w,
-                                                 pc.nb)));
+                                                 pc.nh)));
     __syncthreads();
   }
-  MK_RADIX_SWITCH(p.r1[0], (cstage_mid<RR, FB>(sbuf, pitch, L1, p.iperm1, wt.w, pc)));
+  MK_RADIX_SWITCH(p.r1[0], (cstage_mid<RR, FB, false>(sbuf, pitch, L1, p.iperm1, p.perm1, wt.w, pc)));
   __syncthreads();
   for (int s = 1; s < S - 1; s++) {
     MK_RADIX_SWITCH(p.r1[s], (cstage_dit<RR, FB>(sbuf, pitch, L1, p.ns1[s], p.inv1[s], tab(p.stw1) + p.to1[s], wt.w,
-                                                 pc.nb)));
+                                                 pc)));
     __syncthreads();
   }
   MK_RADIX_SWITCH(p.r1[S - 1], (cstage_last<RR, FB>(sbuf, pitch, p.ns1[S - 1], tab(p.stw1) + p.to1[S - 1], wt.w, pc, p)));
@@ -883,19 +913,15 @@ int dct_launch(const Fft4Plan &p, const RT *x, int64_t ldx, int64_t nrow, C *T, 
   MK_CUDA(cudaGetDevice(&dev));
   if (dev >= 0 && dev < 64 && !g_attr[dev]) {
     const int mhi = FB_HI * (FFT4_LMAX + 1) * (int)sizeof(C);
-    const int mlo = FB_LO * (FFT4_LMAX + 1) * (int)sizeof(C) + FB_LO * FFT4_LMAX * 2 * (int)sizeof(RT);
+    const int mlo = FB_LO * (FFT4_LMAX + 1) * (int)sizeof(C);
 #define MK_FFT4_ATTR(k, v) MK_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, v))
     MK_FFT4_ATTR((k_fft4_a<AM_DCT, FB_LO>), mlo);
     MK_FFT4_ATTR((k_fft4_a<AM_BLUE, FB_LO>), mlo);
-    MK_FFT4_ATTR((k_fft4_a<AM_CPLX, FB_LO>), mlo);
     MK_FFT4_ATTR((k_fft4_b<BM_DCT, FB_LO>), mlo);
-    MK_FFT4_ATTR((k_fft4_b<BM_MUL, FB_LO>), mlo);
     MK_FFT4_ATTR((k_fft4_b<BM_BLUE, FB_LO>), mlo);
     MK_FFT4_ATTR((k_fft4_a<AM_DCT, FB_HI>), mhi);
     MK_FFT4_ATTR((k_fft4_a<AM_BLUE, FB_HI>), mhi);
-    MK_FFT4_ATTR((k_fft4_a<AM_CPLX, FB_HI>), mhi);
     MK_FFT4_ATTR((k_fft4_b<BM_DCT, FB_HI>), mhi);
-    MK_FFT4_ATTR((k_fft4_b<BM_MUL, FB_HI>), mhi);
     MK_FFT4_ATTR((k_fft4_b<BM_BLUE, FB_HI>), mhi);
     MK_FFT4_ATTR((k_fft4_conv<FB_LO>), mlo);
     MK_FFT4_ATTR((k_fft4_conv<FB_HI>), mhi);
@@ -905,87 +931,43 @@ int dct_launch(const Fft4Plan &p, const RT *x, int64_t ldx, int64_t nrow, C *T, 
   static const WrTable wt = make_wr();
   const bool hia = d.fba == FB_HI, hib = d.fbb == FB_HI;
   const int fa = hia ? FB_HI : FB_LO, fb = hib ? FB_HI : FB_LO;
-  const dim3 ga((d.L1 + fa - 1) / fa, (unsigned)npairs), gb((d.L2 + fb - 1) / fb, (unsigned)npairs);
-  const size_t smem_a = (size_t)fa * pitch_odd(d.L2) * sizeof(C);
-  const size_t smem_b = (size_t)fb * pitch_odd(d.L1) * sizeof(C);
-  // FILTER weights go through shared memory on FB_LO passes while two CTAs
-  // still fit an SM; otherwise the last stage reads them directly
-  const size_t smem_wlo = (size_t)FB_LO * d.L1 * 2 * sizeof(RT);
-  const int wpre = epi == FFT4_FILTER && !hib && smem_b + smem_wlo <= 113 * 1024;
-  const size_t smem_w = wpre ? smem_wlo : 0;
-  auto pass_a = [&](int am, const RT *xx, int64_t ldxx, const C *uu) {
-    if (hia) {
-      if (am == AM_DCT) k_fft4_a<AM_DCT, FB_HI><<<ga, Cfg<FB_HI>::NT, smem_a, st>>>(xx, ldxx, uu, nrow, T, d, wt);
-      else if (am == AM_BLUE) k_fft4_a<AM_BLUE, FB_HI><<<ga, Cfg<FB_HI>::NT, smem_a, st>>>(xx, ldxx, uu, nrow, T, d, wt);
-      else k_fft4_a<AM_CPLX, FB_HI><<<ga, Cfg<FB_HI>::NT, smem_a, st>>>(xx, ldxx, uu, nrow, T, d, wt);
-    } else {
-      if (am == AM_DCT) k_fft4_a<AM_DCT, FB_LO><<<ga, Cfg<FB_LO>::NT, smem_a, st>>>(xx, ldxx, uu, nrow, T, d, wt);
-      else if (am == AM_BLUE) k_fft4_a<AM_BLUE, FB_LO><<<ga, Cfg<FB_LO>::NT, smem_a, st>>>(xx, ldxx, uu, nrow, T, d, wt);
-      else k_fft4_a<AM_CPLX, FB_LO><<<ga, Cfg<FB_LO>::NT, smem_a, st>>>(xx, ldxx, uu, nrow, T, d, wt);
-    }
-  };
-  auto pass_b = [&](int bm, C *uu, int e, size_t sm, int wp) {
-    if (hib) {
-      if (bm == BM_DCT)
-        k_fft4_b<BM_DCT, FB_HI><<<gb, Cfg<FB_HI>::NT, sm, st>>>(T, nrow, out, ldo, uu, w, ldw, e, wp, d, wt);
-      else if (bm == BM_MUL)
-        k_fft4_b<BM_MUL, FB_HI><<<gb, Cfg<FB_HI>::NT, sm, st>>>(T, nrow, out, ldo, uu, w, ldw, e, wp, d, wt);
-      else
-        k_fft4_b<BM_BLUE, FB_HI><<<gb, Cfg<FB_HI>::NT, sm, st>>>(T, nrow, out, ldo, uu, w, ldw, e, wp, d, wt);
-    } else {
-      if (bm == BM_DCT)
-        k_fft4_b<BM_DCT, FB_LO><<<gb, Cfg<FB_LO>::NT, sm, st>>>(T, nrow, out, ldo, uu, w, ldw, e, wp, d, wt);
-      else if (bm == BM_MUL)
-        k_fft4_b<BM_MUL, FB_LO><<<gb, Cfg<FB_LO>::NT, sm, st>>>(T, nrow, out, ldo, uu, w, ldw, e, wp, d, wt);
-      else
-        k_fft4_b<BM_BLUE, FB_LO><<<gb, Cfg<FB_LO>::NT, sm, st>>>(T, nrow, out, ldo, uu, w, ldw, e, wp, d, wt);
-    }
-  };
+  const unsigned np = (unsigned)npairs;
+  const size_t smem_a = (size_t)fa * pitch_odd(d.L2) * sizeof(C);  // transforms of length L2
+  const size_t smem_b = (size_t)fb * pitch_odd(d.L1) * sizeof(C);  // transforms of length L1
+  const dim3 ga((d.H1 + fa - 1) / fa, np);
   int rc;
   if (!d.blue) {
-    pass_a(AM_DCT, x, ldx, nullptr);
+    const dim3 gb((d.H2 + fb - 1) / fb, np);
+    if (hia) k_fft4_a<AM_DCT, FB_HI><<<ga, Cfg<FB_HI>::NT, smem_a, st>>>(x, ldx, nrow, T, d, wt);
+    else k_fft4_a<AM_DCT, FB_LO><<<ga, Cfg<FB_LO>::NT, smem_a, st>>>(x, ldx, nrow, T, d, wt);
     if ((rc = launch_status("fft4 pass A"))) return rc;
-    pass_b(BM_DCT, nullptr, epi, smem_b + smem_w, wpre);
+    if (hib) k_fft4_b<BM_DCT, FB_HI><<<gb, Cfg<FB_HI>::NT, smem_b, st>>>(T, nrow, out, ldo, w, ldw, epi, d, wt);
+    else k_fft4_b<BM_DCT, FB_LO><<<gb, Cfg<FB_LO>::NT, smem_b, st>>>(T, nrow, out, ldo, w, ldw, epi, d, wt);
     return launch_status("fft4 pass B");
   }
-  C *U = T + npairs * d.L;
-  pass_a(AM_BLUE, x, ldx, nullptr);
+  C *V = T + npairs * d.tsz;
+  if (hia) k_fft4_a<AM_BLUE, FB_HI><<<ga, Cfg<FB_HI>::NT, smem_a, st>>>(x, ldx, nrow, T, d, wt);
+  else k_fft4_a<AM_BLUE, FB_LO><<<ga, Cfg<FB_LO>::NT, smem_a, st>>>(x, ldx, nrow, T, d, wt);
   if ((rc = launch_status("fft4 Bluestein pass A"))) return rc;
-  if (d.nr1 >= 2 && !d.blue4) {
-    // the middle pass T -> V (= U's space), then pass B on the transposed
-    // shape: length L2 over the rows of V, outputs o1 + L1 o2
-    const size_t smem_c = (size_t)fb * pitch_odd(d.L1) * sizeof(C);
-    if (hib) k_fft4_conv<FB_HI><<<gb, Cfg<FB_HI>::NT, smem_c, st>>>(T, U, d, wt);
-    else k_fft4_conv<FB_LO><<<gb, Cfg<FB_LO>::NT, smem_c, st>>>(T, U, d, wt);
-    if ((rc = launch_status("fft4 Bluestein middle pass"))) return rc;
-    Fft4Dev tr = d;
-    std::swap(tr.L1, tr.L2);
-    std::swap(tr.nr1, tr.nr2);
-    std::swap(tr.r1, tr.r2);
-    std::swap(tr.ns1, tr.ns2);
-    std::swap(tr.to1, tr.to2);
-    std::swap(tr.inv1, tr.inv2);
-    std::swap(tr.stw1, tr.stw2);
-    std::swap(tr.iperm1, tr.iperm2);
-    const dim3 gt((tr.L2 + fa - 1) / fa, (unsigned)npairs);
-    const size_t smem_t = (size_t)fa * pitch_odd(tr.L1) * sizeof(C);
-    const size_t smem_twlo = (size_t)FB_LO * tr.L1 * 2 * sizeof(RT);
-    const int wpre_t = epi == FFT4_FILTER && !hia && smem_t + smem_twlo <= 113 * 1024;
-    const size_t smem_tw = wpre_t ? smem_twlo : 0;
-    if (hia)
-      k_fft4_b<BM_BLUE, FB_HI><<<gt, Cfg<FB_HI>::NT, smem_t, st>>>(U, nrow, out, ldo, nullptr, w, ldw, epi, 0, tr,
-                                                                   wt);
-    else
-      k_fft4_b<BM_BLUE, FB_LO><<<gt, Cfg<FB_LO>::NT, smem_t + smem_tw, st>>>(U, nrow, out, ldo, nullptr, w, ldw, epi,
-                                                                             wpre_t, tr, wt);
-    return launch_status("fft4 Bluestein last pass");
-  }
-  pass_b(BM_MUL, U, FFT4_PLAIN, smem_b, 0);
-  if ((rc = launch_status("fft4 Bluestein pass B"))) return rc;
-  pass_a(AM_CPLX, nullptr, 0, U);
-  if ((rc = launch_status("fft4 Bluestein pass A (second)"))) return rc;
-  pass_b(BM_BLUE, nullptr, epi, smem_b + smem_w, wpre);
-  return launch_status("fft4 Bluestein pass B (second)");
+  const dim3 gc((d.H2 + fb / 2 - 1) / (fb / 2), np);
+  if (hib) k_fft4_conv<FB_HI><<<gc, Cfg<FB_HI>::NT, smem_b, st>>>(T, V, d, wt);
+  else k_fft4_conv<FB_LO><<<gc, Cfg<FB_LO>::NT, smem_b, st>>>(T, V, d, wt);
+  if ((rc = launch_status("fft4 Bluestein middle pass"))) return rc;
+  // pass B on the transposed shape: length L2 over the rows of V, outputs
+  // o1 + L1 o2
+  Fft4Dev tr = d;
+  std::swap(tr.L1, tr.L2);
+  std::swap(tr.nr1, tr.nr2);
+  std::swap(tr.r1, tr.r2);
+  std::swap(tr.ns1, tr.ns2);
+  std::swap(tr.to1, tr.to2);
+  std::swap(tr.inv1, tr.inv2);
+  std::swap(tr.stw1, tr.stw2);
+  std::swap(tr.iperm1, tr.iperm2);
+  const dim3 gt((tr.L2 + fa - 1) / fa, np);
+  if (hia) k_fft4_b<BM_BLUE, FB_HI><<<gt, Cfg<FB_HI>::NT, smem_a, st>>>(V, nrow, out, ldo, w, ldw, epi, tr, wt);
+  else k_fft4_b<BM_BLUE, FB_LO><<<gt, Cfg<FB_LO>::NT, smem_a, st>>>(V, nrow, out, ldo, w, ldw, epi, tr, wt);
+  return launch_status("fft4 Bluestein last pass");
 }
 
 }  // namespace MK_FFT4_NS

@@ -309,6 +309,22 @@ def test_dct1_f64_four_step(K, nrow, n, fb, monkeypatch):
         K.set_dct_engine(0)
 
 
+@pytest.mark.parametrize("dtype,tol", [(torch.float64, 1e-12), (torch.float32, 1e-5)])
+@pytest.mark.parametrize("split", [0, 1, 2])
+def test_dct1_every_short_length(K, dtype, tol, split):
+    """Every row length 2 .. 70 (smooth and Bluestein, one- and two-stage
+    passes, odd and even L1 and L2: the self-mirrored columns and rows of the
+    half transform) with the three closest splits, three rows, against the
+    FP64 oracle.  Tolerances: those of the longer lengths above (rounding
+    grows with the number of stages, which is smallest here)."""
+    from minkasi_gb300.autotune import with_dct_engine
+    for n in range(2, 71):
+        x = np.random.default_rng(n).standard_normal((3, n))
+        d = with_dct_engine((0, split), lambda: K.DCT1(3, n, dtype))
+        assert d.engine in (0, 2)
+        assert rel(d(dev(x, dtype)).cpu().numpy(), oracle.dct1(x)) < tol, n
+
+
 def test_dct1_engines_agree_and_fall_back(K):
     x = np.random.default_rng(9).standard_normal((6, 2311))
     own = K.DCT1(6, 2311, torch.float32)(dev(x, torch.float32)).cpu().numpy()
