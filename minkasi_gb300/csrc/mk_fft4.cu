@@ -216,8 +216,9 @@ int fft4_split_rank() { return g_split_rank.load(); }
 
 // L1 x L2 split of a transform of length L (by g_split_rank among the
 // divisor pairs with both parts <= LMAX and L1 > 1, ordered by closeness to
-// sqrt(L)), radices and stage constants
-static bool split_len(int64_t L, Fft4Dev *t) {
+// sqrt(L)), radices and stage constants.  Bluestein's last pass runs the
+// transposed shape, so there L2 > 1 too.
+static bool split_len(int64_t L, Fft4Dev *t, bool bluestein) {
   if (L < 2 || L > (int64_t)FFT4_LMAX * FFT4_LMAX) return false;
   std::vector<int> f;
   factor(L, f);
@@ -235,7 +236,7 @@ static bool split_len(int64_t L, Fft4Dev *t) {
   std::vector<std::pair<double, int64_t>> cand;
   for (int64_t a : ds) {
     const int64_t b = L / a;
-    if (a > FFT4_LMAX || b > FFT4_LMAX || a == 1) continue;  // pass B needs at least one stage
+    if (a > FFT4_LMAX || b > FFT4_LMAX || a == 1 || (bluestein && b == 1)) continue;  // pass B needs a stage
     cand.push_back({std::fabs(std::log((double)a) - std::log((double)b)), a});
   }
   if (cand.empty()) return false;
@@ -290,12 +291,12 @@ bool fft4_shape(int64_t n, Fft4Dev *d, bool bluestein, bool f64) {
   t.m = n - 1;
   t.Lx = 2 * t.m;
   bool ok = false;
-  if (split_len(t.Lx, &t)) {
+  if (split_len(t.Lx, &t, false)) {
     t.blue = false;
     ok = true;
   } else if (bluestein) {
     for (int64_t M = 3 * t.m; M <= (int64_t)FFT4_LMAX * FFT4_LMAX && !ok; M++) {
-      if (split_len(M, &t)) {
+      if (split_len(M, &t, true)) {
         t.blue = true;
         ok = true;
       }
