@@ -112,7 +112,7 @@ def choose_rot_mode(op) -> int:
     forced = os.environ.get("MINKASI_GB300_ROT")
     if forced:
         return int(forced)
-    key = workload_key(op, "rot")
+    key = workload_key(op, "rot2")
     hit = _lookup(key)
     if hit is not None:
         return int(hit)

@@ -420,12 +420,8 @@ int rotate(DctCore *c, int mode, const void *A, const void *X, int64_t ldx, void
   }
   if (mode == 4) {
     MK_CHECK_ARG(dtype == MK_F64 && c->oz_ws, "sliced tensor-core rotation (rot_mode 4) is FP64 only");
-    std::lock_guard<std::mutex> lk(g_blas_mu);
-    cublasHandle_t h;
-    int rc = blas_handle(&h);
-    if (rc) return rc;
-    return mk::ozaki_rotate_f64(h, (const double *)A, (const double *)X, ldx, (double *)R, ldr, nrow, ncol,
-                                c->oz_ws, c->oz_bytes, st);
+    return mk::ozaki_rotate_f64((const double *)A, (const double *)X, ldx, (double *)R, ldr, nrow, ncol, c->oz_ws,
+                                c->oz_bytes, c->tc_err, st);
   }
   MK_CHECK_ARG(mode == 1 || mode == 3, "bad rot_mode %d", mode);
   return blas_rotate(dtype, A, X, ldx, R, ldr, nrow, ncol, mode == 3, st);

@@ -415,6 +415,30 @@ def test_sliced_fp64_rotation(K, nd, n):
     assert np.array_equal(got[:, 5], np.zeros(nd))
 
 
+@pytest.mark.parametrize("nd,n", [(1, 2), (31, 127), (32, 128), (33, 129), (128, 257), (129, 300), (257, 131), (300, 2)])
+def test_sliced_fp64_rotation_tile_edges(K, nd, n):
+    """The sliced rotation around its tile sizes (32 detectors, 128 samples,
+    accumulations of 128 detectors), negative powers of two (whose leading
+    digit is -128) and a non-finite column, against extended precision.
+    Bound: each of the nd terms drops 6 digit products of at most 2^14 2^-70
+    and rounds both factors at 2^-56, so 2^-53 per term relative to the row and
+    column scales (at most twice the largest entries), plus the last rounding."""
+    rng = np.random.default_rng(100 * nd + n)
+    A = rng.standard_normal((nd, nd))
+    X = rng.standard_normal((nd, n))
+    A[0, :] = -2.0 ** -3
+    X[:, n - 1] = -0.5
+    want = (A.astype(np.longdouble) @ X.astype(np.longdouble))
+    plan = K.NoisePlan(nd, n, torch.float64)
+    got = plan.rotate(dev(A), dev(X), rot_mode=4).cpu().numpy()
+    scale = np.abs(A).max(1)[:, None] * np.abs(X).max(0)[None, :]
+    assert (np.abs(got - want) <= 4 * nd * 2.0 ** -53 * scale + 2.0 ** -53 * np.abs(want)).all()
+    X[nd // 2, 0] = np.inf
+    got = plan.rotate(dev(A), dev(X), rot_mode=4).cpu().numpy()
+    assert np.isnan(got[:, 0]).all() and np.isfinite(got[:, 1:]).all()
+    assert plan.status() == 0
+
+
 def test_apply_noise_golden_f64_sliced_rotation(K, gold):
     """The reference's apply_noise (noise.npz) with the sliced FP64 rotation."""
     g = gold("noise.npz")
