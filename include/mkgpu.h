@@ -303,8 +303,8 @@ int mk_tod2map_fixed_noalloc(void *map, const void *dat, const int32_t *ipix, in
  * The workspace holds only scratch of one call, so plans of any shapes may
  * share one (sized for the largest) when their calls are stream-ordered.
  * What a plan keeps between calls (cuFFT's plan data; the four-step
- * engine's twiddle and permutation tables, at most a few hundred KB; the
- * tensor-core status word) is device memory the plan allocates at creation
+ * engine's twiddle and permutation tables, a few hundred KB in FP32, 16 B per
+ * sample of one row more in FP64; the tensor-core status word) is device memory the plan allocates at creation
  * and frees on destroy.
  * Replaces many_fft_r2r_1d / many_fftf_r2r_1d, minkasi/lib/mkfftw.c:174-254. */
 typedef struct mk_dct_plan mk_dct_plan;

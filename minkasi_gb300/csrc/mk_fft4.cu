@@ -135,7 +135,7 @@ bool radices(int Ls, int *r, int *nr, int rmax) {
 size_t al(size_t x) { return (x + 255) / 256 * 256; }
 
 struct TableLayout {
-  size_t stw1, stw2, iperm1, iperm2, perm1, tlane, tblk, chirp, bhat, tlane2, tblk2, total;
+  size_t stw1, stw2, iperm1, iperm2, perm1, tlane, tblk, tfull, chirp, bhat, tlane2, tblk2, total;
 };
 
 size_t csz(const Fft4Dev &d) { return d.f64 ? sizeof(double2) : sizeof(float2); }
@@ -157,6 +157,8 @@ TableLayout layout(const Fft4Dev &d) {
   o += al((size_t)d.H1 * 32 * csz(d));
   t.tblk = o;
   o += al((size_t)d.H1 * d.nb32 * csz(d));
+  t.tfull = o;
+  o += d.f64 ? al((size_t)d.tsz * csz(d)) : 0;
   t.chirp = o;
   o += d.blue ? al((size_t)(d.m + 2) * csz(d)) : 0;
   t.bhat = o;
@@ -250,8 +252,9 @@ static bool split_len(int64_t L, Fft4Dev *t, bool bluestein) {
   if (!radices(t->L1, t->r1, &t->nr1, rmax) || !radices(t->L2, t->r2, &t->nr2, rmax)) return false;
   t->H1 = t->L1 / 2 + 1;
   t->H2 = t->L2 / 2 + 1;
-  t->nb32 = (t->H2 + 31) / 32;
-  t->P = (2 * t->H2 + 15) / 16 * 16;
+  t->pad = (t->H2 + 31) / 32 * 32 - (t->L2 + 1) / 2;
+  t->nb32 = (t->L2 + t->pad + 31) / 32;
+  t->P = (t->L2 + t->pad + 15) / 16 * 16;
   t->PV = (t->L1 + 15) / 16 * 16;
   t->tsz = (int64_t)t->H1 * t->P;
   t->vsz = (int64_t)t->L2 * t->PV;
@@ -269,6 +272,7 @@ static bool split_len(int64_t L, Fft4Dev *t, bool bluestein) {
       span *= r[s];
     }
   }
+  t->qh = t->L2 % 2 || t->nr2 == 0 ? -1 : (t->L2 / 2) % t->ns2[t->nr2 - 1];
   return true;
 }
 
@@ -373,8 +377,11 @@ int fft4_init(Fft4Plan *p, int64_t n, void *dev_tables, bool bluestein, bool f64
   }
   for (int64_t j1 = 0; j1 < d.H1; j1++) {
     for (int l = 0; l < 32; l++) put(h.data(), t.tlane, 32 * j1 + l, unit((double)(j1 * l % d.L), (double)d.L), d.f64);
-    for (int i = 0; i < d.nb32; i++)
-      put(h.data(), t.tblk, j1 * d.nb32 + i, unit((double)(j1 * 32 * i % d.L), (double)d.L), d.f64);
+    for (int i = 0; i < d.nb32; i++) {
+      // the signed k of the block's first entry: e, or e - pad - L2 in the upper half
+      const int64_t e = 32 * i, k = e < d.L2 / 2 + d.pad ? e : e - d.pad - d.L2;
+      put(h.data(), t.tblk, j1 * d.nb32 + i, unit((double)(j1 * k % d.L), (double)d.L), d.f64);
+    }
   }
   if (d.blue) {
     for (int64_t j = 0; j <= d.m; j++)
@@ -403,12 +410,13 @@ int fft4_init(Fft4Plan *p, int64_t n, void *dev_tables, bool bluestein, bool f64
   d.perm1 = d.blue ? (const int *)(b + t.perm1) : nullptr;
   d.tlane = (const void *)(b + t.tlane);
   d.tblk = (const void *)(b + t.tblk);
+  d.tfull = d.f64 ? (const void *)(b + t.tfull) : nullptr;
   d.chirp = d.blue ? (const void *)(b + t.chirp) : nullptr;
   d.bhat = d.blue ? (const void *)(b + t.bhat) : nullptr;
   d.tlane2 = d.blue ? (const void *)(b + t.tlane2) : nullptr;
   d.tblk2 = d.blue ? (const void *)(b + t.tblk2) : nullptr;
   p->tables = dev_tables;
-  return MK_OK;
+  return d.f64 ? fft4_tfull_f64(d, (double2 *)(b + t.tfull)) : MK_OK;
 }
 
 

@@ -13,16 +13,19 @@
 //   * column L1 - j1 of e is column j1 reversed, so
 //     A_{L1-j1}[k2] = W_L2^{-k2} A_j1[L2 - k2] and
 //     W_L^{(L1-j1) k2} A_{L1-j1}[k2] = W_L^{-j1 k2} A_j1[L2 - k2]:
-//     pass A runs the H1 = L1 / 2 + 1 columns j1 <= L1 / 2 only, and stores per
-//     column and k <= L2 / 2 the two values W_L^{j1 k} A_j1[k] (entry k of row
-//     j1 of T) and W_L^{-j1 k} A_j1[L2 - k] (entry P - 1 - k), of which pass B
-//     reads one for j1 and the other for L1 - j1;
+//     pass A runs the H1 = L1 / 2 + 1 columns j1 <= L1 / 2 only, and multiplies
+//     A_j1[k2] by W_L^{j1 k2} for k2 <= L2 / 2 and by W_L^{j1 (k2 - L2)} beyond;
+//     pass B's column k <= L2 / 2 reads entry k for row j1 and entry L2 - k for
+//     row L1 - j1.  Entries above L2 / 2 sit `pad` further, so that they start
+//     at a multiple of 32 (the twiddle blocks), with the other sign's value of
+//     entry L2 / 2 (L2 even) before them at L2 / 2 + pad;
 //   * F_{L-k} = F_k, and L - (k2 + L2 k1) lies in column L2 - k2, so pass B
 //     runs the H2 = L2 / 2 + 1 columns k2 <= L2 / 2 only and writes each
 //     output to k or L - k, whichever is <= m.
-// One DCT-I of 256 x 130,978 takes 0.193 ms in FP32 and 3.06 ms in FP64 this
-// way, against 0.307 and 5.63 ms with all columns; Bluestein (below) on
-// 256 x 144,278 0.829 and 15.3 ms against 0.953 and 20.1 ms.
+// One DCT-I of 256 x 130,978 takes 0.171 ms in FP32 and 2.52 ms in FP64,
+// against 0.307 and 5.63 ms with all columns (0.193 and 3.06 ms before the
+// butterflies' operation counts and the index arithmetic were cut);
+// Bluestein (below) on 256 x 144,278 0.742 and 13.4 ms against 0.953 and 20.1.
 // Each CTA runs 8 or 16 (FP64: 4 or 8) transforms of one pass in shared memory (mixed-radix
 // decimation in time, butterflies in place), interleaved over its threads.
 // The first stage of each pass reads its inputs straight from global memory
@@ -72,9 +75,10 @@ struct Fft4Dev {
   bool f64;         // FP64 plan: tables of double2, FP64 kernels
   int L1, L2;
   int H1, H2;        // L1 / 2 + 1, L2 / 2 + 1: the columns an even transform needs
-  int P, PV;         // row pitch of T (2 H2) and of V (L1), rounded up to 16
+  int pad, qh;       // T's upper entries are shifted by pad; qh = (L2 / 2) mod (last span of L2), or -1 (L2 odd)
+  int P, PV;         // row pitch of T (L2 + pad) and of V (L1), rounded up to 16
   int64_t tsz, vsz;  // elements of T and of V per row pair
-  int nb32;          // blocks of 32 covering 0 .. L2 / 2
+  int nb32;          // blocks of 32 covering a row of T
   int fba, fbb;      // transforms per CTA of pass A (length L2) and pass B (length L1): 8 or 16
   int nr1, nr2;
   int r1[FFT4_MAXR], r2[FFT4_MAXR];
@@ -86,8 +90,9 @@ struct Fft4Dev {
   const void *stw1, *stw2;
   const int *iperm1, *iperm2;  // natural index at each digit-reversed (DIT input) position
   const int *perm1;            // Bluestein: digit-reversed position of each natural index (length L1)
-  // four-step twiddle W_L^{j1 k} = tblk[j1 nb32 + k / 32] * tlane[32 j1 + k % 32], j1 < H1, k < H2
-  const void *tlane, *tblk;
+  // four-step twiddle of entry e of row j1 of T: tblk[j1 nb32 + e / 32] * tlane[32 j1 + e % 32]; FP64 plans
+  // hold the products too, tfull[j1 P + e]
+  const void *tlane, *tblk, *tfull;
   const void *chirp;  // Bluestein: c_t for t < m, c_m / 2 at m, c_m at m + 1
   const void *bhat;   // Bluestein: DFT_M(b) / M
   // Bluestein's middle pass: W_M^{k2 o1} = tblk2[k2 nb32b + o1 / 32] * tlane2[32 k2 + o1 % 32]
@@ -125,5 +130,7 @@ int fft4_dct(const Fft4Plan &p, const float *x, int64_t ldx, int64_t nrow, float
 // the same for an FP64 plan (fft4_init with f64)
 int fft4_dct_f64(const Fft4Plan &p, const double *x, int64_t ldx, int64_t nrow, double2 *T, double *out,
                  int64_t ldo, int epi, const double *w, int64_t ldw, cudaStream_t st);
+// fills out[H1 P] with an FP64 plan's four-step twiddles (returns when done)
+int fft4_tfull_f64(const Fft4Dev &d, double2 *out);
 
 }  // namespace mk
