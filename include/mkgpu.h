@@ -345,8 +345,8 @@ int mk_get_fft4_split(void);
  * the caller.  The plan shares the DCT workspace contract above and may be
  * used for any TOD of the same (ndet, ndata).  rot_mode selects the
  * detector-rotation GEMM: 0 = automatic, 1 = cuBLAS on the FP64 / FP32 units
- * (DGEMM / SGEMM), 2 = this library's tensor-core kernel (FP32 only: 3xTF32
- * split products, FP32 accumulate), 3 = cuBLAS tensor-core emulation (FP64:
+ * (DGEMM / SGEMM), 2 = this library's tensor-core kernel (FP32 only: three
+ * bf16 parts per value, exact, six of their products, FP32 accumulate), 3 = cuBLAS tensor-core emulation (FP64:
  * fixed-point slices; FP32: BF16x9), 4 = FP64 only: this library's exact
  * slicing of both operands into 7 signed integer slices of 8 bits after
  * power-of-two row / column scaling, their products on the bf16 tensor cores
@@ -379,7 +379,7 @@ int mk_noise_status(mk_noise_plan *plan, int *code, void *stream);
 /* NoiseSmoothedSVD.apply_noise of many TODs in one call, in place on each
  * TOD's (ndet, ndata) float32 timestream data[t] (the batched operator's
  * pooled buffer): the v and vT detector rotations of all TODs with the same
- * detector count run as one tensor-core launch each (3xTF32, as rot_mode 2),
+ * detector count run as one tensor-core launch each (as rot_mode 2),
  * and each TOD's two DCT-I run on its plan (plans[t]: FP32, any DCT engine,
  * ndet in {32, 64, 128, 256}).  Same arithmetic as mk_apply_noise with
  * rot_mode 2 on each TOD, bit for bit.  The group keeps the rotation

@@ -108,7 +108,7 @@ def choose_rot_mode(op) -> int:
     """Fastest rotation GEMM that agrees with the FP64/FP32 cuBLAS result
     (rel. 1e-13 in FP64, 1e-5 in FP32) on the largest TOD shape: cuBLAS on
     the FP64/FP32 units (1), cuBLAS emulation (3), and this library's
-    tensor-core kernels (2: FP32 3xTF32; 4: FP64 exact integer slices)."""
+    tensor-core kernels (2: FP32 as three bf16 parts; 4: FP64 exact integer slices)."""
     forced = os.environ.get("MINKASI_GB300_ROT")
     if forced:
         return int(forced)

@@ -652,7 +652,7 @@ extern "C" int mk_noise_group_create(mk_noise_group **group, int ntod, mk_noise_
     for (int t = 0; t < ntod; t++) {
       const DctCore &c = plans[t]->core;
       if (c.nrow != cl.ndet) continue;
-      const int64_t tiles = (c.n + 127) / 128;
+      const int64_t tiles = mk::rot_tc_items(c.nrow, c.n);
       jv.push_back({data[t], data[t], img_v[t], c.n, c.n, c.n, cl.ntile});
       jvT.push_back({data[t], data[t], img_vT[t], c.n, c.n, c.n, cl.ntile});
       cl.ntile += tiles;

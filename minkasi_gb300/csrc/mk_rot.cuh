@@ -1,5 +1,5 @@
-// Detector-space rotation R = A . X on the tensor cores (FP32 in/out,
-// 3xTF32 split products, FP32 accumulation).  A is (nrow x nrow), X is
+// Detector-space rotation R = A . X on the tensor cores (FP32 in/out, three
+// bf16 parts per value, FP32 accumulation).  A is (nrow x nrow), X is
 // (nrow x ncol) with leading dimension ldx, R has leading dimension ldr; all
 // row-major.  Used by apply_noise for the v / vT rotations.
 #pragma once
@@ -22,17 +22,18 @@ int rot_tc_f32(const float *A, const float *X, int64_t ldx, float *R, int64_t ld
                int64_t x_stride = 1, int halve_ends = 0);
 
 // One TOD of a grouped rotation: R = A . X with A given by its operand image
-// bimg (rot_tc_bprep); tile0 = the first of its ceil(ncol / 128) tiles in the
-// launch (jobs sorted by tile0, contiguous).  R may equal X (in place): the
-// kernel reads all of a tile's inputs before it writes that tile.
+// bimg (rot_tc_bprep); tile0 = the first of its rot_tc_items(nrow, ncol) work
+// items in the launch (jobs sorted by tile0, contiguous).  R may equal X (in
+// place): the kernel reads all of a tile's inputs before it writes that tile.
 struct RotJob {
   const float *X;
   float *R;
   const char *bimg;
   int64_t ldx, ldr, ncol, tile0;
 };
+int64_t rot_tc_items(int64_t nrow, int64_t ncol);
 // the operand image of A (rot_tc_bimg_bytes(nrow) bytes)
 int rot_tc_bprep(const float *A, int64_t nrow, void *bimg, cudaStream_t st);
 // every job of the (device) table in one launch; all jobs have nrow detectors
-int rot_tc_group(const RotJob *jobs_dev, int njobs, int64_t ntile, int64_t nrow, int *err, cudaStream_t st);
+int rot_tc_group(const RotJob *jobs_dev, int njobs, int64_t nitem, int64_t nrow, int *err, cudaStream_t st);
 }  // namespace mk

@@ -1,31 +1,47 @@
-// Detector rotation R = A . X on the 5th-generation tensor cores
-// (tcgen05.mma kind::tf32), FP32 in / FP32 out, 3xTF32 split precision:
-//   A = Ah + Al, X = Xh + Xl (h = round-to-TF32, l = remainder, also TF32)
-//   R ~= Xh.Ah + Xl.Ah + Xh.Al   accumulated in FP32 in tensor memory.
-// The dropped Xl.Al term is ~2^-22 relative, so the result carries FP32-level
-// accuracy (the apply_noise rotations np.dot(v, dat), np.dot(vT, .) of
-// minkasi/mapmaking/noise.py:704,709).
+// Detector rotation R = A . X on the 5th-generation tensor cores, FP32 in /
+// FP32 out: the apply_noise rotations np.dot(v, dat), np.dot(vT, .) of
+// minkasi/mapmaking/noise.py:704,709.
 //
-// Tile mapping (all operands K-major, 128-byte swizzle):
+// Split: every FP32 value is the exact sum of three bf16 values, x = h + m + l
+// (8 significant bits each, every part rounded to nearest), and
+//   R ~= h h + h m + m h + m m + h l + l h   (tcgen05.mma kind::f16, FP32
+// accumulation in tensor memory); the dropped products are below 2^-25
+// relative.  (Two TF32 parts need 8 B per value where three bf16 parts need
+// 6 B, at the same MMA time, and drop products of 2^-22.)
+//
+// Tile mapping (all operands K-major, 64-byte swizzle):
 //   D^T (128 samples x ndet) = X^T (128 samples x K=ndet) . A^T (K x N=ndet)
-//   MMA A-operand: the X^T tile.  Each thread owns one sample row; it loads
-//     its 32 detector values of a K-chunk (coalesced across the warp: 32
-//     consecutive samples of one detector row), splits them, and writes the
-//     hi and lo rows (128 B each) into shared memory.
+//   MMA A-operand: the X^T tile.  A split thread owns one sample; it loads the
+//     32 detector values of a K-chunk (coalesced across the warp: 32
+//     consecutive samples of one detector row) one chunk ahead into registers,
+//     splits them, and writes three rows of 64 B into shared memory.
 //   MMA B-operand: rows j = output detector, K contiguous = A[j][k0..k0+31],
-//     i.e. A row-major.  Its hi/lo split is built once per call by k_bprep
-//     in exactly the shared-memory image and bulk-copied (cp.async.bulk)
-//     per K-chunk, completing on an mbarrier.
+//     i.e. A row-major.  Its split is built by k_bprep in exactly the
+//     shared-memory image and bulk-copied (cp.async.bulk) per K-chunk.
 //   Accumulator: 128 TMEM lanes (= samples) x ndet columns (= detectors).
-//   Epilogue: each warp reads its 32 lanes with tcgen05.ld 32x32b and
-//     stores, per detector column, 32 consecutive samples (128 B, coalesced).
-// Pipeline: 2 shared-memory stages; the MMAs of chunk g run while the
-// threads split chunk g+1.  One elected thread issues the MMAs and the bulk
-// copies.  Every mbarrier wait is bounded: on timeout the CTA records an
-// error code, waits (bounded) for its outstanding MMAs, frees its tensor
-// memory and returns.
-#include <cstdlib>
-
+//
+// MT tiles of 128 samples share one pass over the operand image: it is
+// 6 ndet^2 bytes per pass against 512 ndet bytes of X per tile, so at 256
+// detectors one tile per pass reads three times as much of A's image from L2
+// as of X from memory, which is what bounded the kernel (with the 8 B TF32
+// image: 0.156 ms on 256 x 130,978).  MT = 2 there (one CTA per SM: two
+// accumulators of 256 columns fill tensor memory); MT = 1 below, where two
+// CTAs fit an SM and each has two accumulators.
+//
+// Roles: MT x 4 split warps; MT x 4 epilogue warps (warp w reads TMEM lanes
+// 32 (w % 4) .. of its tile and stores per detector 32 consecutive samples);
+// one warp whose first lane issues the image copies and the MMAs.  Two
+// shared-memory stages: the MMAs of chunk g run while chunk g + 1 is split.
+// Measured against the 3xTF32 kernels before it (8 B per value, one tile per
+// pass; error against FP64 in brackets): 256 x 450,561 0.31 ms (1.7e-6) for
+// 0.47 (1.9e-6), 256 x 130,978 0.110 for 0.146, 128 x 563,201 0.151 (8.2e-7)
+// for 0.259 (9.7e-7), 64 x 65,341 0.017 for 0.025.
+// Every wait is bounded and also polls the CTA's abort flag, so a timeout in
+// one role ends all of them; the MMA thread then drains its outstanding
+// copies and MMAs (bounded) before the tensor memory is freed.
+//
+// A tile's inputs are all read before its outputs are written, so R may be X.
+// One launch covers a table of TODs (per-TOD pointers, lengths, images).
 #include "mk_async.cuh"
 #include "mk_common.cuh"
 #include "mk_rot.cuh"
@@ -38,39 +54,51 @@ using mk::mbar_init;
 using mk::mbar_wait;
 using mk::smem_u32;
 
-constexpr int TILE_M = 128;      // samples per tile (MMA M)
-constexpr int KC = 32;           // K per chunk: one 128-byte swizzle row of tf32
+constexpr int TILE_M = 128;  // samples per MMA tile
+constexpr int KC = 32;       // K per chunk: one 64-byte swizzle row of bf16
 constexpr int NSTAGE = 2;
-constexpr int NTHREADS = 128;
+constexpr uint32_t A_PART = TILE_M * 64;   // one of the three parts of an X tile chunk (8 KB)
+constexpr uint32_t A_TILE = 3 * A_PART;
 
-__device__ __forceinline__ float tf32_round(float x) {
+// two floats rounded to bf16 (nearest; NaN and infinity stay), and the parts as
+// floats again
+__device__ __forceinline__ uint32_t bf16_pair(float a, float b) {
   uint32_t r;
-  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(x));
-  return __uint_as_float(r);
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(b), "f"(a));
+  return r;
+}
+__device__ __forceinline__ float lo_part(uint32_t p) { return __uint_as_float(p << 16); }
+__device__ __forceinline__ float hi_part(uint32_t p) { return __uint_as_float(p & 0xFFFF0000u); }
+
+// the three bf16 parts of two values
+__device__ __forceinline__ void split2(float a, float b, uint32_t &h, uint32_t &m, uint32_t &l) {
+  h = bf16_pair(a, b);
+  a -= lo_part(h);
+  b -= hi_part(h);
+  m = bf16_pair(a, b);
+  l = bf16_pair(a - lo_part(m), b - hi_part(m));
 }
 
-// byte offset of element (row, k) in a K-major, 128B-swizzled tile whose
-// rows hold 32 fp32 (one swizzle row each); 8-row groups are 1024 B apart.
-__host__ __device__ __forceinline__ uint32_t sw128_off(uint32_t row, uint32_t k) {
-  return (row >> 3) * 1024u + (row & 7u) * 128u + ((((k >> 2) ^ (row & 7u)) & 7u) << 4) + (k & 3u) * 4u;
-}
+// byte offset of the 16-byte group c (8 values of k) of row r in a K-major
+// tile of 64-byte rows with the 64-byte swizzle
+__device__ __forceinline__ uint32_t sw64_off(uint32_t r, uint32_t c) { return r * 64u + ((c ^ ((r >> 1) & 3u)) << 4); }
 
-// shared-memory matrix descriptor: K-major, SWIZZLE_128B, 8-row groups 1024 B apart
+// shared-memory matrix descriptor: K-major, SWIZZLE_64B, 8-row groups 512 B apart
 __device__ __forceinline__ uint64_t sdesc(uint32_t saddr) {
   uint64_t d = 0;
-  d |= (uint64_t)((saddr & 0x3FFFFu) >> 4);          // start address
-  d |= (uint64_t)1 << 16;                              // leading byte offset (unused for SW128 K-major)
-  d |= (uint64_t)(1024u >> 4) << 32;                   // stride byte offset
-  d |= (uint64_t)1 << 46;                              // descriptor version (tcgen05)
-  d |= (uint64_t)2 << 61;                              // swizzle: 128B
+  d |= (uint64_t)((saddr & 0x3FFFFu) >> 4);  // start address
+  d |= (uint64_t)1 << 16;                    // leading byte offset (unused)
+  d |= (uint64_t)(512u >> 4) << 32;          // stride byte offset
+  d |= (uint64_t)1 << 46;                    // descriptor version (tcgen05)
+  d |= (uint64_t)4 << 61;                    // swizzle: 64B
   return d;
 }
 
-__device__ __forceinline__ void mma_tf32(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+__device__ __forceinline__ void mma_bf16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
                                          uint32_t accum) {
   asm volatile(
       "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-      " tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem_d),
+      " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem_d),
       "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accum));
 }
 
@@ -97,220 +125,20 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
   for (int i = 0; i < 32; i++) v[i] = __uint_as_float(r[i]);
 }
 
-// B-operand image in global memory: for each K-chunk c, the hi tile then the
-// lo tile, each ndet rows x 32 k in the swizzled layout above.
+// B-operand image in global memory: per K-chunk c the h, m and l tiles, each
+// ndet rows x 32 k in the swizzled layout above
 __global__ void k_bprep(const float *__restrict__ A, int ndet, char *__restrict__ img) {
-  const int nchunk = ndet / KC;
-  const size_t tile = (size_t)ndet * 128;
+  const size_t part = (size_t)ndet * 64;
   for (int idx = blockIdx.x * blockDim.x + threadIdx.x; idx < ndet * ndet; idx += gridDim.x * blockDim.x) {
-    int j = idx / ndet, k = idx % ndet;
-    int c = k / KC, kk = k % KC;
-    float a = A[(size_t)j * ndet + k];
-    float h = tf32_round(a);
-    float l = tf32_round(a - h);
-    char *base = img + (size_t)c * 2 * tile;
-    *(float *)(base + sw128_off(j, kk)) = h;
-    *(float *)(base + tile + sw128_off(j, kk)) = l;
+    const int j = idx / ndet, k = idx % ndet;
+    uint32_t h, m, l;
+    split2(A[idx], 0.f, h, m, l);
+    char *p = img + (size_t)(k / KC) * 3 * part + sw64_off(j, (k % KC) >> 3) + (k & 7) * 2;
+    *(uint16_t *)p = (uint16_t)h;
+    *(uint16_t *)(p + part) = (uint16_t)m;
+    *(uint16_t *)(p + 2 * part) = (uint16_t)l;
   }
-  (void)nchunk;
 }
-
-// shared memory: [stage][Ahi 16KB | Alo 16KB | Bhi ndet*128 | Blo ndet*128], 1024-aligned
-// Raw X chunks (32 detectors x 128 samples, 16 KB) are fetched RSTAGE chunks
-// ahead with 4-byte cp.async into a ring in shared memory.  Each thread
-// copies exactly the 32 values of its own sample row, so after its own
-// cp.async.wait_group it can read them back without a CTA barrier.
-constexpr int RSTAGE = 2;
-
-__device__ __forceinline__ void cp_async4(float *dst, const float *src, bool valid) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(smem_u32(dst)), "l"(src),
-               "r"(valid ? 4 : 0)
-               : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() {
-  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
-}
-
-// queue the copy of chunk q (tile, c) of this CTA into raw slot q % RSTAGE;
-// always commits one group so that group counting stays uniform
-__device__ __forceinline__ void prefetch_chunk(const float *__restrict__ X, int64_t ldx, int64_t xs, int64_t ncol,
-                                               int nchunk, int64_t ntile, uint32_t q, float *raw,
-                                               int tid) {
-  const int64_t tile = blockIdx.x + (int64_t)(q / nchunk) * gridDim.x;
-  const int c = (int)(q % nchunk);
-  if (tile < ntile) {
-    const int64_t my = tile * TILE_M + tid;
-    const bool ok = my < ncol;
-    const float *src = X + (int64_t)(c * KC) * ldx + (ok ? my : 0) * xs;
-    float *dst = raw + (size_t)(q % RSTAGE) * KC * TILE_M + tid;
-#pragma unroll
-    for (int kk = 0; kk < KC; kk++) cp_async4(dst + kk * TILE_M, src + (int64_t)kk * ldx, ok);
-  }
-  cp_async_commit();
-}
-
-__global__ void __launch_bounds__(NTHREADS, 1)
-    k_rot_tc(const float *__restrict__ X, int64_t ldx, float *__restrict__ R, int64_t ldr, int ndet,
-             int64_t ncol, const char *__restrict__ bimg, int *__restrict__ err, int64_t mirror_n,
-             int64_t xs, int halve_ends) {
-  extern __shared__ __align__(1024) unsigned char smem_raw[];
-  unsigned char *smem = (unsigned char *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  const uint32_t a_bytes = TILE_M * 128;          // 16 KB
-  const uint32_t b_bytes = (uint32_t)ndet * 128;  // per hi or lo tile
-  const uint32_t stage_bytes = 2 * a_bytes + 2 * b_bytes;
-  float *raw = (float *)(smem + NSTAGE * stage_bytes);
-  __shared__ uint64_t bar_b[NSTAGE], bar_mma[NSTAGE];
-  __shared__ uint32_t tmem_base_sh;
-  __shared__ int abort_sh;
-
-  const int tid = threadIdx.x, warp = tid >> 5;
-  const int nchunk = ndet / KC;
-  const uint32_t ncols = ndet < 32 ? 32u : (uint32_t)ndet;  // power of two by construction
-  const uint32_t idesc = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(ndet >> 3) << 17) |
-                         ((uint32_t)(TILE_M >> 4) << 24);
-
-  if (tid == 0) {
-    for (int s = 0; s < NSTAGE; s++) {
-      mbar_init(&bar_b[s], 1);
-      mbar_init(&bar_mma[s], 1);
-    }
-    abort_sh = 0;
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  if (warp == 0) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
-                     smem_u32(&tmem_base_sh)),
-                 "r"(ncols));
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
-  }
-  asm volatile("tcgen05.fence::before_thread_sync;");
-  __syncthreads();
-  asm volatile("tcgen05.fence::after_thread_sync;");
-  const uint32_t tmem = tmem_base_sh;
-
-  // Control flow is CTA-uniform: only thread 0 waits on mbarriers; the
-  // outcome reaches the other threads through abort_sh and __syncthreads.
-  const int64_t ntile = (ncol + TILE_M - 1) / TILE_M;
-  for (uint32_t q = 0; q < (uint32_t)RSTAGE; q++) prefetch_chunk(X, ldx, xs, ncol, nchunk, ntile, q, raw, tid);
-  uint32_t g = 0;  // chunks issued by this CTA so far
-  for (int64_t tile = blockIdx.x; tile < ntile; tile += gridDim.x) {
-    const int64_t n0 = tile * TILE_M;
-    const int64_t my = n0 + tid;
-    // DCT-I endpoint halving folded into the load (noise.py:710-711)
-    const float hscale = (halve_ends && (my == 0 || my == ncol - 1)) ? 0.5f : 1.0f;
-    for (int c = 0; c < nchunk; c++, g++) {
-      const uint32_t s = g % NSTAGE, use = g / NSTAGE;
-      unsigned char *st = smem + s * stage_bytes;
-      // this thread's sample row: 32 detectors of chunk c from the raw ring,
-      // split into hi / lo; then queue the chunk RSTAGE ahead into that slot
-      float h[KC], l[KC];
-      cp_async_wait<RSTAGE - 1>();
-      const float *rw = raw + (size_t)(g % RSTAGE) * KC * TILE_M + tid;
-#pragma unroll
-      for (int kk = 0; kk < KC; kk++) {
-        float x = rw[kk * TILE_M] * hscale;
-        h[kk] = tf32_round(x);
-        l[kk] = tf32_round(x - h[kk]);
-      }
-      prefetch_chunk(X, ldx, xs, ncol, nchunk, ntile, g + RSTAGE, raw, tid);
-      if (tid == 0) {
-        // stage s is free once the MMAs of chunk g-2 have completed
-        if (g >= NSTAGE && !mbar_wait(&bar_mma[s], (use - 1) & 1)) {
-          abort_sh = 1;
-        } else {
-          mbar_expect_tx(&bar_b[s], 2 * b_bytes);
-          bulk_g2s(st + 2 * a_bytes, bimg + (size_t)c * 2 * b_bytes, 2 * b_bytes, &bar_b[s]);
-        }
-      }
-      __syncthreads();
-      if (abort_sh) break;
-      unsigned char *ah = st, *al = st + a_bytes;
-#pragma unroll
-      for (int q = 0; q < KC / 4; q++) {
-        uint32_t off = sw128_off(tid, 4 * q);
-        *(float4 *)(ah + off) = make_float4(h[4 * q], h[4 * q + 1], h[4 * q + 2], h[4 * q + 3]);
-        *(float4 *)(al + off) = make_float4(l[4 * q], l[4 * q + 1], l[4 * q + 2], l[4 * q + 3]);
-      }
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-      __syncthreads();
-      if (tid == 0) {
-        if (!mbar_wait(&bar_b[s], use & 1)) {
-          abort_sh = 1;  // seen by everyone at the next __syncthreads
-        } else {
-          asm volatile("tcgen05.fence::after_thread_sync;");
-          const uint32_t sa_h = smem_u32(ah), sa_l = smem_u32(al);
-          const uint32_t sb_h = smem_u32(st + 2 * a_bytes), sb_l = sb_h + b_bytes;
-#pragma unroll
-          for (int k8 = 0; k8 < KC / 8; k8++) {
-            const uint32_t ko = k8 * 32;  // 8 tf32 = 32 bytes along K
-            const uint32_t acc0 = (c == 0 && k8 == 0) ? 0u : 1u;
-            mma_tf32(tmem, sdesc(sa_h + ko), sdesc(sb_h + ko), idesc, acc0);
-            mma_tf32(tmem, sdesc(sa_l + ko), sdesc(sb_h + ko), idesc, 1u);
-            mma_tf32(tmem, sdesc(sa_h + ko), sdesc(sb_l + ko), idesc, 1u);
-          }
-          mma_commit(&bar_mma[s]);
-        }
-      }
-    }
-    // epilogue: wait for the tile's last chunk, TMEM -> registers -> R
-    if (tid == 0 && !abort_sh) {
-      const uint32_t sl = (g - 1) % NSTAGE, ul = (g - 1) / NSTAGE;
-      if (!mbar_wait(&bar_mma[sl], ul & 1)) abort_sh = 1;
-    }
-    __syncthreads();
-    if (abort_sh) break;
-    asm volatile("tcgen05.fence::after_thread_sync;");
-    const uint32_t lane_base = (uint32_t)(warp * 32) << 16;
-    for (int c0 = 0; c0 < ndet; c0 += 32) {
-      float v[32];
-      tmem_ld32(tmem + lane_base + (uint32_t)c0, v);
-      if (my < ncol) {
-#pragma unroll
-        for (int j = 0; j < 32; j++) __stcs(R + (int64_t)(c0 + j) * ldr + my, v[j]);
-        // even extension for the DCT-I that follows: R[., mirror_n - my] = R[., my]
-        if (mirror_n > 0 && my >= 1 && my <= ncol - 2) {
-#pragma unroll
-          for (int j = 0; j < 32; j++) __stcs(R + (int64_t)(c0 + j) * ldr + (mirror_n - my), v[j]);
-        }
-      }
-    }
-    asm volatile("tcgen05.fence::before_thread_sync;");
-    __syncthreads();
-  }
-  cp_async_wait<0>();  // no copy into this CTA's shared memory outlives it
-  if (abort_sh && tid == 0) {
-    atomicExch(err, 1);
-    // bounded drain of MMAs possibly still in flight before freeing tensor memory
-    for (uint32_t q = (g > NSTAGE ? g - NSTAGE : 0); q < g; q++)
-      (void)mbar_wait(&bar_mma[q % NSTAGE], (q / NSTAGE) & 1);
-  }
-  asm volatile("tcgen05.fence::before_thread_sync;");
-  __syncthreads();
-  if (warp == 0)
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(ncols));
-}
-
-// ---- warp-specialised version ---------------------------------------------
-// The same tiles, products and operand images, with the roles split so that
-// no CTA-wide barrier sits in the main loop:
-//   warps 0-3 (split): thread t owns sample row t of every tile; it splits its
-//     32 values of a K-chunk into hi / lo and writes them into the chunk's
-//     A stage, then arrives on full_a[stage];
-//   warp 4, lane 0 (MMA): bulk-copies the chunk's B image into the stage
-//     (full_b[stage]), waits for both halves, issues the 12 MMAs and commits
-//     them to mma_done[stage] (which frees the stage for chunk g + 2); after
-//     a tile's last chunk it commits to acc_full[buffer];
-//   warps 5-8 (epilogue): tensor memory holds two accumulators (2 x ndet
-//     columns), so while the MMAs of tile i + 1 run, these warps read tile i
-//     (warp w reads TMEM lanes 32 (w % 4) ..) and store it, then arrive on
-//     acc_empty[buffer].
-// Every wait is bounded and also polls the CTA's abort flag, so a timeout in
-// one role ends all of them; the MMA thread then drains its outstanding
-// MMAs (bounded) before the tensor memory is freed.
-constexpr int WS_SPLIT = 4, WS_EPI = 4;
-constexpr int WS_THREADS = (WS_SPLIT + 1 + WS_EPI) * 32;
 
 __device__ __forceinline__ bool ws_wait(uint64_t *bar, uint32_t parity, volatile int *abort_flag) {
   for (uint32_t i = 0; i < mk::SPIN_LIMIT; i++) {
@@ -328,38 +156,22 @@ __device__ __forceinline__ int job_at(const mk::RotJob *jobs, int njobs, int64_t
   return cur;
 }
 
-// queue the copy of chunk q of this CTA (tile blockIdx.x + (q / nchunk) *
-// gridDim.x, K-chunk q % nchunk) into raw slot q % RSTAGE; always commits one
-// group so that group counting stays uniform
-__device__ __forceinline__ void prefetch_job(const mk::RotJob *jobs, int njobs, int &pcur, int64_t xs, int nchunk,
-                                             int64_t ntile, uint32_t q, float *raw, int tid) {
-  const int64_t tile = blockIdx.x + (int64_t)(q / nchunk) * gridDim.x;
-  const int c = (int)(q % nchunk);
-  if (tile < ntile) {
-    pcur = job_at(jobs, njobs, tile, pcur);
-    const mk::RotJob &J = jobs[pcur];
-    const int64_t my = (tile - J.tile0) * TILE_M + tid;
-    const bool ok = my < J.ncol;
-    const float *src = J.X + (int64_t)(c * KC) * J.ldx + (ok ? my : 0) * xs;
-    float *dst = raw + (size_t)(q % RSTAGE) * KC * TILE_M + tid;
-#pragma unroll
-    for (int kk = 0; kk < KC; kk++) cp_async4(dst + kk * TILE_M, src + (int64_t)kk * J.ldx, ok);
-  }
-  cp_async_commit();
-}
+// plain (R may be X) streaming load; zero past the TOD's end
+__device__ __forceinline__ float load1(const float *p, bool ok) { return ok ? __ldcs(p) : 0.f; }
 
+// One item = MT tiles of 128 samples of one job (RotJob::tile0 counts items).
 // `jobs` (device memory, sorted by tile0) lists the TODs of a grouped launch,
 // all with ndet detectors; for one TOD it is null and `j0` is that TOD.
 // mirror_n, xs and halve_ends apply to single-TOD launches (0, 1, 0 in groups).
-__global__ void __launch_bounds__(WS_THREADS, 1)
-    k_rot_tc_ws(const mk::RotJob *__restrict__ jobs_in, int njobs, const mk::RotJob j0, int64_t ntile, int ndet,
-                int *__restrict__ err, int64_t mirror_n, int64_t xs, int halve_ends) {
+template <int MT>
+__global__ void __launch_bounds__((8 * MT + 1) * 32, 3 - MT)
+    k_rot_tc(const mk::RotJob *jobs_in, int njobs, const mk::RotJob j0, int64_t nitem, int ndet, int nbuf,
+             uint32_t tcols, int *err, int64_t mirror_n, int64_t xs, int halve_ends) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char *smem = (unsigned char *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  const uint32_t a_bytes = TILE_M * 128;
-  const uint32_t b_bytes = (uint32_t)ndet * 128;
-  const uint32_t stage_bytes = 2 * a_bytes + 2 * b_bytes;
-  float *raw = (float *)(smem + NSTAGE * stage_bytes);
+  constexpr int NSPLIT = 4 * MT, NEPI = 4 * MT;
+  const uint32_t b_part = (uint32_t)ndet * 64;
+  const uint32_t stage_bytes = MT * A_TILE + 3 * b_part;
   __shared__ uint64_t full_a[NSTAGE], full_b[NSTAGE], mma_done[NSTAGE], acc_full[2], acc_empty[2];
   __shared__ uint32_t tmem_base_sh;
   __shared__ int abort_sh;
@@ -369,82 +181,100 @@ __global__ void __launch_bounds__(WS_THREADS, 1)
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int nchunk = ndet / KC;
-  const uint32_t ncols = 2u * (ndet < 32 ? 32u : (uint32_t)ndet);  // two accumulators, a power of two
-  const uint32_t idesc = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(ndet >> 3) << 17) |
-                         ((uint32_t)(TILE_M >> 4) << 24);
   if (tid == 0) {
     for (int s = 0; s < NSTAGE; s++) {
-      mbar_init(&full_a[s], WS_SPLIT * 32);
+      mbar_init(&full_a[s], NSPLIT * 32);
       mbar_init(&full_b[s], 1);
       mbar_init(&mma_done[s], 1);
     }
     for (int b = 0; b < 2; b++) {
       mbar_init(&acc_full[b], 1);
-      mbar_init(&acc_empty[b], WS_EPI * 32);
+      mbar_init(&acc_empty[b], NEPI * 32);
     }
     abort_sh = 0;
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    mk::mbar_init_fence();
   }
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
                      smem_u32(&tmem_base_sh)),
-                 "r"(ncols));
+                 "r"(tcols));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
   asm volatile("tcgen05.fence::before_thread_sync;");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;");
   const uint32_t tmem = tmem_base_sh;
-  uint32_t g_issued = 0;  // MMA thread: chunks whose MMAs were committed
+  uint32_t g_copied = 0, g_issued = 0;  // MMA thread: chunks whose image copy / MMAs were issued
 
-  if (warp < WS_SPLIT) {
-    // ---- split role ----
-    int pcur = 0, cur = 0;
-    for (uint32_t q = 0; q < (uint32_t)RSTAGE; q++) prefetch_job(jobs, njobs, pcur, xs, nchunk, ntile, q, raw, tid);
+  if (warp < NSPLIT) {
+    // ---- split role: thread = sample; the values of the next chunk are
+    // loaded into the registers that the current one leaves
+    const int mt = warp >> 2, row = (warp & 3) * 32 + lane;
+    int cur = 0;
     uint32_t g = 0;
-    for (int64_t tile = blockIdx.x; tile < ntile && !*abort_flag; tile += gridDim.x) {
-      cur = job_at(jobs, njobs, tile, cur);
-      const int64_t my = (tile - jobs[cur].tile0) * TILE_M + tid, ncol = jobs[cur].ncol;
-      const float hscale = (halve_ends && (my == 0 || my == ncol - 1)) ? 0.5f : 1.0f;
+    float v[KC];
+    int64_t item = blockIdx.x, ldx = 0;
+    const float *src = nullptr;
+    bool ok = false;
+    float hs = 1.f, hs_next = 1.f;
+    auto open = [&]() {  // this thread's sample of `item`
+      cur = job_at(jobs, njobs, item, cur);
+      const mk::RotJob &J = jobs[cur];
+      const int64_t my = ((item - J.tile0) * MT + mt) * TILE_M + row;
+      ok = my < J.ncol;
+      ldx = J.ldx;
+      src = J.X + (ok ? my : 0) * xs;
+      hs_next = halve_ends && (my == 0 || my == J.ncol - 1) ? 0.5f : 1.0f;
+    };
+    if (item < nitem) {
+      open();
+#pragma unroll
+      for (int kk = 0; kk < KC; kk++) v[kk] = load1(src + kk * ldx, ok);
+    }
+    for (bool stop = false; item < nitem && !stop && !*abort_flag;) {
+      hs = hs_next;
       for (int c = 0; c < nchunk; c++, g++) {
-        const uint32_t s = g % NSTAGE, use = g / NSTAGE;
-        float h[KC], l[KC];
-        cp_async_wait<RSTAGE - 1>();
-        const float *rw = raw + (size_t)(g % RSTAGE) * KC * TILE_M + tid;
-#pragma unroll
-        for (int kk = 0; kk < KC; kk++) {
-          const float x = rw[kk * TILE_M] * hscale;
-          h[kk] = tf32_round(x);
-          l[kk] = tf32_round(x - h[kk]);
+        const uint32_t s = g % NSTAGE;
+        if (g >= NSTAGE && !ws_wait(&mma_done[s], (g / NSTAGE - 1) & 1, abort_flag)) {
+          stop = true;
+          break;
         }
-        prefetch_job(jobs, njobs, pcur, xs, nchunk, ntile, g + RSTAGE, raw, tid);
-        if (g >= NSTAGE && !ws_wait(&mma_done[s], (use - 1) & 1, abort_flag)) break;
-        unsigned char *ah = smem + s * stage_bytes, *al = ah + a_bytes;
-#pragma unroll
-        for (int q = 0; q < KC / 4; q++) {
-          const uint32_t off = sw128_off(tid, 4 * q);
-          *(float4 *)(ah + off) = make_float4(h[4 * q], h[4 * q + 1], h[4 * q + 2], h[4 * q + 3]);
-          *(float4 *)(al + off) = make_float4(l[4 * q], l[4 * q + 1], l[4 * q + 2], l[4 * q + 3]);
+        if (c + 1 < nchunk) {
+          src += KC * ldx;
+        } else {
+          item += gridDim.x;
+          ok = false;
+          if (item < nitem) open();
         }
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        unsigned char *at = smem + s * stage_bytes + mt * A_TILE;
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+          uint32_t h[4], m[4], l[4];
+#pragma unroll
+          for (int i = 0; i < 4; i++) split2(v[8 * q + 2 * i] * hs, v[8 * q + 2 * i + 1] * hs, h[i], m[i], l[i]);
+#pragma unroll
+          for (int i = 0; i < 8; i++) v[8 * q + i] = load1(src + (8 * q + i) * ldx, ok);
+          const uint32_t off = sw64_off(row, q);
+          *(uint4 *)(at + off) = make_uint4(h[0], h[1], h[2], h[3]);
+          *(uint4 *)(at + A_PART + off) = make_uint4(m[0], m[1], m[2], m[3]);
+          *(uint4 *)(at + 2 * A_PART + off) = make_uint4(l[0], l[1], l[2], l[3]);
+        }
+        mk::fence_proxy_async_smem();
         mk::mbar_arrive(&full_a[s]);
       }
     }
-    cp_async_wait<0>();  // no copy into this CTA's shared memory outlives it
-  } else if (warp == WS_SPLIT) {
-    // ---- MMA role (one thread) ----
+  } else if (warp == NSPLIT + NEPI) {
+    // ---- image copies and MMAs (one thread)
     if (lane == 0) {
-      uint32_t g = 0;
-      int64_t it = 0;
+      const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(ndet >> 3) << 17) |
+                             ((uint32_t)(TILE_M >> 4) << 24);
+      uint32_t g = 0, it = 0;
       int cur = 0;
-      for (int64_t tile = blockIdx.x; tile < ntile && !*abort_flag; tile += gridDim.x, it++) {
-        cur = job_at(jobs, njobs, tile, cur);
+      bool ok = true;
+      for (int64_t item = blockIdx.x; item < nitem && ok && !*abort_flag; item += gridDim.x, it++) {
+        cur = job_at(jobs, njobs, item, cur);
         const char *bimg = jobs[cur].bimg;
-        const uint32_t ab = (uint32_t)(it & 1), au = (uint32_t)(it >> 1);
-        if (it >= 2 && !ws_wait(&acc_empty[ab], (au - 1) & 1, abort_flag)) break;
-        asm volatile("tcgen05.fence::after_thread_sync;");
-        const uint32_t dacc = tmem + ab * (ncols / 2);
-        bool ok = true;
+        const uint32_t ab = nbuf == 2 ? it & 1 : 0, au = nbuf == 2 ? it >> 1 : it;
         for (int c = 0; c < nchunk; c++, g++) {
           const uint32_t s = g % NSTAGE, use = g / NSTAGE;
           unsigned char *st = smem + s * stage_bytes;
@@ -452,22 +282,32 @@ __global__ void __launch_bounds__(WS_THREADS, 1)
             ok = false;
             break;
           }
-          mbar_expect_tx(&full_b[s], 2 * b_bytes);
-          bulk_g2s(st + 2 * a_bytes, bimg + (size_t)c * 2 * b_bytes, 2 * b_bytes, &full_b[s]);
-          if (!ws_wait(&full_b[s], use & 1, abort_flag) || !ws_wait(&full_a[s], use & 1, abort_flag)) {
+          mbar_expect_tx(&full_b[s], 3 * b_part);
+          bulk_g2s(st + MT * A_TILE, bimg + (size_t)c * 3 * b_part, 3 * b_part, &full_b[s]);
+          g_copied = g + 1;
+          if (c == 0 && au >= 1 && !ws_wait(&acc_empty[ab], (au - 1) & 1, abort_flag)) ok = false;
+          if (!ok || !ws_wait(&full_b[s], use & 1, abort_flag) || !ws_wait(&full_a[s], use & 1, abort_flag)) {
             ok = false;
             break;
           }
           asm volatile("tcgen05.fence::after_thread_sync;");
-          const uint32_t sa_h = smem_u32(st), sa_l = sa_h + a_bytes;
-          const uint32_t sb_h = smem_u32(st + 2 * a_bytes), sb_l = sb_h + b_bytes;
+          const uint32_t sb = smem_u32(st + MT * A_TILE);
 #pragma unroll
-          for (int k8 = 0; k8 < KC / 8; k8++) {
-            const uint32_t ko = k8 * 32;
-            const uint32_t acc0 = (c == 0 && k8 == 0) ? 0u : 1u;
-            mma_tf32(dacc, sdesc(sa_h + ko), sdesc(sb_h + ko), idesc, acc0);
-            mma_tf32(dacc, sdesc(sa_l + ko), sdesc(sb_h + ko), idesc, 1u);
-            mma_tf32(dacc, sdesc(sa_h + ko), sdesc(sb_l + ko), idesc, 1u);
+          for (int mt = 0; mt < MT; mt++) {
+            const uint32_t sa = smem_u32(st) + mt * A_TILE;
+            const uint32_t dacc = tmem + (ab * MT + mt) * (uint32_t)ndet;
+#pragma unroll
+            for (int k16 = 0; k16 < KC / 16; k16++) {
+              const uint32_t ko = k16 * 32;
+              const uint64_t ah = sdesc(sa + ko), am = sdesc(sa + A_PART + ko), al = sdesc(sa + 2 * A_PART + ko);
+              const uint64_t bh = sdesc(sb + ko), bm = sdesc(sb + b_part + ko), bl = sdesc(sb + 2 * b_part + ko);
+              mma_bf16(dacc, ah, bl, idesc, c == 0 && k16 == 0 ? 0u : 1u);
+              mma_bf16(dacc, al, bh, idesc, 1u);
+              mma_bf16(dacc, am, bm, idesc, 1u);
+              mma_bf16(dacc, ah, bm, idesc, 1u);
+              mma_bf16(dacc, am, bh, idesc, 1u);
+              mma_bf16(dacc, ah, bh, idesc, 1u);
+            }
           }
           mma_commit(&mma_done[s]);
           g_issued = g + 1;
@@ -477,29 +317,31 @@ __global__ void __launch_bounds__(WS_THREADS, 1)
       }
     }
   } else {
-    // ---- epilogue role ----
+    // ---- epilogue role
+    const int ew = warp - NSPLIT, mt = ew >> 2;
     const int q = warp & 3;  // TMEM lane quarter this warp may access
     const int row = 32 * q + lane;
-    int64_t it = 0;
+    uint32_t it = 0;
     int cur = 0;
-    for (int64_t tile = blockIdx.x; tile < ntile; tile += gridDim.x, it++) {
-      cur = job_at(jobs, njobs, tile, cur);
-      const uint32_t ab = (uint32_t)(it & 1), au = (uint32_t)(it >> 1);
+    for (int64_t item = blockIdx.x; item < nitem; item += gridDim.x, it++) {
+      cur = job_at(jobs, njobs, item, cur);
+      const uint32_t ab = nbuf == 2 ? it & 1 : 0, au = nbuf == 2 ? it >> 1 : it;
       // every lane waits; the warp goes on only if all of them saw the
       // phase complete (tcgen05.ld below needs the whole warp converged)
       const bool okw = ws_wait(&acc_full[ab], au & 1, abort_flag);
       if (!__all_sync(0xffffffffu, okw)) break;
       asm volatile("tcgen05.fence::after_thread_sync;");
       const mk::RotJob &J = jobs[cur];
-      const int64_t my = (tile - J.tile0) * TILE_M + row, ncol = J.ncol, ldr = J.ldr;
+      const int64_t my = ((item - J.tile0) * MT + mt) * TILE_M + row, ncol = J.ncol, ldr = J.ldr;
       float *R = J.R;
-      const uint32_t base = tmem + ((uint32_t)(32 * q) << 16) + ab * (ncols / 2);
+      const uint32_t base = tmem + ((uint32_t)(32 * q) << 16) + (ab * MT + mt) * (uint32_t)ndet;
       for (int c0 = 0; c0 < ndet; c0 += 32) {
         float v[32];
         tmem_ld32(base + (uint32_t)c0, v);
         if (my < ncol) {
 #pragma unroll
           for (int j = 0; j < 32; j++) __stcs(R + (int64_t)(c0 + j) * ldr + my, v[j]);
+          // even extension for the DCT-I that follows: R[., mirror_n - my] = R[., my]
           if (mirror_n > 0 && my >= 1 && my <= ncol - 2) {
 #pragma unroll
             for (int j = 0; j < 32; j++) __stcs(R + (int64_t)(c0 + j) * ldr + (mirror_n - my), v[j]);
@@ -511,32 +353,46 @@ __global__ void __launch_bounds__(WS_THREADS, 1)
     }
   }
   __syncthreads();
-  if (*abort_flag && tid == WS_SPLIT * 32) {
+  if (*abort_flag && tid == (NSPLIT + NEPI) * 32) {
     atomicExch(err, 1);
-    // bounded drain of the MMAs this thread issued before freeing tensor memory
+    // bounded waits for the copies and MMAs this thread issued
+    for (uint32_t g = (g_copied > NSTAGE ? g_copied - NSTAGE : 0); g < g_copied; g++)
+      (void)mbar_wait(&full_b[g % NSTAGE], (g / NSTAGE) & 1);
     for (uint32_t g = (g_issued > NSTAGE ? g_issued - NSTAGE : 0); g < g_issued; g++)
       (void)mbar_wait(&mma_done[g % NSTAGE], (g / NSTAGE) & 1);
   }
   asm volatile("tcgen05.fence::before_thread_sync;");
   __syncthreads();
   if (warp == 0)
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(ncols));
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(tcols));
 }
 
-size_t ws_smem_bytes(int nd) {
-  const size_t stage = 2 * (size_t)TILE_M * 128 + 2 * (size_t)nd * 128;
-  return NSTAGE * stage + (size_t)RSTAGE * KC * TILE_M * sizeof(float) + 1024;
-}
+int tiles_per_item(int64_t nrow) { return nrow == 256 ? 2 : 1; }
 
-int ws_prepare(size_t smem) {
-  static int attr_ws[64] = {0};
+template <int MT>
+int launch(const mk::RotJob *jobs, int njobs, const mk::RotJob &j0, int64_t nitem, int nd, int *err, cudaStream_t st,
+           int64_t mirror_n, int64_t xs, int halve_ends) {
+  const size_t smem = NSTAGE * ((size_t)MT * A_TILE + 3 * (size_t)nd * 64) + 1024;
+  static int attr[64] = {0};
   int dev = 0;
   MK_CUDA(cudaGetDevice(&dev));
-  if (dev >= 0 && dev < 64 && attr_ws[dev] < (int)smem) {
-    MK_CUDA(cudaFuncSetAttribute(k_rot_tc_ws, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    attr_ws[dev] = (int)smem;
+  if (dev >= 0 && dev < 64 && attr[dev] < (int)smem) {
+    MK_CUDA(cudaFuncSetAttribute(k_rot_tc<MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    attr[dev] = (int)smem;
   }
-  return MK_OK;
+  const int nbuf = MT * nd * 2 <= 512 / (MT == 1 ? 2 : 1) ? 2 : 1;  // accumulators; MT = 1: two CTAs per SM
+  const uint32_t tcols = (uint32_t)(MT * nd * nbuf);
+  int64_t grid = (int64_t)mk::sm_count() * (MT == 1 ? 2 : 1);
+  if (grid > nitem) grid = nitem;
+  k_rot_tc<MT><<<(unsigned)grid, (8 * MT + 1) * 32, smem, st>>>(jobs, njobs, j0, nitem, nd, nbuf, tcols, err, mirror_n,
+                                                                xs, halve_ends);
+  return mk::launch_status("rot_tc");
+}
+
+int launch_nd(const mk::RotJob *jobs, int njobs, const mk::RotJob &j0, int64_t nitem, int nd, int *err,
+              cudaStream_t st, int64_t mirror_n, int64_t xs, int halve_ends) {
+  if (tiles_per_item(nd) == 2) return launch<2>(jobs, njobs, j0, nitem, nd, err, st, mirror_n, xs, halve_ends);
+  return launch<1>(jobs, njobs, j0, nitem, nd, err, st, mirror_n, xs, halve_ends);
 }
 
 }  // namespace
@@ -547,63 +403,26 @@ bool rot_tc_supported(int64_t nrow) {
   return nrow == 32 || nrow == 64 || nrow == 128 || nrow == 256;
 }
 
-size_t rot_tc_bimg_bytes(int64_t nrow) { return (size_t)nrow * (size_t)nrow * 8; }
+size_t rot_tc_bimg_bytes(int64_t nrow) { return (size_t)nrow * (size_t)nrow * 6; }
+
+int64_t rot_tc_items(int64_t nrow, int64_t ncol) {
+  const int64_t per = (int64_t)TILE_M * tiles_per_item(nrow);
+  return (ncol + per - 1) / per;
+}
 
 int rot_tc_f32(const float *A, const float *X, int64_t ldx, float *R, int64_t ldr, int64_t nrow,
                int64_t ncol, void *bimg, int *err, cudaStream_t st, int64_t mirror_n, int64_t x_stride,
                int halve_ends) {
-  MK_CHECK_ARG(rot_tc_supported(nrow), "tensor-core rotation supports ndet in {32,64,128,256}, got %lld",
-               (long long)nrow);
-  MK_CHECK_ARG(bimg && err && ((uintptr_t)bimg % 16) == 0, "tensor-core rotation: bad scratch");
   MK_CHECK_ARG(mirror_n == 0 || (mirror_n == 2 * (ncol - 1) && ldr >= mirror_n),
                "tensor-core rotation: bad mirror extent");
   MK_CHECK_ARG(x_stride == 1 || x_stride == 2, "tensor-core rotation: element stride must be 1 or 2");
+  MK_CHECK_ARG(err, "tensor-core rotation: bad scratch");
   if (ncol <= 0) return MK_OK;
-  const int nd = (int)nrow;
-  k_bprep<<<(nd * nd + 255) / 256, 256, 0, st>>>(A, nd, (char *)bimg);
-  const size_t stage = 2 * (size_t)TILE_M * 128 + 2 * (size_t)nd * 128;
-  const size_t smem = NSTAGE * stage + (size_t)RSTAGE * KC * TILE_M * sizeof(float) + 1024;
-  static int attr_set[64] = {0};
-  int dev = 0;
-  MK_CUDA(cudaGetDevice(&dev));
-  if (dev >= 0 && dev < 64 && attr_set[dev] < (int)smem) {
-    MK_CUDA(cudaFuncSetAttribute(k_rot_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    attr_set[dev] = (int)smem;
-  }
-  int64_t ntile = (ncol + TILE_M - 1) / TILE_M;
-  // one TOD: the single-role kernel, measured 10 % faster than the
-  // warp-specialised one on a 256 x 130,978 TOD (both wait on the loads of
-  // X: two 16 KB chunks in flight per SM); MINKASI_GB300_ROT_TC_WS=1 selects
-  // the warp-specialised kernel, which the grouped (many-TOD) launch uses
-  static const bool ws = [] {
-    const char *e = getenv("MINKASI_GB300_ROT_TC_WS");
-    return e && e[0] == '1';
-  }();
-  if (ws) {
-    const size_t wsmem = ws_smem_bytes(nd);
-    int rc = ws_prepare(wsmem);
-    if (rc) return rc;
-    RotJob j0{X, R, (const char *)bimg, ldx, ldr, ncol, 0};
-    // one CTA per SM: its two accumulators take up to all 512 TMEM columns
-    int64_t grid = (int64_t)sm_count();
-    if (grid > ntile) grid = ntile;
-    k_rot_tc_ws<<<(unsigned)grid, WS_THREADS, wsmem, st>>>(nullptr, 1, j0, ntile, nd, err, mirror_n, x_stride,
-                                                           halve_ends);
-    return launch_status("rot_tc_f32");
-  }
-  int per_sm = (int)(220 * 1024 / smem);
-  if (per_sm < 1) per_sm = 1;
-  if (per_sm > 2) per_sm = 2;  // tensor memory: <= 2 x 256 columns per SM
-  int64_t grid = (int64_t)sm_count() * per_sm;
-  if (grid > ntile) grid = ntile;
-  k_rot_tc<<<(unsigned)grid, NTHREADS, smem, st>>>(X, ldx, R, ldr, nd, ncol, (const char *)bimg, err,
-                                                   mirror_n, x_stride, halve_ends);
-  return launch_status("rot_tc_f32");
+  const int rc = rot_tc_bprep(A, nrow, bimg, st);
+  if (rc) return rc;
+  const RotJob j0{X, R, (const char *)bimg, ldx, ldr, ncol, 0};
+  return launch_nd(nullptr, 1, j0, rot_tc_items(nrow, ncol), (int)nrow, err, st, mirror_n, x_stride, halve_ends);
 }
-
-}  // namespace mk
-
-namespace mk {
 
 int rot_tc_bprep(const float *A, int64_t nrow, void *bimg, cudaStream_t st) {
   MK_CHECK_ARG(rot_tc_supported(nrow), "tensor-core rotation supports ndet in {32,64,128,256}, got %lld",
@@ -614,20 +433,12 @@ int rot_tc_bprep(const float *A, int64_t nrow, void *bimg, cudaStream_t st) {
   return launch_status("rot_tc_bprep");
 }
 
-int rot_tc_group(const RotJob *jobs_dev, int njobs, int64_t ntile, int64_t nrow, int *err, cudaStream_t st) {
+int rot_tc_group(const RotJob *jobs_dev, int njobs, int64_t nitem, int64_t nrow, int *err, cudaStream_t st) {
   MK_CHECK_ARG(rot_tc_supported(nrow), "tensor-core rotation supports ndet in {32,64,128,256}, got %lld",
                (long long)nrow);
   MK_CHECK_ARG(jobs_dev && njobs >= 1 && err, "tensor-core rotation group: bad arguments");
-  if (ntile <= 0) return MK_OK;
-  const int nd = (int)nrow;
-  const size_t wsmem = ws_smem_bytes(nd);
-  int rc = ws_prepare(wsmem);
-  if (rc) return rc;
-  int64_t grid = (int64_t)sm_count();
-  if (grid > ntile) grid = ntile;
-  RotJob none{};
-  k_rot_tc_ws<<<(unsigned)grid, WS_THREADS, wsmem, st>>>(jobs_dev, njobs, none, ntile, nd, err, 0, 1, 0);
-  return launch_status("rot_tc_group");
+  if (nitem <= 0) return MK_OK;
+  return launch_nd(jobs_dev, njobs, RotJob{}, nitem, (int)nrow, err, st, 0, 1, 0);
 }
 
 }  // namespace mk

@@ -11,7 +11,7 @@ Bluestein's algorithm) with random data, and reports per kernel the time and, fo
 algorithmic GB/s (4 B pixel index + one sample per sample; the map is
 L2-resident).  Rotations report their relative error against cuBLAS on the
 FP64 / FP32 units and their TF/s counted as 2 ndet^2 ndata flops
-(3 split products for the tensor-core 3xTF32 kernel are not counted).
+(the split products of the tensor-core kernels are not counted).
 Prints one JSON object.  This is also the command the ncu captures use.
 """
 from __future__ import annotations

@@ -292,7 +292,7 @@ def run_pcg_mixed(b: Mapset, x0: Mapset, tods: TodVec, precon=None, tol: float =
 
     mode="reliable" (default): PCG whose vectors, dot products and scalars are
     FP64 but whose operator applications run in FP32 (FP32 projections, FP32
-    DCT/filter, 3xTF32 tensor-core rotations); every ``replace_every``
+    DCT/filter, tensor-core rotations of three bf16 parts); every ``replace_every``
     iterations, and whenever the recursive residual claims convergence, the
     residual is replaced by the FP64 true residual b - A64 x (an FP64
     operator application, as costly as 10-25 FP32 iterations on GB300; the

@@ -38,6 +38,30 @@ def test_tc_rotation_matches_fp64(K, ndet, ncol):
     assert rel(R2, ref) < 5e-6
 
 
+@pytest.mark.parametrize("ndet", [32, 64, 128, 256])
+@pytest.mark.parametrize("ncol", [2, 127, 129, 255, 257, 40_001])
+def test_tc_rotation_tile_edges_and_nonfinite(K, ndet, ncol):
+    """Around the tiles of 128 samples and the items of two tiles, more items
+    than CTAs, entries over the FP32 range, and NaN / infinity in one sample
+    each (all of its outputs become NaN, every other sample stays).  Bound per
+    sample: each output is accumulated in 6 ndet / 16 <= 96 steps, each off by
+    at most 2^-23 of a partial sum (taken as at most twice the largest
+    output): 2.3e-5."""
+    rng = np.random.default_rng(ndet + ncol)
+    A = rng.standard_normal((ndet, ndet)).astype(np.float32)
+    X = (rng.standard_normal((ndet, ncol)) * 10.0 ** rng.integers(-20, 20, size=ncol)[None, :]).astype(np.float32)
+    ref = A.astype(np.float64) @ X.astype(np.float64)
+    plan = K.NoisePlan(ndet, ncol, torch.float32)
+    At = torch.from_numpy(A).to(cuda)
+    R = plan.rotate(At, torch.from_numpy(X).to(cuda), rot_mode=2).cpu().numpy()
+    assert (np.abs(R - ref).max(0) <= 2.3e-5 * np.abs(ref).max(0)).all()
+    X[ndet // 3, 0], X[ndet // 2, ncol - 1] = np.nan, np.inf
+    R2 = plan.rotate(At, torch.from_numpy(X).to(cuda), rot_mode=2).cpu().numpy()
+    assert np.isnan(R2[:, 0]).all() and np.isnan(R2[:, ncol - 1]).all()
+    assert np.array_equal(R2[:, 1:ncol - 1], R[:, 1:ncol - 1])
+    assert plan.status() == 0
+
+
 def test_tc_apply_noise_matches_golden(K, gold):
     g = gold("noise.npz")
     x = g["x"]
