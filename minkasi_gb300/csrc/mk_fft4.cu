@@ -28,6 +28,7 @@
 #define MK_FFT4_NTHI MK_FFT4_NT16
 #define MK_FFT4_NTLO MK_FFT4_NT8
 #define MK_FFT4_MINBLO MK_FFT4_MINB8
+#define MK_FFT4_SMOOTH 1
 #include "mk_fft4_kern.cuh"
 
 namespace mk {
@@ -175,10 +176,20 @@ struct Cd {
   double x, y;
 };
 
-Cd unit(double num, double den) {
-  // exp(-2 pi i num / den) in double
-  const double a = 2.0 * M_PI * num / den;
-  return {std::cos(a), -std::sin(a)};
+Cd unit(int64_t t, int64_t L) {
+  // exp(-2 pi i t / L) in double, the angle reduced to an eighth of the circle
+  // in integers (its rounding would otherwise exceed the result's)
+  t %= L;
+  if (t < 0) t += L;
+  const bool neg = 2 * t > L;
+  if (neg) t = L - t;
+  const bool half = 4 * t > L;
+  const int64_t u = half ? L - 2 * t : 2 * t;  // angle = pi u / L, u <= L / 2
+  const bool swap = 4 * u > L;
+  const double a = M_PI * (swap ? 0.5 * (double)(L - 2 * u) : (double)u) / (double)L;
+  double c = std::cos(a), s = std::sin(a);
+  if (swap) std::swap(c, s);
+  return {half ? -c : c, neg ? s : -s};
 }
 
 // a complex table entry at byte offset `off`, index i: float2 or double2
@@ -187,6 +198,18 @@ void put(char *base, size_t off, int64_t i, Cd v, bool f64) {
     reinterpret_cast<double2 *>(base + off)[i] = make_double2(v.x, v.y);
   } else {
     reinterpret_cast<float2 *>(base + off)[i] = make_float2((float)v.x, (float)v.y);
+  }
+}
+
+// a fixed-point twiddle: 2^62 (x, y), each as a high and a signed low word
+void put_i64(char *base, size_t off, int64_t i, Cd v) {
+  int *w = reinterpret_cast<int *>(base + off) + 4 * i;
+  const double c[2] = {v.x, v.y};
+  for (int k = 0; k < 2; k++) {
+    const int64_t q = (int64_t)std::llrint(c[k] * 0x1p62);
+    const int32_t l = (int32_t)(uint32_t)(uint64_t)q;
+    w[2 * k] = (int)((q - l) >> 32);
+    w[2 * k + 1] = l;
   }
 }
 
@@ -316,6 +339,7 @@ bool fft4_shape(int64_t n, Fft4Dev *d, bool bluestein, bool f64) {
 size_t fft4_table_bytes(const Fft4Dev &d) { return layout(d).total; }
 
 size_t fft4_t_bytes(const Fft4Dev &d, int64_t nrow) {
+  if (d.i64()) return fft4_i64_bytes(d, nrow);
   return (size_t)((nrow + 1) / 2) * (size_t)(d.tsz + (d.blue ? d.vsz : 0)) * csz(d);
 }
 
@@ -327,9 +351,9 @@ static int bluestein_bhat(const Fft4Dev &d, char *base, size_t off) {
   std::vector<cufftDoubleComplex> b((size_t)M);
   for (auto &v : b) v.x = v.y = 0.0;
   for (int64_t t = 0; t <= 2 * m; t++) {
-    const double a = M_PI * (double)((t * t) % (2 * Lx)) / (double)Lx;  // conj(c_t) = exp(+i a)
-    b[(size_t)t].x = std::cos(a);
-    b[(size_t)t].y = std::sin(a);
+    const Cd c = unit((t * t) % (2 * Lx), 2 * Lx);  // b_t = conj(c_t)
+    b[(size_t)t].x = c.x;
+    b[(size_t)t].y = -c.y;
     if (t > 0 && t <= m) b[(size_t)(M - t)] = b[(size_t)t];
   }
   cufftDoubleComplex *db = nullptr;
@@ -363,8 +387,12 @@ int fft4_init(Fft4Plan *p, int64_t n, void *dev_tables, bool bluestein, bool f64
     const size_t so = pass ? t.stw2 : t.stw1;
     for (int s = 0; s < nr; s++)
       for (int rr = 1; rr < r[s]; rr++)
-        for (int k = 0; k < ns[s]; k++)
-          put(h.data(), so, to[s] + (rr - 1) * ns[s] + k, unit((double)rr * k, (double)ns[s] * r[s]), d.f64);
+        for (int k = 0; k < ns[s]; k++) {
+          const int64_t i = to[s] + (rr - 1) * ns[s] + k;
+          const Cd v = unit((int64_t)rr * k, (int64_t)ns[s] * r[s]);
+          if (d.i64()) put_i64(h.data(), so, i, v);
+          else put(h.data(), so, i, v, d.f64);
+        }
   }
   {
     std::vector<int> P1(d.L1), P2(d.L2);
@@ -376,17 +404,17 @@ int fft4_init(Fft4Plan *p, int64_t n, void *dev_tables, bool bluestein, bool f64
     for (int j = 0; j < d.L2; j++) I2[P2[j]] = j;
   }
   for (int64_t j1 = 0; j1 < d.H1; j1++) {
-    for (int l = 0; l < 32; l++) put(h.data(), t.tlane, 32 * j1 + l, unit((double)(j1 * l % d.L), (double)d.L), d.f64);
+    for (int l = 0; l < 32; l++) put(h.data(), t.tlane, 32 * j1 + l, unit(j1 * l, d.L), d.f64);
     for (int i = 0; i < d.nb32; i++) {
       // the signed k of the block's first entry: e, or e - pad - L2 in the upper half
       const int64_t e = 32 * i, k = e < d.L2 / 2 + d.pad ? e : e - d.pad - d.L2;
-      put(h.data(), t.tblk, j1 * d.nb32 + i, unit((double)(j1 * k % d.L), (double)d.L), d.f64);
+      put(h.data(), t.tblk, j1 * d.nb32 + i, unit(j1 * k, d.L), d.f64);
     }
   }
   if (d.blue) {
     for (int64_t j = 0; j <= d.m; j++)
-      put(h.data(), t.chirp, j, unit((double)((j * j) % (2 * d.Lx)), 2.0 * (double)d.Lx), d.f64);
-    Cd cm = unit((double)((d.m * d.m) % (2 * d.Lx)), 2.0 * (double)d.Lx);
+      put(h.data(), t.chirp, j, unit((j * j) % (2 * d.Lx), 2 * d.Lx), d.f64);
+    Cd cm = unit((d.m * d.m) % (2 * d.Lx), 2 * d.Lx);
     put(h.data(), t.chirp, d.m + 1, cm, d.f64);
     cm.x *= 0.5;
     cm.y *= 0.5;
@@ -396,9 +424,9 @@ int fft4_init(Fft4Plan *p, int64_t n, void *dev_tables, bool bluestein, bool f64
     d.nb32b = (d.L1 + 31) / 32;
     for (int64_t k2 = 0; k2 < d.L2; k2++) {
       for (int l = 0; l < 32; l++)
-        put(h.data(), t.tlane2, 32 * k2 + l, unit((double)(k2 * l % d.L), (double)d.L), d.f64);
+        put(h.data(), t.tlane2, 32 * k2 + l, unit(k2 * l, d.L), d.f64);
       for (int i = 0; i < d.nb32b; i++)
-        put(h.data(), t.tblk2, k2 * d.nb32b + i, unit((double)(k2 * 32 * i % d.L), (double)d.L), d.f64);
+        put(h.data(), t.tblk2, k2 * d.nb32b + i, unit(k2 * 32 * i, d.L), d.f64);
     }
   }
   MK_CUDA(cudaMemcpy(dev_tables, h.data(), t.total, cudaMemcpyHostToDevice));
@@ -416,6 +444,7 @@ int fft4_init(Fft4Plan *p, int64_t n, void *dev_tables, bool bluestein, bool f64
   d.tlane2 = d.blue ? (const void *)(b + t.tlane2) : nullptr;
   d.tblk2 = d.blue ? (const void *)(b + t.tblk2) : nullptr;
   p->tables = dev_tables;
+  if (d.i64()) return fft4_i64_tfull(d, b + t.tfull);
   return d.f64 ? fft4_tfull_f64(d, (double2 *)(b + t.tfull)) : MK_OK;
 }
 

@@ -22,10 +22,10 @@
 //   * F_{L-k} = F_k, and L - (k2 + L2 k1) lies in column L2 - k2, so pass B
 //     runs the H2 = L2 / 2 + 1 columns k2 <= L2 / 2 only and writes each
 //     output to k or L - k, whichever is <= m.
-// One DCT-I of 256 x 130,978 takes 0.171 ms in FP32 and 2.52 ms in FP64,
-// against 0.307 and 5.63 ms with all columns (0.193 and 3.06 ms before the
-// butterflies' operation counts and the index arithmetic were cut);
-// Bluestein (below) on 256 x 144,278 0.742 and 13.4 ms against 0.953 and 20.1.
+// In FP32 one DCT-I of 256 x 130,978 takes 0.171 ms against 0.307 with all
+// columns (0.193 before the butterflies' operation counts and the index
+// arithmetic were cut); Bluestein (below) on 256 x 144,278 0.727 ms against
+// 0.953 (FP64 13.1 against 20.1).  FP64 without Bluestein: mk_fft4_i64.cu.
 // Each CTA runs 8 or 16 (FP64: 4 or 8) transforms of one pass in shared memory (mixed-radix
 // decimation in time, butterflies in place), interleaved over its threads.
 // The first stage of each pass reads its inputs straight from global memory
@@ -85,7 +85,7 @@ struct Fft4Dev {
   // per stage: span Ns of the earlier stages, 1 / Ns, offset of its twiddles
   int ns1[FFT4_MAXR], ns2[FFT4_MAXR], to1[FFT4_MAXR], to2[FFT4_MAXR];
   float inv1[FFT4_MAXR], inv2[FFT4_MAXR];
-  // complex tables (float2 or double2 by precision)
+  // complex tables: float2, double2, or (FP64 without Bluestein, i64()) 16-byte fixed-point entries
   // stage twiddles W_{Ns R}^{r k} at [to + (r - 1) Ns + k]
   const void *stw1, *stw2;
   const int *iperm1, *iperm2;  // natural index at each digit-reversed (DIT input) position
@@ -98,6 +98,8 @@ struct Fft4Dev {
   // Bluestein's middle pass: W_M^{k2 o1} = tblk2[k2 nb32b + o1 / 32] * tlane2[32 k2 + o1 % 32]
   const void *tlane2, *tblk2;
   int nb32b;  // ceil(L1 / 32)
+  // the plan's passes run in fixed point (mk_fft4_i64.cu): stw1, stw2 and tfull hold its twiddles
+  __host__ __device__ bool i64() const { return f64 && !blue; }
 };
 
 // epilogues of pass B
@@ -127,10 +129,19 @@ int fft4_init(Fft4Plan *p, int64_t n, void *dev_tables, bool bluestein = true, b
 // T is scratch of fft4_t_bytes; w (ld ldw) only for FFT4_FILTER.
 int fft4_dct(const Fft4Plan &p, const float *x, int64_t ldx, int64_t nrow, float2 *T, float *out,
              int64_t ldo, int epi, const float *w, int64_t ldw, cudaStream_t st);
-// the same for an FP64 plan (fft4_init with f64)
+// the same for an FP64 plan (fft4_init with f64) that runs Bluestein
 int fft4_dct_f64(const Fft4Plan &p, const double *x, int64_t ldx, int64_t nrow, double2 *T, double *out,
                  int64_t ldo, int epi, const double *w, int64_t ldw, cudaStream_t st);
 // fills out[H1 P] with an FP64 plan's four-step twiddles (returns when done)
 int fft4_tfull_f64(const Fft4Dev &d, double2 *out);
+
+// FP64 plans without Bluestein (d.i64()): scratch bytes, the transform, and the
+// fixed-point four-step twiddles.  chained: x is the output of this plan's
+// last FFT4_FILTER transform of as many rows (whose largest values the scratch
+// still holds).
+size_t fft4_i64_bytes(const Fft4Dev &d, int64_t nrow);
+int fft4_dct_i64(const Fft4Plan &p, const double *x, int64_t ldx, int64_t nrow, void *scratch, double *out,
+                 int64_t ldo, int epi, const double *w, int64_t ldw, bool chained, cudaStream_t st);
+int fft4_i64_tfull(const Fft4Dev &d, void *out);
 
 }  // namespace mk

@@ -1,5 +1,6 @@
-// FP64 DCT-I by the four-step FFT: the kernels of mk_fft4_kern.cuh in
-// double precision (8 or 4 transforms per CTA, 256 threads).
+// FP64 DCT-I by the four-step FFT through Bluestein's algorithm: the kernels of
+// mk_fft4_kern.cuh in double precision (8 or 4 transforms per CTA, 256
+// threads).  Lengths that need no Bluestein run in mk_fft4_i64.cu.
 #define MK_FFT4_NS f4d
 #define MK_FFT4_C double2
 #define MK_FFT4_RT double
@@ -8,6 +9,7 @@
 #define MK_FFT4_NTHI 256
 #define MK_FFT4_NTLO 256
 #define MK_FFT4_MINBLO 2
+#define MK_FFT4_SMOOTH 0
 #include "mk_fft4.cuh"
 #undef MK_FFT4_RMAX
 #define MK_FFT4_RMAX MK_FFT4_RMAX64

@@ -7,6 +7,7 @@
 //   MK_FFT4_NTHI / MK_FFT4_NTLO        threads per CTA for each
 //   MK_FFT4_MINBLO                     CTAs per SM the narrow tile's registers are sized for
 //   (MK_FFT4_MINBHI, default 2: the same for the wide tile)
+//   MK_FFT4_SMOOTH                     1: lengths without Bluestein too (0 in FP64: mk_fft4_i64.cu has those)
 // and includes this file once.  dct_launch is the host entry of the
 // precision.
 #include <cufft.h>
@@ -24,6 +25,7 @@ namespace MK_FFT4_NS {
 using C = MK_FFT4_C;
 using RT = MK_FFT4_RT;
 constexpr bool F32 = sizeof(RT) == 4;
+static_assert(MK_FFT4_RMAX >= 11, "every prime of a supported length is a radix");
 #ifndef MK_FFT4_PACK
 #define MK_FFT4_PACK 1
 #endif
@@ -640,6 +642,9 @@ template <int R, int BM, int EPI>
 __device__ __forceinline__ void bput(C *v, int q, int Ns, const PassB &pb) {
 #pragma unroll
   for (int r = 0; r < R; r++) {
+    // Bluestein keeps the outputs kk <= m < M / 3: none has r >= R / 3, and the
+    // butterfly that forms them drops out
+    if (BM == BM_BLUE && 3 * r >= R) continue;
     int kk = pb.k2 + pb.L2 * (q + r * Ns);
     if (BM == BM_DCT) {
       if (pb.self && kk > pb.m) continue;  // a self-mirrored column holds both values of a pair
@@ -971,16 +976,18 @@ int dct_launch(const Fft4Plan &p, const RT *x, int64_t ldx, int64_t nrow, C *T, 
     const int mhi = FB_HI * (FFT4_LMAX + 1) * (int)sizeof(C);
     const int mlo = FB_LO * (FFT4_LMAX + 1) * (int)sizeof(C);
 #define MK_FFT4_ATTR(k, v) MK_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, v))
-    MK_FFT4_ATTR((k_fft4_a<AM_DCT, FB_LO>), mlo);
     MK_FFT4_ATTR((k_fft4_a<AM_BLUE, FB_LO>), mlo);
-    MK_FFT4_ATTR((k_fft4_b<BM_DCT, FB_LO>), mlo);
     MK_FFT4_ATTR((k_fft4_b<BM_BLUE, FB_LO>), mlo);
-    MK_FFT4_ATTR((k_fft4_a<AM_DCT, FB_HI>), mhi);
     MK_FFT4_ATTR((k_fft4_a<AM_BLUE, FB_HI>), mhi);
-    MK_FFT4_ATTR((k_fft4_b<BM_DCT, FB_HI>), mhi);
     MK_FFT4_ATTR((k_fft4_b<BM_BLUE, FB_HI>), mhi);
     MK_FFT4_ATTR((k_fft4_conv<FB_LO>), mlo);
     MK_FFT4_ATTR((k_fft4_conv<FB_HI>), mhi);
+#if MK_FFT4_SMOOTH
+    MK_FFT4_ATTR((k_fft4_a<AM_DCT, FB_LO>), mlo);
+    MK_FFT4_ATTR((k_fft4_b<BM_DCT, FB_LO>), mlo);
+    MK_FFT4_ATTR((k_fft4_a<AM_DCT, FB_HI>), mhi);
+    MK_FFT4_ATTR((k_fft4_b<BM_DCT, FB_HI>), mhi);
+#endif
 #undef MK_FFT4_ATTR
     g_attr[dev] = true;
   }
@@ -991,6 +998,7 @@ int dct_launch(const Fft4Plan &p, const RT *x, int64_t ldx, int64_t nrow, C *T, 
   const size_t smem_b = (size_t)fb * pitch_odd(d.L1) * sizeof(C);  // transforms of length L1
   const dim3 ga((d.H1 + fa - 1) / fa, np);
   int rc;
+#if MK_FFT4_SMOOTH
   if (!d.blue) {
     const dim3 gb((d.H2 + fb - 1) / fb, np);
     if (hia) k_fft4_a<AM_DCT, FB_HI><<<ga, Cfg<FB_HI>::NT, smem_a, st>>>(x, ldx, nrow, T, d);
@@ -1000,6 +1008,9 @@ int dct_launch(const Fft4Plan &p, const RT *x, int64_t ldx, int64_t nrow, C *T, 
     else k_fft4_b<BM_DCT, FB_LO><<<gb, Cfg<FB_LO>::NT, smem_b, st>>>(T, nrow, out, ldo, w, ldw, epi, d);
     return launch_status("fft4 pass B");
   }
+#else
+  MK_CHECK_ARG(d.blue, "fft4: plan does not match the call");
+#endif
   C *V = T + npairs * d.tsz;
   if (hia) k_fft4_a<AM_BLUE, FB_HI><<<ga, Cfg<FB_HI>::NT, smem_a, st>>>(x, ldx, nrow, T, d);
   else k_fft4_a<AM_BLUE, FB_LO><<<ga, Cfg<FB_LO>::NT, smem_a, st>>>(x, ldx, nrow, T, d);

@@ -28,9 +28,11 @@
 // otherwise, up to its length limit):
 //   E = v . dat;  E = DCT(E) * mywt;  E = DCT(E) with columns 0 and n-1
 //   halved;  out = vT . E.
-// Each DCT is two kernels (three with Bluestein) that form the even
-// extension while loading and apply the weights or the halving while
-// storing, two detector rows per complex transform.
+// Each DCT is two kernels (three with Bluestein) that form the even extension
+// while loading and apply the weights or the halving while storing, two
+// detector rows per complex transform; FP64 plans need the rows' largest
+// values first (a pass over them before the first DCT, the first DCT's output
+// kernel for the second).
 #include <cublas_v2.h>
 #include <cufft.h>
 
@@ -317,8 +319,13 @@ int core_fft(DctCore *c, cudaStream_t st) {
   return MK_OK;
 }
 
-// one four-step DCT-I of the plan's rows (ld n), in the plan's precision
-int own_dct(DctCore *c, const void *in, void *out, int epi, const void *w, int64_t ldw, cudaStream_t st) {
+// one four-step DCT-I of the plan's rows (ld n), in the plan's precision;
+// chained: `in` is the output of the FFT4_FILTER transform just before it
+int own_dct(DctCore *c, const void *in, void *out, int epi, const void *w, int64_t ldw, cudaStream_t st,
+            bool chained = false) {
+  if (c->f4.d.i64())
+    return mk::fft4_dct_i64(c->f4, (const double *)in, c->n, c->nrow, c->T, (double *)out, c->n, epi,
+                            (const double *)w, ldw, chained, st);
   if (c->dtype == MK_F64)
     return mk::fft4_dct_f64(c->f4, (const double *)in, c->n, c->nrow, (double2 *)c->T, (double *)out, c->n, epi,
                             (const double *)w, ldw, st);
@@ -437,7 +444,7 @@ int apply_noise_t(DctCore *c, const T *v, const T *vT, const T *w, int64_t ldw, 
     T *E = (T *)c->E;
     if ((rc = rotate(c, rot_mode, v, dat, n, E, n, nd, n, st))) return rc;
     if ((rc = own_dct(c, E, E, mk::FFT4_FILTER, w, ldw, st))) return rc;
-    if ((rc = own_dct(c, E, E, mk::FFT4_HALVE, nullptr, 0, st))) return rc;
+    if ((rc = own_dct(c, E, E, mk::FFT4_HALVE, nullptr, 0, st, true))) return rc;
     return rotate(c, rot_mode, vT, E, n, out, n, nd, n, st);
   }
   const bool fused_mirror = (rot_mode == 2);  // the tensor-core epilogue writes the extension

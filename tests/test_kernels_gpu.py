@@ -325,6 +325,47 @@ def test_dct1_every_short_length(K, dtype, tol, split):
         assert rel(d(dev(x, dtype)).cpu().numpy(), oracle.dct1(x)) < tol, n
 
 
+@pytest.mark.parametrize("n", [2, 9, 5001, 65341])
+def test_dct1_f64_ranges_of_values(K, n):
+    """The block fixed point of the FP64 DCT-I: rows from 1e-300 to 1e290, an
+    impulse far above the rest, offsets, zero rows, rows of different scale in
+    a pair (held to the larger one, as any transform of the packed pair is),
+    an odd row out, and NaN / infinity (both rows of their pair become NaN, the
+    others stay).  1e-12 of the pair's largest output, as for the FP64 passes."""
+    rng = np.random.default_rng(n)
+    x = rng.standard_normal((13, n))
+    for i, sc in enumerate((1e-300, 1e-100, 1e100, 1e290)):
+        x[2 * i:2 * i + 2] *= sc
+    x[8, n // 3] += 1e9
+    x[9] += 1e6
+    x[10] = 0.0
+    x[11] *= 1e-8
+    d = K.DCT1(13, n, torch.float64)
+    y = d(dev(x)).cpu().numpy()
+    ref = oracle.dct1(x)
+    for p in range(0, 13, 2):
+        assert rel(y[p:p + 2], ref[p:p + 2]) < 1e-12, p
+    assert (d(dev(np.zeros((13, n)))).cpu().numpy() == 0).all()
+    x[2, n - 1], x[5, 0] = np.nan, -np.inf
+    z = d(dev(x)).cpu().numpy()
+    assert np.isnan(z[2:6]).all()
+    keep = [0, 1] + list(range(6, 13))
+    assert np.array_equal(z[keep], y[keep])
+
+
+def test_apply_noise_f64_nonfinite_sample(K):
+    """A NaN sample makes the whole filtered TOD NaN (every output mixes all
+    detectors and samples), through the sliced rotation and both transforms."""
+    rng = np.random.default_rng(5)
+    v = np.linalg.qr(rng.standard_normal((6, 6)))[0]
+    x, w = rng.standard_normal((6, 4097)), rng.random((6, 4097))
+    plan = K.NoisePlan(6, 4097, torch.float64)
+    good = plan.apply(dev(v), dev(v.T), dev(w), dev(x), rot_mode=4).cpu().numpy()
+    assert rel(good, oracle.apply_noise(v, v.T, w, x)) < 1e-12
+    x[3, 77] = np.nan
+    assert np.isnan(plan.apply(dev(v), dev(v.T), dev(w), dev(x), rot_mode=4).cpu().numpy()).all()
+
+
 def test_dct1_engines_agree_and_fall_back(K):
     x = np.random.default_rng(9).standard_normal((6, 2311))
     own = K.DCT1(6, 2311, torch.float32)(dev(x, torch.float32)).cpu().numpy()
