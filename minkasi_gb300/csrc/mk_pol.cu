@@ -15,8 +15,8 @@
 // form, FP64) or read from a cos/sin pair computed once per TOD by
 // mk_pol_sincos (the pointing is fixed across PCG iterations, so this trades
 // 8 more bytes per sample for no FP64 transcendental work on GB300's narrow
-// FP64 pipe).  tod2map sums runs of equal pixels over 4 consecutive samples
-// per thread in registers and issues one atomic per Stokes component per run.
+// FP64 pipe).  tod2map sums runs of equal pixels over windows of 128 samples
+// per warp and issues one atomic per Stokes component per run.
 #include <math.h>
 
 #include "mk_common.cuh"
@@ -31,18 +31,35 @@ template <> struct Pol<MK_POL_IQU> { static constexpr int N = 3; };
 template <> struct Pol<MK_POL_QU_PRECON> { static constexpr int N = 3; };
 template <> struct Pol<MK_POL_IQU_PRECON> { static constexpr int N = 6; };
 
-// per-sample Stokes weights, in the reference's operation order
-template <int MODE, typename T>
-__device__ __forceinline__ void pol_terms(T d, T c, T s, T (&o)[Pol<MODE>::N]) {
+// acc (or 0 if `fresh`; FIRST: nothing yet) plus the sample's Stokes weights: one FP64 operation
+// per term where the last product joins the sum as an FMA (the FP64 pipe bounds
+// the kernel)
+template <int MODE, typename T, bool FIRST>
+__device__ __forceinline__ void pol_add(T (&acc)[Pol<MODE>::N], bool fresh, T d, T c, T s) {
+  T b[Pol<MODE>::N];
+#pragma unroll
+  for (int k = 0; k < Pol<MODE>::N; k++) b[k] = fresh ? T(0) : acc[k];
   if constexpr (MODE == MK_POL_QU) {
-    o[0] = d * c; o[1] = d * s;
+    acc[0] = fma(d, c, b[0]);
+    acc[1] = fma(d, s, b[1]);
   } else if constexpr (MODE == MK_POL_IQU) {
-    o[0] = d; o[1] = d * c; o[2] = d * s;
-  } else if constexpr (MODE == MK_POL_QU_PRECON) {
-    o[0] = (d * c) * c; o[1] = (d * s) * s; o[2] = (d * s) * c;
+    acc[0] = FIRST ? d : b[0] + d;
+    acc[1] = fma(d, c, b[1]);
+    acc[2] = fma(d, s, b[2]);
   } else {
-    o[0] = d; o[1] = d * c; o[2] = d * s;
-    o[3] = (d * c) * c; o[4] = (d * s) * c; o[5] = (d * s) * s;
+    const T dc = d * c, ds = d * s;
+    if constexpr (MODE == MK_POL_QU_PRECON) {
+      acc[0] = fma(dc, c, b[0]);
+      acc[1] = fma(ds, s, b[1]);
+      acc[2] = fma(ds, c, b[2]);
+    } else {
+      acc[0] = FIRST ? d : b[0] + d;
+      acc[1] = FIRST ? dc : b[1] + dc;
+      acc[2] = FIRST ? ds : b[2] + ds;
+      acc[3] = fma(dc, c, b[3]);
+      acc[4] = fma(ds, c, b[4]);
+      acc[5] = fma(ds, s, b[5]);
+    }
   }
 }
 
@@ -86,53 +103,142 @@ __global__ void __launch_bounds__(256) k_polmap2tod(T *__restrict__ dat, const T
   }
 }
 
+// four consecutive values (16-byte aligned)
+__device__ __forceinline__ void load4(const double *p, double *v) {
+  const double2 a = __ldcs(reinterpret_cast<const double2 *>(p)), b = __ldcs(reinterpret_cast<const double2 *>(p) + 1);
+  v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
+}
+__device__ __forceinline__ void load4(const float *p, float *v) {
+  const float4 a = __ldcs(reinterpret_cast<const float4 *>(p));
+  v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+}
+
+// Scatter: a warp takes windows of 256 consecutive samples, 8 per lane (16-byte
+// loads if VEC: every array 16-byte aligned).  Runs of equal pixels are summed
+// in registers, joined across lanes, written to shared memory in sample order
+// and added to the map component by component: 32 consecutive (run, component)
+// pairs per instruction, which are neighbouring words of the map, as in
+// tod2map's warp_runs.  IQU on 64 x 65,341 samples, 256^2 pixels: FP64 45 us for
+// 51 with an atomic per component and 4-sample run in each thread, FP32 14 for
+// 46; on 256 x 130,978, 1024^2: 235 for 405 and 104 for 304.
 // ROWS: d = rowval[i / ndata] (1 if rowval is NULL): hit / weight maps
-template <int MODE, typename T, bool TRIG, bool ROWS>
-__global__ void __launch_bounds__(256) k_tod2polmap(T *__restrict__ map, const T *__restrict__ dat,
-                                                    const T *__restrict__ cs, const T *__restrict__ sn,
-                                                    const double *__restrict__ tg,
-                                                    const int32_t *__restrict__ ipix, int64_t n, int64_t npix,
-                                                    const T *__restrict__ rowval, int64_t ndata) {
+constexpr unsigned FULL = 0xffffffffu;
+template <int MODE>
+constexpr int PW = Pol<MODE>::N > 3 ? 2 : 4;  // warps per CTA (their runs fit in shared memory)
+
+template <int MODE, typename T, bool TRIG, bool ROWS, bool VEC>
+__global__ void __launch_bounds__(PW<MODE> * 32) k_tod2polmap(T *__restrict__ map, const T *__restrict__ dat,
+                                                        const T *__restrict__ cs, const T *__restrict__ sn,
+                                                        const double *__restrict__ tg,
+                                                        const int32_t *__restrict__ ipix, int64_t n, int64_t npix,
+                                                        const T *__restrict__ rowval, int64_t ndata) {
   constexpr int NP = Pol<MODE>::N;
-  constexpr int U = 4;
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  const int64_t nu = (n + U - 1) / U;
-  for (int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; g < nu; g += stride) {
-    int32_t key = -1;
+  __shared__ T rsum[PW<MODE>][256 * NP];
+  __shared__ int32_t rkey[PW<MODE>][256];
+  const int lane = threadIdx.x & 31;
+  T *const sum = rsum[threadIdx.x >> 5];
+  int32_t *const key = rkey[threadIdx.x >> 5];
+  const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int64_t nwarp = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  for (int64_t base = warp * 256; base < n; base += nwarp * 256) {
+    const int64_t i0 = base + 8 * lane, left = n - i0;
+    const int m = left <= 0 ? 0 : (left >= 8 ? 8 : (int)left);  // valid samples, a prefix of the window
+    int32_t p[8];
+    T d[8], c[8], s[8];
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+      p[j] = INT32_MIN;
+      d[j] = c[j] = s[j] = T(0);
+    }
+    if (VEC && m == 8) {
+#pragma unroll
+      for (int h = 0; h < 8; h += 4) {
+        const int4 q = __ldcs(reinterpret_cast<const int4 *>(ipix + i0 + h));
+        p[h] = q.x; p[h + 1] = q.y; p[h + 2] = q.z; p[h + 3] = q.w;
+        if constexpr (!ROWS) load4(dat + i0 + h, d + h);
+        if constexpr (!TRIG) {
+          load4(cs + i0 + h, c + h);
+          load4(sn + i0 + h, s + h);
+        }
+      }
+    } else {
+#pragma unroll
+      for (int j = 0; j < 8; j++) {
+        if (j >= m) continue;
+        p[j] = __ldcs(ipix + i0 + j);
+        if constexpr (!ROWS) d[j] = __ldcs(dat + i0 + j);
+        if constexpr (!TRIG) angle<T, TRIG>(cs, sn, tg, i0 + j, c[j], s[j]);
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+      if (j >= m) continue;
+      if constexpr (ROWS) d[j] = rowval ? rowval[(i0 + j) / ndata] : T(1);
+      if constexpr (TRIG) angle<T, TRIG>(cs, sn, tg, i0 + j, c[j], s[j]);
+    }
+    // which samples end a run, and the places of the lane's closed runs
+    int32_t kf = INT32_MIN, kl = INT32_MIN;
+    unsigned ends = 0;
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+      if (j < m) {
+        if (j == 0) kf = p[0];
+        else if (p[j] != p[j - 1]) ends |= 1u << (j - 1);
+        kl = p[j];
+      }
+    }
+    const bool single = ends == 0;
+    const int32_t kl_prev = __shfl_up_sync(FULL, kl, 1), kf_next = __shfl_down_sync(FULL, kf, 1);
+    const bool cont_in = lane > 0 && m > 0 && kl_prev == kf;
+    const bool cont_out = lane < 31 && kf_next == kl && m > 0;
+    if (m > 0 && !cont_out) ends |= 1u << (m - 1);
+    const int cnt = __popc(ends);
+    int at = cnt;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+      const int up = __shfl_up_sync(FULL, at, off);
+      if (lane >= off) at += up;
+    }
+    const int total = __shfl_sync(FULL, at, 31), first = at - cnt;
+    at = first;
     T acc[NP];
 #pragma unroll
     for (int k = 0; k < NP; k++) acc[k] = T(0);
 #pragma unroll
-    for (int u = 0; u < U; u++) {
-      const int64_t i = g * U + u;
-      if (i >= n) break;
-      const int32_t p = __ldcs(ipix + i);
-      T d;
-      if (ROWS)
-        d = rowval ? rowval[i / ndata] : T(1);
-      else
-        d = __ldcs(dat + i);
-      T c, s;
-      angle<T, TRIG>(cs, sn, tg, i, c, s);
-      T o[NP];
-      pol_terms<MODE, T>(d, c, s, o);
-      if (p != key) {
-        if ((uint32_t)key < (uint64_t)npix) {
+    for (int j = 0; j < 8; j++) {
+      if (j >= m) continue;
+      if (j == 0) pol_add<MODE, T, true>(acc, true, d[0], c[0], s[0]);
+      else pol_add<MODE, T, false>(acc, ends >> (j - 1) & 1, d[j], c[j], s[j]);
+      if (ends >> j & 1) {
+        key[at] = p[j];
 #pragma unroll
-          for (int k = 0; k < NP; k++) atomicAdd(map + (int64_t)key * NP + k, acc[k]);
-        }
-        key = p;
-#pragma unroll
-        for (int k = 0; k < NP; k++) acc[k] = o[k];
-      } else {
-#pragma unroll
-        for (int k = 0; k < NP; k++) acc[k] += o[k];
+        for (int k = 0; k < NP; k++) sum[at * NP + k] = acc[k];
+        at++;
       }
     }
-    if ((uint32_t)key < (uint64_t)npix) {
+    // what a lane hands on (see warp_runs in mk_proj.cu)
+    bool pend = single && cont_in;
+    for (int off = 1; __any_sync(FULL, pend); off <<= 1) {
+      const bool pup = __shfl_up_sync(FULL, (int)pend, off) != 0;
 #pragma unroll
-      for (int k = 0; k < NP; k++) atomicAdd(map + (int64_t)key * NP + k, acc[k]);
+      for (int k = 0; k < NP; k++) {
+        const T up = __shfl_up_sync(FULL, acc[k], off);
+        if (pend) acc[k] += up;
+      }
+      if (pend) pend = pup;
     }
+#pragma unroll
+    for (int k = 0; k < NP; k++) {
+      const T prev = __shfl_up_sync(FULL, acc[k], 1);
+      if (cont_in && cnt > 0) sum[first * NP + k] += prev;
+    }
+    __syncwarp();
+    for (int e = lane; e < total * NP; e += 32) {
+      const int r = e / NP;
+      const int32_t q = key[r];
+      if ((uint32_t)q < (uint64_t)npix) atomicAdd(map + (int64_t)q * NP + (e - r * NP), sum[e]);
+    }
+    __syncwarp();
   }
 }
 
@@ -193,9 +299,11 @@ template <int MODE, typename T, bool TRIG, bool ROWS>
 int tod2polmap_t(void *map, const void *dat, const void *cs, const void *sn, const double *tg,
                  const int32_t *ipix, int64_t n, int64_t npix, const void *rowval, int64_t ndata,
                  cudaStream_t st) {
-  auto k = k_tod2polmap<MODE, T, TRIG, ROWS>;
-  k<<<mk_grid_fit(k, (n + 3) / 4, 256), 256, 0, st>>>((T *)map, (const T *)dat, (const T *)cs, (const T *)sn,
-                                                       tg, ipix, n, npix, (const T *)rowval, ndata);
+  const auto off16 = [](const void *q) { return (uintptr_t)q % 16 != 0; };
+  const bool vec = !off16(ipix) && (ROWS || !off16(dat)) && (TRIG || (!off16(cs) && !off16(sn)));
+  auto k = vec ? k_tod2polmap<MODE, T, TRIG, ROWS, true> : k_tod2polmap<MODE, T, TRIG, ROWS, false>;
+  k<<<mk_grid((n + 7) / 8, PW<MODE> * 32, 64), PW<MODE> * 32, 0, st>>>((T *)map, (const T *)dat, (const T *)cs, (const T *)sn, tg,
+                                                            ipix, n, npix, (const T *)rowval, ndata);
   return mk::launch_status("mk_tod2polmap");
 }
 

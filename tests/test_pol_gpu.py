@@ -59,6 +59,32 @@ def test_pol_fp32(K, gold):
     assert rel(m.cpu().numpy(), g["t2m_IQU_PRECON"]) < 2e-5
 
 
+@pytest.mark.parametrize("n", [1, 7, 8, 9, 255, 256, 257, 3000])
+@pytest.mark.parametrize("off", [0, 1])
+def test_tod2polmap_windows_and_runs(K, n, off):
+    """Windows of 256 samples, 8 per lane: remainders, unaligned arrays, runs
+    from 1 to 600 samples, indices outside the map, all modes and both
+    precisions, against numpy sums in double precision (tolerances of the
+    tests above)."""
+    import oracle
+    rng = np.random.default_rng(n + off)
+    npix, N = 50, 2 * n + off
+    runs = np.concatenate([np.full(k, p) for k, p in zip(rng.integers(1, 1 + rng.integers(1, 600), size=N),
+                                                         rng.integers(-3, npix + 3, size=N))])[:N]
+    ip = runs.astype(np.int32)
+    d, tg = rng.standard_normal(N), rng.uniform(0, 6.28, N)
+    ok = (ip >= 0) & (ip < npix)
+    for dt, tol in ((torch.float64, 1e-12), (torch.float32, 2e-5)):
+        c, s = K.pol_sincos(dev(tg), dt)
+        sl = slice(off, None)
+        for mode, npol in (("QU", 2), ("IQU", 3), ("QU_PRECON", 3), ("IQU_PRECON", 6)):
+            ref = np.zeros((npix, npol))
+            oracle.tod2polmap(ref, d[sl][ok[sl]], mode, tg[sl][ok[sl]], ip[sl][ok[sl]])
+            m = torch.zeros(npix * npol, dtype=dt, device=cuda)
+            K.tod2polmap(m, dev(d, dt)[sl].view(1, -1), mode, (c[sl], s[sl]), dev(ip)[sl])
+            assert rel(m.cpu().numpy().reshape(npix, npol), ref) < tol, (mode, dt)
+
+
 def test_pol_bad_arguments(K, gold):
     g = gold("pol.npz")
     with pytest.raises(K._lib.MkError):  # no map2tod for PRECON modes, as in the reference
