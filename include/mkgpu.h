@@ -336,6 +336,15 @@ int mk_dct1_describe(int64_t n, int *engine, int64_t *L, int *L1, int *L2);
 int mk_set_fft4_split(int rank);
 int mk_get_fft4_split(void);
 
+/* G (nrow x nrow, FP64) = X . X^T for X (nrow x ncol, leading dimension ldx):
+ * the matrix whose eigenvectors are the left singular vectors that
+ * NoiseSmoothedSVD builds on (minkasi/mapmaking/noise.py:627-640).  Both
+ * triangles are written; the sums are in a fixed order (reproducible).
+ * `scratch` is mk_gram_scratch_bytes() bytes of device memory, free to be
+ * reused when the stream has run the call. */
+size_t mk_gram_scratch_bytes(int64_t nrow, int64_t ncol);
+int mk_gram(double *G, const double *X, int64_t ldx, int64_t nrow, int64_t ncol, void *scratch, void *stream);
+
 /* NoiseSmoothedSVD.apply_noise, minkasi/mapmaking/noise.py:680-714:
  *   out = halve_ends( vT . DCT1( mywt[:, :ndata] * DCT1( v . dat ) ) )
  * where halve_ends multiplies columns 0 and ndata-1 by 1/2.  v, vT are
@@ -344,8 +353,8 @@ int mk_get_fft4_split(void);
  * `out` may alias `dat`.  Prewhitening (noisevec) is folded into v and vT by
  * the caller.  The plan shares the DCT workspace contract above and may be
  * used for any TOD of the same (ndet, ndata).  rot_mode selects the
- * detector-rotation GEMM: 0 = automatic, 1 = cuBLAS on the FP64 / FP32 units
- * (DGEMM / SGEMM), 2 = this library's tensor-core kernel (FP32 only: three
+ * detector-rotation GEMM: 0 = automatic (FP64: this library's kernel on the
+ * FP64 units; FP32: SGEMM), 1 = cuBLAS on the FP64 / FP32 units (DGEMM / SGEMM), 2 = this library's tensor-core kernel (FP32 only: three
  * bf16 parts per value, exact, six of their products, FP32 accumulate), 3 = cuBLAS tensor-core emulation (FP64:
  * fixed-point slices; FP32: BF16x9), 4 = FP64 only: this library's exact
  * slicing of both operands into 7 signed integer slices of 8 bits after

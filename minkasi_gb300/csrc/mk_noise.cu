@@ -42,6 +42,7 @@
 #include <vector>
 
 #include "mk_common.cuh"
+#include "mk_f64mm.cuh"
 #include "mk_fft4.cuh"
 #include "mk_ozaki.cuh"
 #include "mk_rot.cuh"
@@ -410,15 +411,21 @@ int blas_rotate(int dtype, const void *A, const void *X, int64_t ldx, void *R, i
   return MK_OK;
 }
 
-// mode 0 (automatic) means cuBLAS here; the host autotuner picks 2 or 3 per
-// workload after checking their accuracy against it.
+// mode 0 (automatic): FP32 cuBLAS, FP64 this library's kernel on the FP64 pipe
+// (FP64 arithmetic throughout, as DGEMM; faster at every size tried, 2 to 300
+// detectors: see mk_f64mm.cu); the host autotuner picks another mode per workload
+// after checking its accuracy against cuBLAS.
 // mirror_n: see rot_tc_f32 (only the tensor-core kernel fuses the extension;
 // the caller runs k_mirror otherwise).
 int rotate(DctCore *c, int mode, const void *A, const void *X, int64_t ldx, void *R, int64_t ldr,
            int64_t nrow, int64_t ncol, cudaStream_t st, int64_t mirror_n = 0, int64_t x_stride = 1,
            int halve_ends = 0) {
   const int dtype = c->dtype;
-  if (mode == 0) mode = 1;
+  if (mode == 0) {
+    if (dtype == MK_F64)
+      return mk::rot_f64((const double *)A, (const double *)X, ldx, (double *)R, ldr, nrow, ncol, st);
+    mode = 1;
+  }
   if (mode == 2) {
     MK_CHECK_ARG(dtype == MK_F32, "tensor-core rotation (rot_mode 2) is FP32 only");
     MK_CHECK_ARG(c->tc_bimg != nullptr, "tensor-core rotation needs ndet in {32,64,128,256}");
