@@ -336,15 +336,6 @@ int mk_dct1_describe(int64_t n, int *engine, int64_t *L, int *L1, int *L2);
 int mk_set_fft4_split(int rank);
 int mk_get_fft4_split(void);
 
-/* G (nrow x nrow, FP64) = X . X^T for X (nrow x ncol, leading dimension ldx):
- * the matrix whose eigenvectors are the left singular vectors that
- * NoiseSmoothedSVD builds on (minkasi/mapmaking/noise.py:627-640).  Both
- * triangles are written; the sums are in a fixed order (reproducible).
- * `scratch` is mk_gram_scratch_bytes() bytes of device memory, free to be
- * reused when the stream has run the call. */
-size_t mk_gram_scratch_bytes(int64_t nrow, int64_t ncol);
-int mk_gram(double *G, const double *X, int64_t ldx, int64_t nrow, int64_t ncol, void *scratch, void *stream);
-
 /* NoiseSmoothedSVD.apply_noise, minkasi/mapmaking/noise.py:680-714:
  *   out = halve_ends( vT . DCT1( mywt[:, :ndata] * DCT1( v . dat ) ) )
  * where halve_ends multiplies columns 0 and ndata-1 by 1/2.  v, vT are

@@ -1,4 +1,4 @@
-// FP64 products on the FP64 pipe (see mk_f64mm.cu).
+// FP64 rotation on the FP64 pipe (see mk_f64mm.cu).
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>

@@ -380,18 +380,6 @@ def _workspace(nbytes: int, device) -> torch.Tensor:
     return torch.empty(max(int(nbytes), 256), dtype=torch.uint8, device=device)
 
 
-def gram(X: torch.Tensor) -> torch.Tensor:
-    """X X^T of an FP64 (nrow, ncol) array, both triangles (mk_gram)."""
-    _dev(X, "X")
-    if X.dtype != torch.float64 or X.dim() != 2:
-        raise TypeError("gram: X must be a 2-d float64 tensor")
-    n, m = X.shape
-    G = torch.empty((n, n), dtype=torch.float64, device=X.device)
-    ws = _workspace(int(lib().mk_gram_scratch_bytes(n, m)), X.device)
-    check(lib().mk_gram(_p(G), _p(X), m, n, m, _p(ws), _stream()), "gram")
-    return G
-
-
 def set_dct_engine(engine: int) -> None:
     """Transform used by DCT / noise plans created from now on: 0 (default)
     the four-step shared-memory FFT, in the plan's precision (through

@@ -85,13 +85,13 @@ def _eig_desc(c: np.ndarray) -> np.ndarray:
 
 def left_singular_vectors(dat: torch.Tensor) -> torch.Tensor:
     """u of the thin SVD of dat (ndet x ndata), columns by descending singular
-    value: eigenvectors of the Gram matrix d d^T (FP64, on the GPU),
+    value: eigenvectors of the Gram matrix d d^T (an FP64 GEMM on the GPU),
     decomposed on the host (ndet x ndet), then refined once by
     re-diagonalising the Gram matrix of the rotated data."""
-    u = _eig_desc(K.gram(dat).cpu().numpy())
+    u = _eig_desc((dat @ dat.T).cpu().numpy())
     ut = torch.from_numpy(np.ascontiguousarray(u)).to(dat.device)
     d2 = ut.T @ dat
-    u = u @ _eig_desc(K.gram(d2).cpu().numpy())
+    u = u @ _eig_desc((d2 @ d2.T).cpu().numpy())
     return torch.from_numpy(np.ascontiguousarray(u)).to(dat.device)
 
 
