@@ -136,7 +136,7 @@ bool radices(int Ls, int *r, int *nr, int rmax) {
 size_t al(size_t x) { return (x + 255) / 256 * 256; }
 
 struct TableLayout {
-  size_t stw1, stw2, iperm1, iperm2, perm1, tlane, tblk, tfull, chirp, bhat, tlane2, tblk2, total;
+  size_t stw1, stw2, iperm1, iperm2, perm1, tlane, tblk, chirp, bhat, tlane2, tblk2, tfull, total;
 };
 
 size_t csz(const Fft4Dev &d) { return d.f64 ? sizeof(double2) : sizeof(float2); }
@@ -155,11 +155,9 @@ TableLayout layout(const Fft4Dev &d) {
   t.perm1 = o;
   o += d.blue ? al((size_t)d.L1 * sizeof(int)) : 0;
   t.tlane = o;
-  o += al((size_t)d.H1 * 32 * csz(d));
+  o += d.i64() ? 0 : al((size_t)d.H1 * 32 * csz(d));
   t.tblk = o;
-  o += al((size_t)d.H1 * d.nb32 * csz(d));
-  t.tfull = o;
-  o += d.f64 ? al((size_t)d.tsz * csz(d)) : 0;
+  o += d.i64() ? 0 : al((size_t)d.H1 * d.nb32 * csz(d));
   t.chirp = o;
   o += d.blue ? al((size_t)(d.m + 2) * csz(d)) : 0;
   t.bhat = o;
@@ -168,6 +166,8 @@ TableLayout layout(const Fft4Dev &d) {
   o += d.blue ? al((size_t)d.L2 * 32 * csz(d)) : 0;
   t.tblk2 = o;
   o += d.blue ? al((size_t)d.L2 * ((d.L1 + 31) / 32) * csz(d)) : 0;
+  t.tfull = o;  // filled on the device: the host computes and uploads what lies before it
+  o += d.f64 ? al((size_t)d.tsz * csz(d)) : 0;
   t.total = o;
   return t;
 }
@@ -380,7 +380,7 @@ int fft4_init(Fft4Plan *p, int64_t n, void *dev_tables, bool bluestein, bool f64
                (long long)n);
   Fft4Dev &d = p->d;
   const TableLayout t = layout(d);
-  std::vector<char> h(t.total, 0);
+  std::vector<char> h(t.tfull, 0);
   for (int pass = 0; pass < 2; pass++) {
     const int nr = pass ? d.nr2 : d.nr1;
     const int *r = pass ? d.r2 : d.r1, *ns = pass ? d.ns2 : d.ns1, *to = pass ? d.to2 : d.to1;
@@ -403,7 +403,7 @@ int fft4_init(Fft4Plan *p, int64_t n, void *dev_tables, bool bluestein, bool f64
     if (d.blue) std::copy(P1.begin(), P1.end(), (int *)(h.data() + t.perm1));
     for (int j = 0; j < d.L2; j++) I2[P2[j]] = j;
   }
-  for (int64_t j1 = 0; j1 < d.H1; j1++) {
+  for (int64_t j1 = 0; j1 < d.H1 && !d.i64(); j1++) {
     for (int l = 0; l < 32; l++) put(h.data(), t.tlane, 32 * j1 + l, unit(j1 * l, d.L), d.f64);
     for (int i = 0; i < d.nb32; i++) {
       // the signed k of the block's first entry: e, or e - pad - L2 in the upper half
@@ -429,7 +429,7 @@ int fft4_init(Fft4Plan *p, int64_t n, void *dev_tables, bool bluestein, bool f64
         put(h.data(), t.tblk2, k2 * d.nb32b + i, unit(k2 * 32 * i, d.L), d.f64);
     }
   }
-  MK_CUDA(cudaMemcpy(dev_tables, h.data(), t.total, cudaMemcpyHostToDevice));
+  MK_CUDA(cudaMemcpy(dev_tables, h.data(), h.size(), cudaMemcpyHostToDevice));
   char *b = (char *)dev_tables;
   d.stw1 = (const void *)(b + t.stw1);
   d.stw2 = (const void *)(b + t.stw2);

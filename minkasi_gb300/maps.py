@@ -180,6 +180,13 @@ class SkyMap:
         new.lims = None if self.lims is None else list(self.lims)
         return new
 
+    def empty_like(self) -> "SkyMap":
+        """A copy whose map is not initialised."""
+        new = copy.copy(self)
+        new.map = torch.empty_like(self.map)
+        new.lims = None if self.lims is None else list(self.lims)
+        return new
+
     def clear(self):
         self.map.zero_()
 
@@ -378,7 +385,7 @@ class Mapset:
     def copy(self) -> "Mapset":
         new = self.__class__()
         for m in self.maps:
-            new.add_map(m.copy())
+            new.add_map(m)  # (which copies it)
         return new
 
     def clear(self):

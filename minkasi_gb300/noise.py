@@ -46,25 +46,26 @@ def clear_plan_cache() -> None:
     _PLAN_CACHE.clear()
 
 
-def dct1(x: torch.Tensor) -> torch.Tensor:
-    """Unnormalised DCT-I along the last axis (fft_r2r, tools/fft.py:290-344)."""
+def dct1(x: torch.Tensor, plan: Optional[K.DCT1] = None) -> torch.Tensor:
+    """Unnormalised DCT-I along the last axis (fft_r2r, tools/fft.py:290-344).
+    ``plan``: a plan of x's shape for a caller with several transforms."""
     x2 = x.reshape(1, -1) if x.dim() == 1 else x
-    out = K.DCT1(x2.shape[0], x2.shape[1], x2.dtype, x2.device)(x2.contiguous())
-    return out.reshape(x.shape)
+    plan = plan or K.DCT1(x2.shape[0], x2.shape[1], x2.dtype, x2.device)
+    return plan(x2.contiguous()).reshape(x.shape)
 
 
-def smooth_many_vecs(vecs: torch.Tensor, fwhm: float = 20.0) -> torch.Tensor:
+def smooth_many_vecs(vecs: torch.Tensor, fwhm: float = 20.0, plan: Optional[K.DCT1] = None) -> torch.Tensor:
     """Gaussian smoothing of each row as a DCT-I convolution (smooth.py:49-78)."""
     n = vecs.shape[1]
-    x = np.arange(n)
     sig = fwhm / np.sqrt(8 * np.log(2))
-    to_conv = np.exp(-0.5 * (x / sig) ** 2)
+    x = torch.arange(n, dtype=torch.float64, device=vecs.device)
+    to_conv = torch.exp(-0.5 * (x / sig) ** 2)
     tot = to_conv[0] + to_conv[-1] + 2 * to_conv[1:-1].sum()
-    to_conv = as_device(to_conv / tot, vecs.dtype, vecs.device)
-    to_conv_ft = dct1(to_conv)
-    xtrans = dct1(vecs)
+    to_conv_ft = dct1((to_conv / tot).to(vecs.dtype))
+    plan = plan or K.DCT1(vecs.shape[0], n, vecs.dtype, vecs.device)
+    xtrans = dct1(vecs, plan)
     xtrans *= to_conv_ft[None, :]
-    back = dct1(xtrans)
+    back = dct1(xtrans, plan)
     return back / (2 * (n - 1))
 
 
@@ -118,8 +119,9 @@ class NoiseSmoothedSVD:
             self.v = u.T.contiguous()
             self.vT = torch.from_numpy(np.linalg.inv(self.v.cpu().numpy())).to(self.v.device).contiguous()
         dat_rot = self.v @ dat
-        dat_trans = dct1(dat_rot)
-        spec = smooth_many_vecs(dat_trans ** 2, fwhm)
+        plan = K.DCT1(dat.shape[0], dat.shape[1], dat.dtype, dat.device)
+        dat_trans = dct1(dat_rot, plan)
+        spec = smooth_many_vecs(dat_trans ** 2, fwhm, plan)
         spec[:, 1:] = 1.0 / spec[:, 1:]
         spec[:, 0] = 0
         self.mywt = spec.contiguous()

@@ -288,15 +288,21 @@ class TodVec:
     def dot(self, mapset: Mapset, mapset_out: Optional[Mapset] = None, report_times: bool = False,
             cache_maps: bool = False, mask: Optional[Mapset] = None):
         """A x summed over TODs, then over ranks (core.py:967-1026)."""
-        if mapset_out is None:
+        fast = not report_times and self._fast(mapset)
+        fresh = mapset_out is None
+        if fresh and fast:
+            mapset_out = mapset.__class__()
+            mapset_out.maps.append(mapset.maps[0].empty_like())
+            mapset_out.nmap = 1
+        elif fresh:
             mapset_out = mapset.copy()
             mapset_out.clear()
         times = np.zeros(self.ntod)
-        if self._fast(mapset) and not report_times:
+        if fast:
             if mask is not None:
                 K.mul(mapset.maps[0].map, mapset.maps[0].map, mask.maps[0].map)
             eng = self.engine(mapset.maps[0])
-            eng.apply(mapset.maps[0].map, mapset_out.maps[0].map, accumulate=True)
+            eng.apply(mapset.maps[0].map, mapset_out.maps[0].map, accumulate=not fresh)
             if mask is not None:
                 K.mul(mapset_out.maps[0].map, mapset_out.maps[0].map, mask.maps[0].map)
         else:
