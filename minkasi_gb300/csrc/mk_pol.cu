@@ -20,6 +20,7 @@
 #include <math.h>
 
 #include "mk_common.cuh"
+#include "mk_wide.cuh"
 
 namespace {
 
@@ -103,24 +104,15 @@ __global__ void __launch_bounds__(256) k_polmap2tod(T *__restrict__ dat, const T
   }
 }
 
-// four consecutive values (16-byte aligned)
-__device__ __forceinline__ void load4(const double *p, double *v) {
-  const double2 a = __ldcs(reinterpret_cast<const double2 *>(p)), b = __ldcs(reinterpret_cast<const double2 *>(p) + 1);
-  v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
-}
-__device__ __forceinline__ void load4(const float *p, float *v) {
-  const float4 a = __ldcs(reinterpret_cast<const float4 *>(p));
-  v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
-}
-
-// Scatter: a warp takes windows of 256 consecutive samples, 8 per lane (16-byte
-// loads if VEC: every array 16-byte aligned).  Runs of equal pixels are summed
+// Scatter: a warp takes windows of 256 consecutive samples, 8 per lane (32-byte
+// loads if VEC: every array 32-byte aligned).  Runs of equal pixels are summed
 // in registers, joined across lanes, written to shared memory in sample order
 // and added to the map component by component: 32 consecutive (run, component)
 // pairs per instruction, which are neighbouring words of the map, as in
-// tod2map's warp_runs.  IQU on 64 x 65,341 samples, 256^2 pixels: FP64 45 us for
-// 51 with an atomic per component and 4-sample run in each thread, FP32 14 for
-// 46; on 256 x 130,978, 1024^2: 235 for 405 and 104 for 304.
+// tod2map's warp_runs.  IQU on 64 x 65,341 samples, 256^2 pixels: FP64 43 us (45
+// with 16-byte loads) for 51 with an atomic per component and 4-sample run in
+// each thread, FP32 13 for 46; on 256 x 130,978, 1024^2: 225 (235) for 405 and
+// 104 for 304.
 // ROWS: d = rowval[i / ndata] (1 if rowval is NULL): hit / weight maps
 constexpr unsigned FULL = 0xffffffffu;
 template <int MODE>
@@ -151,15 +143,11 @@ __global__ void __launch_bounds__(PW<MODE> * 32) k_tod2polmap(T *__restrict__ ma
       d[j] = c[j] = s[j] = T(0);
     }
     if (VEC && m == 8) {
-#pragma unroll
-      for (int h = 0; h < 8; h += 4) {
-        const int4 q = __ldcs(reinterpret_cast<const int4 *>(ipix + i0 + h));
-        p[h] = q.x; p[h + 1] = q.y; p[h + 2] = q.z; p[h + 3] = q.w;
-        if constexpr (!ROWS) load4(dat + i0 + h, d + h);
-        if constexpr (!TRIG) {
-          load4(cs + i0 + h, c + h);
-          load4(sn + i0 + h, s + h);
-        }
+      mk::ld32(ipix + i0, p);
+      if constexpr (!ROWS) mk::ld8_wide(dat + i0, d);
+      if constexpr (!TRIG) {
+        mk::ld8_wide(cs + i0, c);
+        mk::ld8_wide(sn + i0, s);
       }
     } else {
 #pragma unroll
@@ -299,8 +287,7 @@ template <int MODE, typename T, bool TRIG, bool ROWS>
 int tod2polmap_t(void *map, const void *dat, const void *cs, const void *sn, const double *tg,
                  const int32_t *ipix, int64_t n, int64_t npix, const void *rowval, int64_t ndata,
                  cudaStream_t st) {
-  const auto off16 = [](const void *q) { return (uintptr_t)q % 16 != 0; };
-  const bool vec = !off16(ipix) && (ROWS || !off16(dat)) && (TRIG || (!off16(cs) && !off16(sn)));
+  const bool vec = mk::aligned32(ipix) && (ROWS || mk::aligned32(dat)) && (TRIG || (mk::aligned32(cs) && mk::aligned32(sn)));
   auto k = vec ? k_tod2polmap<MODE, T, TRIG, ROWS, true> : k_tod2polmap<MODE, T, TRIG, ROWS, false>;
   k<<<mk_grid((n + 7) / 8, PW<MODE> * 32, 64), PW<MODE> * 32, 0, st>>>((T *)map, (const T *)dat, (const T *)cs, (const T *)sn, tg,
                                                             ipix, n, npix, (const T *)rowval, ndata);

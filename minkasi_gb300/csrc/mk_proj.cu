@@ -14,6 +14,7 @@
 
 #include "mk_async.cuh"
 #include "mk_common.cuh"
+#include "mk_wide.cuh"
 
 namespace {
 
@@ -37,7 +38,11 @@ __device__ __forceinline__ T gather(const T *__restrict__ map, int32_t p, int64_
 // kernel otherwise.
 constexpr int MU = 4;
 
-template <typename T, bool ADD>
+// WIDE (FP64, dat 32-byte aligned): a lane's 4 doubles move in one access, so
+// a warp's store covers 8 whole lines instead of half of 16 twice over
+// (256 x 130,978 FP64 on a 1024^2 map: 82.7 -> 76.1 us, 5.3 TB/s;
+// 64 x 65,341: 14.3 -> 10.6 us).
+template <typename T, bool ADD, bool WIDE>
 __global__ void __launch_bounds__(256) k_map2tod_vec(T *__restrict__ dat, const T *__restrict__ map,
                                                      const int32_t *__restrict__ ipix, int64_t n,
                                                      int64_t npix) {
@@ -72,7 +77,15 @@ __global__ void __launch_bounds__(256) k_map2tod_vec(T *__restrict__ dat, const 
     for (int u = 0; u < MU; u++) {
       const int64_t g = base + 32 * u + lane;
       if (g >= n4) continue;
-      if constexpr (sizeof(T) == 8) {
+      if constexpr (WIDE) {
+        if (ADD) {
+          double a[4];
+          mk::ld32(dat + 4 * g, a);
+#pragma unroll
+          for (int j = 0; j < 4; j++) v[u][j] += a[j];
+        }
+        mk::st32(dat + 4 * g, v[u]);
+      } else if constexpr (sizeof(T) == 8) {
         double2 *d2 = reinterpret_cast<double2 *>(dat) + 2 * g;
         if (ADD) {
           const double2 a = __ldcs(d2), b = __ldcs(d2 + 1);
@@ -509,12 +522,11 @@ int map2tod_t(void *dat, const void *map, const int32_t *ipix, int64_t n, int64_
   bool vec = ((uintptr_t)dat % 16 == 0) && ((uintptr_t)ipix % 16 == 0) && n >= 4;
   const int B = 256;
   if (vec) {
-    if (do_add)
-      k_map2tod_vec<T, true><<<mk_grid_fit(k_map2tod_vec<T, true>, ((n >> 2) + MU - 1) / MU, B), B, 0, st>>>(
-          (T *)dat, (const T *)map, ipix, n, npix);
-    else
-      k_map2tod_vec<T, false><<<mk_grid_fit(k_map2tod_vec<T, false>, ((n >> 2) + MU - 1) / MU, B), B, 0, st>>>(
-          (T *)dat, (const T *)map, ipix, n, npix);
+    constexpr bool F64 = sizeof(T) == 8;
+    const bool wide = F64 && mk::aligned32(dat);
+    auto k = do_add ? (wide ? k_map2tod_vec<T, true, F64> : k_map2tod_vec<T, true, false>)
+                    : (wide ? k_map2tod_vec<T, false, F64> : k_map2tod_vec<T, false, false>);
+    k<<<mk_grid_fit(k, ((n >> 2) + MU - 1) / MU, B), B, 0, st>>>((T *)dat, (const T *)map, ipix, n, npix);
   } else {
     if (do_add)
       k_map2tod_scalar<T, true><<<mk_grid_fit(k_map2tod_scalar<T, true>, n, B), B, 0, st>>>(
@@ -541,9 +553,7 @@ int map2tod_t(void *dat, const void *map, const int32_t *ipix, int64_t n, int64_
 // their places), and the warp then adds them 32 at a time: consecutive runs of
 // a scan lie on neighbouring pixels, so one instruction's atomics share
 // 32-byte sectors of the map, and L2 takes a sector at once.  key, sum: room
-// for 256 runs, this warp's own.  256 x 130,978 on 1024^2 pixels (3.6 samples a
-// run): FP64 85 us for 92 with each lane issuing its runs one by one, FP32 66
-// for 89; 128 x 383,329 on 2048^2 (1.9 a run): 157 for 186, 119 for 165.
+// for 256 runs, this warp's own.
 template <typename T>
 __device__ __forceinline__ void warp_runs(T *__restrict__ map, const int32_t (&p)[8], const T (&v)[8], int m,
                                           int lane, int64_t npix, int32_t *key, T *sum) {
@@ -609,7 +619,13 @@ __device__ __forceinline__ void warp_runs(T *__restrict__ map, const int32_t (&p
   __syncwarp();
 }
 
-template <typename T>
+// WIDE: ipix and dat 32-byte aligned (else 16).  The L1's tag stage bounds the
+// kernel (91 % busy with 16-byte loads, FP64), so half the load instructions
+// count: 256 x 130,978 FP64 on a 1024^2 map 84.7 -> 79.8 us (5.0 TB/s),
+// 128 x 383,329 on 2048^2 157 -> 142 us, 64 x 65,341 15.2 -> 14.7 us; FP32
+// unchanged (67.0 us).  Two groups of 4 samples a lane (coalesced 16-byte
+// loads, two prefix sums) took 89.8, 142 and 18.8 us.
+template <typename T, bool WIDE>
 __global__ void __launch_bounds__(256, 5) k_tod2map_atomic8(T *__restrict__ map, const T *__restrict__ dat,
                                                          const int32_t *__restrict__ ipix, int64_t n,
                                                          int64_t npix) {
@@ -625,8 +641,13 @@ __global__ void __launch_bounds__(256, 5) k_tod2map_atomic8(T *__restrict__ map,
     int32_t p[8];
     T v[8];
     if (m == 8) {
-      load8i(ipix + i0, p);
-      load8(dat + i0, v);
+      if (WIDE) {
+        mk::ld32(ipix + i0, p);
+        mk::ld8_wide(dat + i0, v);
+      } else {
+        load8i(ipix + i0, p);
+        load8(dat + i0, v);
+      }
     } else {
 #pragma unroll
       for (int j = 0; j < 8; j++) {
@@ -646,7 +667,8 @@ int tod2map_t(void *map, const void *dat, const int32_t *ipix, int64_t n, int64_
     // more CTAs than fit at once: the warps' windows are short, and a deep
     // queue of CTAs keeps every SM's atomic issue busy to the end (64 CTAs per
     // SM against 16: 66 and 70 us on 256 x 130,978 in FP32)
-    k_tod2map_atomic8<T><<<mk_grid((n + 7) / 8, B, 64), B, 0, st>>>((T *)map, (const T *)dat, ipix, n, npix);
+    auto k = mk::aligned32(dat) && mk::aligned32(ipix) ? k_tod2map_atomic8<T, true> : k_tod2map_atomic8<T, false>;
+    k<<<mk_grid((n + 7) / 8, B, 64), B, 0, st>>>((T *)map, (const T *)dat, ipix, n, npix);
     return mk::launch_status("mk_tod2map");
   }
   constexpr int U = 4;

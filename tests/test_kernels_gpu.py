@@ -82,6 +82,38 @@ def test_map2tod_unaligned_view(K):
     assert np.array_equal(d.cpu().numpy(), m[ipix])
 
 
+@pytest.mark.parametrize("dt", [torch.float64, torch.float32])
+@pytest.mark.parametrize("off", [0, 1, 2, 4, 8])
+@pytest.mark.parametrize("n", [7, 8, 256, 1027])
+def test_projections_at_every_alignment(K, n, off, dt):
+    """Views that start 0 to 8 elements past a 32-byte boundary (data and
+    pixels by the same number of elements, and the data alone): the 32-byte,
+    16-byte and single accesses give the same samples, and a TOD's
+    neighbours in memory stay as they were."""
+    rng = np.random.default_rng(n + off)
+    npix = 61
+    ipix = (np.mod(np.cumsum(rng.integers(-1, 2, size=n)) // 3, npix + 4) - 2).astype(np.int32)
+    ok = (ipix >= 0) & (ipix < npix)
+    m0, d0 = rng.integers(-50, 50, size=npix).astype(float), rng.integers(-50, 50, size=n).astype(float)
+    got = np.where(ok, m0[np.clip(ipix, 0, npix - 1)], 0)
+    ref = m0.copy()
+    np.add.at(ref, ipix[ok], d0[ok])
+    for poff in (off, 0):
+        pix = torch.zeros(n + poff, dtype=torch.int32, device=cuda)[poff:]
+        pix.copy_(dev(ipix))
+        base = torch.full((n + off + 4,), 7.0, dtype=dt, device=cuda)
+        d = base[off : off + n]
+        d.copy_(dev(d0, dt))
+        m = dev(m0, dt)
+        K.tod2map(m, d, pix)  # whole numbers: every order of the sums is exact
+        assert np.array_equal(m.cpu().double().numpy(), ref)
+        K.map2tod(d, dev(m0, dt), pix, True)
+        assert np.array_equal(d.cpu().double().numpy(), d0 + got)
+        K.map2tod(d, dev(m0, dt), pix, False)
+        assert np.array_equal(d.cpu().double().numpy(), got)
+        assert bool((base[:off] == 7).all()) and bool((base[off + n :] == 7).all())
+
+
 def test_tod2map_golden(K, gold):
     g = gold("proj.npz")
     m = dev(g["map"])
