@@ -512,6 +512,34 @@ def test_sliced_fp64_rotation_tile_edges(K, nd, n):
     assert plan.status() == 0
 
 
+@pytest.mark.parametrize("nd,n", [(63, 33), (64, 200), (65, 31), (130, 129), (192, 97), (256, 20001), (257, 65)])
+def test_sliced_fp64_rotation_value_ranges(K, nd, n):
+    """The slicing kernel's forms (up to 64, 128 and 256 detectors in registers,
+    more in two passes) on columns of every kind: entries from 2^-60 of the
+    largest down to zero, whole columns near the top of the range, denormal and
+    zero columns, cancellation to zero, NaN.  Bound as in the test above, plus
+    the rounding of denormal results."""
+    rng = np.random.default_rng(nd + n)
+    A = rng.standard_normal((nd, nd)) / nd
+    X = rng.standard_normal((nd, n)) * 2.0 ** rng.integers(-60, 1, size=(nd, n))
+    X[:, 1] *= 2.0 ** 1000
+    X[:, 2] *= 2.0 ** -1040
+    X[:, 3] = 0
+    X[:, 4] = 5e-324
+    X[rng.integers(0, nd, 5), rng.integers(5, n - 2, 5)] = 0
+    A[nd - 1], X[:, 0] = np.where(np.arange(nd) % 2, 1.0, -1.0), 0.75  # row nd - 1: 0 or -0.75
+    want = (A.astype(np.longdouble) @ X.astype(np.longdouble))
+    X[0, n - 1] = np.nan
+    plan = K.NoisePlan(nd, n, torch.float64)
+    got = plan.rotate(dev(A), dev(X), rot_mode=4).cpu().numpy()
+    assert np.isnan(got[:, n - 1]).all()
+    got, want = got[:, : n - 1], want[:, : n - 1]
+    scale = np.abs(A).max(1)[:, None].astype(np.longdouble) * np.abs(X[:, : n - 1]).max(0)[None, :]
+    assert (np.abs(got - want) <= 4 * nd * 2.0 ** -53 * scale + 2.0 ** -53 * np.abs(want) + np.longdouble(5e-324)).all()
+    assert (got[:, 3] == 0).all() and got[nd - 1, 0] == want[nd - 1, 0]
+    assert plan.status() == 0
+
+
 @pytest.mark.parametrize("nd,n", [(1, 2), (2, 700), (7, 63), (8, 64), (9, 65), (53, 2001), (64, 513), (257, 130)])
 def test_f64_rotation(K, nd, n):
     """The FP64-pipe rotation (rot_mode 0) around its blocks (8 detectors, 64
