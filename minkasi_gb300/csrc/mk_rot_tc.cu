@@ -30,11 +30,14 @@
 //
 // Roles: MT x 4 split warps; MT x 4 epilogue warps (warp w reads TMEM lanes
 // 32 (w % 4) .. of its tile and stores per detector 32 consecutive samples);
-// one warp whose first lane issues the image copies and the MMAs.  Two
-// shared-memory stages: the MMAs of chunk g run while chunk g + 1 is split.
+// one warp of which one lane issues the image copies and the MMAs (the warp
+// stays converged: with operands in uniform registers a chunk's MMAs issue
+// faster than they run; 256 x 450,561 309 -> 292 us, 256 x 130,978 111 -> 105, no
+// change below 256 detectors).  Two shared-memory stages: the MMAs of chunk g
+// run while chunk g + 1 is split.
 // Measured against the 3xTF32 kernels before it (8 B per value, one tile per
-// pass; error against FP64 in brackets): 256 x 450,561 0.31 ms (1.7e-6) for
-// 0.47 (1.9e-6), 256 x 130,978 0.110 for 0.146, 128 x 563,201 0.151 (8.2e-7)
+// pass; error against FP64 in brackets): 256 x 450,561 0.29 ms (1.7e-6) for
+// 0.47 (1.9e-6), 256 x 130,978 0.105 for 0.146, 128 x 563,201 0.151 (8.2e-7)
 // for 0.259 (9.7e-7), 64 x 65,341 0.017 for 0.025.
 // Every wait is bounded and also polls the CTA's abort flag, so a timeout in
 // one role ends all of them; the MMA thread then drains its outstanding
@@ -83,28 +86,35 @@ __device__ __forceinline__ void split2(float a, float b, uint32_t &h, uint32_t &
 // tile of 64-byte rows with the 64-byte swizzle
 __device__ __forceinline__ uint32_t sw64_off(uint32_t r, uint32_t c) { return r * 64u + ((c ^ ((r >> 1) & 3u)) << 4); }
 
-// shared-memory matrix descriptor: K-major, SWIZZLE_64B, 8-row groups 512 B apart
-__device__ __forceinline__ uint64_t sdesc(uint32_t saddr) {
-  uint64_t d = 0;
-  d |= (uint64_t)((saddr & 0x3FFFFu) >> 4);  // start address
-  d |= (uint64_t)1 << 16;                    // leading byte offset (unused)
-  d |= (uint64_t)(512u >> 4) << 32;          // stride byte offset
-  d |= (uint64_t)1 << 46;                    // descriptor version (tcgen05)
-  d |= (uint64_t)4 << 61;                    // swizzle: 64B
-  return d;
+// shared-memory matrix descriptors: K-major, SWIZZLE_64B, 8-row groups 512 B
+// apart.  Low word: address / 16 (and an unused leading offset), so a step
+// within a stage is an addition; high word: stride 512 B, version (tcgen05),
+// swizzle 64B
+__device__ __forceinline__ uint32_t sdesc_lo(uint32_t saddr) { return (saddr >> 4) | (1u << 16); }
+constexpr uint32_t SDESC_HI = (512u >> 4) | (1u << 14) | (4u << 29);
+
+// one lane of a converged warp, the same one at every call
+__device__ __forceinline__ uint32_t elect_one() {
+  uint32_t e;
+  asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}" : "=r"(e));
+  return e;
 }
 
-__device__ __forceinline__ void mma_bf16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                         uint32_t accum) {
+// MMA by the lane whose lead is set (executed by the whole warp, so that the
+// operands stay in uniform registers); acc: add to the accumulator
+__device__ __forceinline__ void mma_bf16(uint32_t lead, uint32_t tmem_d, uint32_t alo, uint32_t blo, uint32_t idesc,
+                                         uint32_t acc) {
   asm volatile(
-      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-      " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem_d),
-      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accum));
+      "{\n .reg .pred p, l;\n .reg .b64 a, b;\n setp.ne.b32 p, %4, 0;\n setp.ne.b32 l, %6, 0;\n"
+      " mov.b64 a, {%1, %5};\n mov.b64 b, {%2, %5};\n"
+      " @l tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, p;\n}\n" ::"r"(tmem_d),
+      "r"(alo), "r"(blo), "r"(idesc), "r"(acc), "n"(SDESC_HI), "r"(lead));
 }
 
-__device__ __forceinline__ void mma_commit(uint64_t *bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                   smem_u32(bar))
+__device__ __forceinline__ void mma_commit(uint32_t lead, uint64_t *bar) {
+  asm volatile("{\n .reg .pred l;\n setp.ne.b32 l, %1, 0;\n"
+               " @l tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}" ::"r"(smem_u32(bar)),
+               "r"(lead)
                : "memory");
 }
 
@@ -147,6 +157,13 @@ __device__ __forceinline__ bool ws_wait(uint64_t *bar, uint32_t parity, volatile
   }
   *abort_flag = 1;
   return false;
+}
+
+// a converged warp waits; true if every lane saw the phase complete
+__device__ __forceinline__ bool warp_wait(uint64_t *bar, uint32_t parity, volatile int *abort_flag) {
+  const bool ok = __all_sync(0xffffffffu, ws_wait(bar, parity, abort_flag));
+  asm volatile("tcgen05.fence::after_thread_sync;");
+  return ok;
 }
 
 // The job (TOD) that owns tile t of the launch; jobs are sorted by tile0 and
@@ -264,57 +281,54 @@ __global__ void __launch_bounds__((8 * MT + 1) * 32, 3 - MT)
       }
     }
   } else if (warp == NSPLIT + NEPI) {
-    // ---- image copies and MMAs (one thread)
-    if (lane == 0) {
-      const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(ndet >> 3) << 17) |
-                             ((uint32_t)(TILE_M >> 4) << 24);
-      uint32_t g = 0, it = 0;
-      int cur = 0;
-      bool ok = true;
-      for (int64_t item = blockIdx.x; item < nitem && ok && !*abort_flag; item += gridDim.x, it++) {
-        cur = job_at(jobs, njobs, item, cur);
-        const char *bimg = jobs[cur].bimg;
-        const uint32_t ab = nbuf == 2 ? it & 1 : 0, au = nbuf == 2 ? it >> 1 : it;
-        for (int c = 0; c < nchunk; c++, g++) {
-          const uint32_t s = g % NSTAGE, use = g / NSTAGE;
-          unsigned char *st = smem + s * stage_bytes;
-          if (g >= NSTAGE && !ws_wait(&mma_done[s], (use - 1) & 1, abort_flag)) {
-            ok = false;
-            break;
-          }
+    // ---- image copies and MMAs (one lane issues; the warp stays converged)
+    const uint32_t lead = elect_one();
+    const uint32_t idesc =
+        (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(ndet >> 3) << 17) | ((uint32_t)(TILE_M >> 4) << 24);
+    uint32_t it = 0;
+    int cur = 0;
+    bool ok = true;
+    for (int64_t item = blockIdx.x; item < nitem && ok; item += gridDim.x, it++) {
+      cur = job_at(jobs, njobs, item, cur);
+      const char *bimg = jobs[cur].bimg;
+      const uint32_t ab = nbuf == 2 ? it & 1 : 0, au = nbuf == 2 ? it >> 1 : it;
+      for (int c = 0; c < nchunk; c++) {
+        const uint32_t g = g_issued, s = g % NSTAGE, use = g / NSTAGE;
+        unsigned char *st = smem + s * stage_bytes;
+        if (g >= NSTAGE && !warp_wait(&mma_done[s], (use - 1) & 1, abort_flag)) {
+          ok = false;
+          break;
+        }
+        if (lead) {
           mbar_expect_tx(&full_b[s], 3 * b_part);
           bulk_g2s(st + MT * A_TILE, bimg + (size_t)c * 3 * b_part, 3 * b_part, &full_b[s]);
-          g_copied = g + 1;
-          if (c == 0 && au >= 1 && !ws_wait(&acc_empty[ab], (au - 1) & 1, abort_flag)) ok = false;
-          if (!ok || !ws_wait(&full_b[s], use & 1, abort_flag) || !ws_wait(&full_a[s], use & 1, abort_flag)) {
-            ok = false;
-            break;
-          }
-          asm volatile("tcgen05.fence::after_thread_sync;");
-          const uint32_t sb = smem_u32(st + MT * A_TILE);
-#pragma unroll
-          for (int mt = 0; mt < MT; mt++) {
-            const uint32_t sa = smem_u32(st) + mt * A_TILE;
-            const uint32_t dacc = tmem + (ab * MT + mt) * (uint32_t)ndet;
-#pragma unroll
-            for (int k16 = 0; k16 < KC / 16; k16++) {
-              const uint32_t ko = k16 * 32;
-              const uint64_t ah = sdesc(sa + ko), am = sdesc(sa + A_PART + ko), al = sdesc(sa + 2 * A_PART + ko);
-              const uint64_t bh = sdesc(sb + ko), bm = sdesc(sb + b_part + ko), bl = sdesc(sb + 2 * b_part + ko);
-              mma_bf16(dacc, ah, bl, idesc, c == 0 && k16 == 0 ? 0u : 1u);
-              mma_bf16(dacc, al, bh, idesc, 1u);
-              mma_bf16(dacc, am, bm, idesc, 1u);
-              mma_bf16(dacc, ah, bm, idesc, 1u);
-              mma_bf16(dacc, am, bh, idesc, 1u);
-              mma_bf16(dacc, ah, bh, idesc, 1u);
-            }
-          }
-          mma_commit(&mma_done[s]);
-          g_issued = g + 1;
         }
+        g_copied = g + 1;
+        if (c == 0 && au >= 1) ok = warp_wait(&acc_empty[ab], (au - 1) & 1, abort_flag);
+        ok = ok && warp_wait(&full_b[s], use & 1, abort_flag) && warp_wait(&full_a[s], use & 1, abort_flag);
         if (!ok) break;
-        mma_commit(&acc_full[ab]);
+        const uint32_t ad = sdesc_lo(smem_u32(st)), bd = sdesc_lo(smem_u32(st + MT * A_TILE));
+        constexpr uint32_t AP = A_PART / 16;
+        const uint32_t bp = b_part / 16;
+#pragma unroll
+        for (int mt = 0; mt < MT; mt++) {
+          const uint32_t dacc = tmem + (ab * MT + mt) * (uint32_t)ndet;
+#pragma unroll
+          for (int k16 = 0; k16 < KC / 16; k16++) {
+            const uint32_t h = ad + (mt * A_TILE + k16 * 32) / 16, b = bd + k16 * 2;
+            mma_bf16(lead, dacc, h, b + 2 * bp, idesc, c == 0 && k16 == 0 ? 0u : 1u);
+            mma_bf16(lead, dacc, h + 2 * AP, b, idesc, 1u);
+            mma_bf16(lead, dacc, h + AP, b + bp, idesc, 1u);
+            mma_bf16(lead, dacc, h, b + bp, idesc, 1u);
+            mma_bf16(lead, dacc, h + AP, b, idesc, 1u);
+            mma_bf16(lead, dacc, h, b, idesc, 1u);
+          }
+        }
+        mma_commit(lead, &mma_done[s]);
+        g_issued = g + 1;
       }
+      if (!ok) break;
+      mma_commit(lead, &acc_full[ab]);
     }
   } else {
     // ---- epilogue role
@@ -326,11 +340,7 @@ __global__ void __launch_bounds__((8 * MT + 1) * 32, 3 - MT)
     for (int64_t item = blockIdx.x; item < nitem; item += gridDim.x, it++) {
       cur = job_at(jobs, njobs, item, cur);
       const uint32_t ab = nbuf == 2 ? it & 1 : 0, au = nbuf == 2 ? it >> 1 : it;
-      // every lane waits; the warp goes on only if all of them saw the
-      // phase complete (tcgen05.ld below needs the whole warp converged)
-      const bool okw = ws_wait(&acc_full[ab], au & 1, abort_flag);
-      if (!__all_sync(0xffffffffu, okw)) break;
-      asm volatile("tcgen05.fence::after_thread_sync;");
+      if (!warp_wait(&acc_full[ab], au & 1, abort_flag)) break;
       const mk::RotJob &J = jobs[cur];
       const int64_t my = ((item - J.tile0) * MT + mt) * TILE_M + row, ncol = J.ncol, ldr = J.ldr;
       float *R = J.R;
