@@ -12,6 +12,7 @@
 // precision.
 #include <cufft.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstdlib>
 #include <utility>
@@ -417,6 +418,22 @@ struct Cfg {
   static_assert(NT % FB == 0, "a thread keeps its slot through a stage");
 };
 
+// threads to launch for ntile tiles of FB transforms with smem bytes each: NT,
+// or half of it where CTAs of NT threads would need a second, mostly empty
+// wave and CTAs of half the size, of which twice as many fit the registers, all
+// run at once.  Beyond one wave the larger CTAs hide latency better (256 x
+// 130,978 FP32: 165 us for 198).  DCT with NT and with half, FP32: 64 x 65,341
+// (384 tiles a pass; 304 CTAs of 512 threads run at once) 29.4 and 24.1 us, 96 x
+// 65,341 34.0 and 29.8, 48 x 130,978 41.6 and 35.6.
+template <int FB>
+int threads_for(int64_t ntile, size_t smem) {
+  constexpr int NT = Cfg<FB>::NT, HALF = NT / 2;
+  if (HALF < 256) return NT;
+  const int64_t sms = sm_count(), fit = 227 * 1024 / (int64_t)(smem + 1024);
+  const int64_t full = std::min<int64_t>(Cfg<FB>::MINB, fit), half = std::min<int64_t>(2 * Cfg<FB>::MINB, fit);
+  return ntile > full * sms && ntile <= half * sms ? HALF : NT;
+}
+
 // row pitch (C) of a tile of FB interleaved transforms: odd, so the
 // rows fall in distinct shared-memory banks
 __host__ __device__ __forceinline__ int pitch_odd(int Ls) { return Ls | 1; }
@@ -435,7 +452,7 @@ __host__ __device__ __forceinline__ int pitch_odd(int Ls) { return Ls | 1; }
 template <int R, int FB>
 __device__ __forceinline__ void stage_dit(C *slot, int Ls, int Ns, float invNs, const C *stw) {
   const int nq = Ls / R;
-  for (int q = threadIdx.x / FB; q < nq; q += Cfg<FB>::NT / FB) {
+  for (int q = threadIdx.x / FB; q < nq; q += (int)blockDim.x / FB) {
     const int g = __float2int_rz(((float)q + 0.5f) * invNs);
     const int k = q - g * Ns;
     C *a = slot + g * Ns * R + k;
@@ -488,7 +505,7 @@ __device__ __forceinline__ void astage_first(C *sbuf, int pitch, int Ls, const P
   const int nq = Ls / R, b = threadIdx.x % FB;
   if (b >= pa.nb) return;
   const int step = pa.L1 * nq;
-  for (int q = threadIdx.x / FB; q < nq; q += Cfg<FB>::NT / FB) {
+  for (int q = threadIdx.x / FB; q < nq; q += (int)blockDim.x / FB) {
     const int j = pa.j1_0 + b + pa.L1 * __ldg(pa.iperm + q * R);
     C v[R];
 #pragma unroll
@@ -522,7 +539,7 @@ template <int R, int FB>
 __device__ __forceinline__ void astage_last(const C *sbuf, int pitch, int Ns, const C *stw, const PassA &pa,
                                             const Fft4Dev &p, C *Tp) {
   const int h2 = p.L2 / 2;
-  for (int bf = threadIdx.x; bf < FB * Ns; bf += Cfg<FB>::NT) {
+  for (int bf = threadIdx.x; bf < FB * Ns; bf += (int)blockDim.x) {
     const int b = bf / Ns, q = bf - b * Ns;
     if (b >= pa.nb) break;  // b grows with bf
     const C *a = sbuf + b * pitch + q;
@@ -586,7 +603,7 @@ __global__ void __launch_bounds__(Cfg<FB>::NT, Cfg<FB>::MINB) k_fft4_a(const RT 
   if (S == 0 && tid < pa.nb) sbuf[tid * pitch] = a_input<AM>(pa, pa.j1_0 + tid);  // L2 == 1
   __syncthreads();
   const int k2 = tid & 31, h2 = L2 / 2;
-  for (int b = tid >> 5; b < pa.nb; b += Cfg<FB>::NT / 32) {
+  for (int b = tid >> 5; b < pa.nb; b += (int)blockDim.x / 32) {
     const int j1 = pa.j1_0 + b;
     const RowTw tw = row_tw(p, j1);
     C *row = Tp + j1 * p.P;
@@ -676,7 +693,7 @@ __device__ __forceinline__ void bput_epi(C *v, int q, int Ns, const PassB &pb) {
 template <int R, int BM, int FB, bool LAST>
 __device__ __forceinline__ void bstage_first(C *slot, int Ls, const TCol &col, const int *iperm, const PassB &pb) {
   const int nq = Ls / R;
-  for (int q = threadIdx.x / FB; q < nq; q += Cfg<FB>::NT / FB) {
+  for (int q = threadIdx.x / FB; q < nq; q += (int)blockDim.x / FB) {
     C v[R];
     bload<R, BM, FB>(v, col, __ldg(iperm + q * R), nq);
     Dft<R>::run(v);
@@ -692,7 +709,7 @@ __device__ __forceinline__ void bstage_first(C *slot, int Ls, const TCol &col, c
 
 template <int R, int BM, int FB>
 __device__ __forceinline__ void bstage_last(const C *slot, int Ns, const C *stw, const PassB &pb) {
-  for (int q = threadIdx.x / FB; q < Ns; q += Cfg<FB>::NT / FB) {
+  for (int q = threadIdx.x / FB; q < Ns; q += (int)blockDim.x / FB) {
     const C *a = slot + q;
     C v[R];
 #pragma unroll
@@ -793,7 +810,7 @@ __device__ __forceinline__ int c_col(const PassC &pc, int b) {
 template <int R, int FB>
 __device__ __forceinline__ void cstage_first(C *slot, int Ns, const C *stw, const TCol &col) {
   constexpr int H = FB / 2;
-  for (int q = threadIdx.x / H; q < Ns; q += Cfg<FB>::NT / H) {
+  for (int q = threadIdx.x / H; q < Ns; q += (int)blockDim.x / H) {
     C v[R];
     bload<R, BM_DCT, FB>(v, col, q, Ns);
     Dft<R>::run(v);
@@ -811,7 +828,7 @@ template <int R, int FB>
 __device__ __forceinline__ void cstage_dif(C *slot, int Ls, int Ns, float invNs, const C *stw) {
   constexpr int H = FB / 2;
   const int nq = Ls / R;
-  for (int q = threadIdx.x / H; q < nq; q += Cfg<FB>::NT / H) {
+  for (int q = threadIdx.x / H; q < nq; q += (int)blockDim.x / H) {
     const int g = __float2int_rz(((float)q + 0.5f) * invNs);
     const int k = q - g * Ns;
     C *a = slot + g * Ns * R + k;
@@ -838,7 +855,7 @@ __device__ __forceinline__ void cstage_mid(C *slot, C *slot_p, int k2, int kp, i
                                            const int *perm, const TCol &col, const PassC &pc) {
   constexpr int H = FB / 2;
   const int nq = L1 / R, step = pc.L2 * nq;
-  for (int q = threadIdx.x / H; q < nq; q += Cfg<FB>::NT / H) {
+  for (int q = threadIdx.x / H; q < nq; q += (int)blockDim.x / H) {
     const int kq = __ldg(iperm + q * R);
     C *a = slot + q * R;
     C v[R];
@@ -886,7 +903,7 @@ __device__ __forceinline__ void put_v(const PassC &pc, const Fft4Dev &p, int k2,
 template <int R, int FB>
 __device__ __forceinline__ void cstage_last(const C *sbuf, int pitch, int Ns, const C *stw, const PassC &pc,
                                             const Fft4Dev &p) {
-  for (int bf = threadIdx.x; bf < FB * Ns; bf += Cfg<FB>::NT) {
+  for (int bf = threadIdx.x; bf < FB * Ns; bf += (int)blockDim.x) {
     const int b = bf / Ns, q = bf - b * Ns;
     const int k2 = c_col<FB>(pc, b);
     if (k2 < 0) continue;
@@ -927,7 +944,7 @@ __global__ void __launch_bounds__(Cfg<FB>::NT, Cfg<FB>::MINB) k_fft4_conv(const 
     if (on)
       MK_RADIX_SWITCH(p.r1[0], (cstage_mid<RR, FB, true>(slot, slot_p, k2, kp, L1, p.iperm1, p.perm1, col, pc)));
     __syncthreads();
-    for (int e = threadIdx.x; e < FB * L1; e += Cfg<FB>::NT) {
+    for (int e = threadIdx.x; e < FB * L1; e += (int)blockDim.x) {
       const int be = e / L1, o1 = e - be * L1, ke = c_col<FB>(pc, be);
       if (ke >= 0) put_v(pc, p, ke, o1, sbuf[be * pitch + o1]);
     }
@@ -1001,23 +1018,23 @@ int dct_launch(const Fft4Plan &p, const RT *x, int64_t ldx, int64_t nrow, C *T, 
 #if MK_FFT4_SMOOTH
   if (!d.blue) {
     const dim3 gb((d.H2 + fb - 1) / fb, np);
-    if (hia) k_fft4_a<AM_DCT, FB_HI><<<ga, Cfg<FB_HI>::NT, smem_a, st>>>(x, ldx, nrow, T, d);
-    else k_fft4_a<AM_DCT, FB_LO><<<ga, Cfg<FB_LO>::NT, smem_a, st>>>(x, ldx, nrow, T, d);
+    if (hia) k_fft4_a<AM_DCT, FB_HI><<<ga, threads_for<FB_HI>((int64_t)ga.x * np, smem_a), smem_a, st>>>(x, ldx, nrow, T, d);
+    else k_fft4_a<AM_DCT, FB_LO><<<ga, threads_for<FB_LO>((int64_t)ga.x * np, smem_a), smem_a, st>>>(x, ldx, nrow, T, d);
     if ((rc = launch_status("fft4 pass A"))) return rc;
-    if (hib) k_fft4_b<BM_DCT, FB_HI><<<gb, Cfg<FB_HI>::NT, smem_b, st>>>(T, nrow, out, ldo, w, ldw, epi, d);
-    else k_fft4_b<BM_DCT, FB_LO><<<gb, Cfg<FB_LO>::NT, smem_b, st>>>(T, nrow, out, ldo, w, ldw, epi, d);
+    if (hib) k_fft4_b<BM_DCT, FB_HI><<<gb, threads_for<FB_HI>((int64_t)gb.x * np, smem_b), smem_b, st>>>(T, nrow, out, ldo, w, ldw, epi, d);
+    else k_fft4_b<BM_DCT, FB_LO><<<gb, threads_for<FB_LO>((int64_t)gb.x * np, smem_b), smem_b, st>>>(T, nrow, out, ldo, w, ldw, epi, d);
     return launch_status("fft4 pass B");
   }
 #else
   MK_CHECK_ARG(d.blue, "fft4: plan does not match the call");
 #endif
   C *V = T + npairs * d.tsz;
-  if (hia) k_fft4_a<AM_BLUE, FB_HI><<<ga, Cfg<FB_HI>::NT, smem_a, st>>>(x, ldx, nrow, T, d);
-  else k_fft4_a<AM_BLUE, FB_LO><<<ga, Cfg<FB_LO>::NT, smem_a, st>>>(x, ldx, nrow, T, d);
+  if (hia) k_fft4_a<AM_BLUE, FB_HI><<<ga, threads_for<FB_HI>((int64_t)ga.x * np, smem_a), smem_a, st>>>(x, ldx, nrow, T, d);
+  else k_fft4_a<AM_BLUE, FB_LO><<<ga, threads_for<FB_LO>((int64_t)ga.x * np, smem_a), smem_a, st>>>(x, ldx, nrow, T, d);
   if ((rc = launch_status("fft4 Bluestein pass A"))) return rc;
   const dim3 gc((d.H2 + fb / 2 - 1) / (fb / 2), np);
-  if (hib) k_fft4_conv<FB_HI><<<gc, Cfg<FB_HI>::NT, smem_b, st>>>(T, V, d);
-  else k_fft4_conv<FB_LO><<<gc, Cfg<FB_LO>::NT, smem_b, st>>>(T, V, d);
+  if (hib) k_fft4_conv<FB_HI><<<gc, threads_for<FB_HI>((int64_t)gc.x * np, smem_b), smem_b, st>>>(T, V, d);
+  else k_fft4_conv<FB_LO><<<gc, threads_for<FB_LO>((int64_t)gc.x * np, smem_b), smem_b, st>>>(T, V, d);
   if ((rc = launch_status("fft4 Bluestein middle pass"))) return rc;
   // pass B on the transposed shape: length L2 over the rows of V, outputs
   // o1 + L1 o2
@@ -1031,8 +1048,8 @@ int dct_launch(const Fft4Plan &p, const RT *x, int64_t ldx, int64_t nrow, C *T, 
   std::swap(tr.stw1, tr.stw2);
   std::swap(tr.iperm1, tr.iperm2);
   const dim3 gt((tr.L2 + fa - 1) / fa, np);
-  if (hia) k_fft4_b<BM_BLUE, FB_HI><<<gt, Cfg<FB_HI>::NT, smem_a, st>>>(V, nrow, out, ldo, w, ldw, epi, tr);
-  else k_fft4_b<BM_BLUE, FB_LO><<<gt, Cfg<FB_LO>::NT, smem_a, st>>>(V, nrow, out, ldo, w, ldw, epi, tr);
+  if (hia) k_fft4_b<BM_BLUE, FB_HI><<<gt, threads_for<FB_HI>((int64_t)gt.x * np, smem_a), smem_a, st>>>(V, nrow, out, ldo, w, ldw, epi, tr);
+  else k_fft4_b<BM_BLUE, FB_LO><<<gt, threads_for<FB_LO>((int64_t)gt.x * np, smem_a), smem_a, st>>>(V, nrow, out, ldo, w, ldw, epi, tr);
   return launch_status("fft4 Bluestein last pass");
 }
 

@@ -552,6 +552,19 @@ def test_f64_rotation(K, nd, n):
     assert (np.abs(got - Al @ Xl) <= nd * 2.0 ** -53 * (np.abs(A) @ np.abs(X))).all()
 
 
+@pytest.mark.parametrize("nd,n", [(52, 65341), (64, 65341), (96, 65341), (48, 130978), (33, 72140)])
+def test_dct1_f32_one_wave_of_half_size_blocks(K, nd, n):
+    """Row counts whose tiles need more blocks than run at once at full size:
+    they run with half the threads (smooth lengths and a Bluestein one), with the
+    rounding of the other forms: 2^-24 for each of at most log2(4 n) additions
+    in each of the (at most three) transforms, in the 2-norm."""
+    import scipy.fft as sf
+    x = np.random.default_rng(n).standard_normal((nd, n)).astype(np.float32)
+    want = sf.dct(x.astype(np.float64), type=1, axis=-1)
+    got = K.DCT1(nd, n, torch.float32)(dev(x)).cpu().numpy()
+    assert rel(got, want) < 3 * np.log2(4 * n) * 2.0 ** -24
+
+
 def test_apply_noise_golden_f64_sliced_rotation(K, gold):
     """The reference's apply_noise (noise.npz) with the sliced FP64 rotation."""
     g = gold("noise.npz")
