@@ -692,8 +692,8 @@ def solve_c1(dev, tol=1e-6):
 def precision_c1(tv, m, hits, pre, ml, op64, dev):
     """The precision configuration on the 1-TOD inputs: a system with a known
     solution, b = A s (FP64 operator) for a seeded sky s on the hit pixels,
-    solved from x0 = 0 by the mixed-precision PCG (FP32 operator with 3xTF32
-    tensor-core rotations; FP64 dots and residual replacement) and by
+    solved from x0 = 0 by the mixed-precision PCG (FP32 operator with
+    tensor-core rotations of three bf16 parts; FP64 dots and residual replacement) and by
     classic iterative refinement (FP64 residual, 20 FP32 inner PCG
     iterations per step).  At every FP64 residual evaluation: the true
     residual and the map error against s, hit-region mean removed (A

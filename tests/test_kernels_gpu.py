@@ -557,7 +557,7 @@ def test_dct1_f32_one_wave_of_half_size_blocks(K, nd, n):
     """Row counts whose tiles need more blocks than run at once at full size:
     they run with half the threads (smooth lengths and a Bluestein one), with the
     rounding of the other forms: 2^-24 for each of at most log2(4 n) additions
-    in each of the (at most three) transforms, in the 2-norm."""
+    in each of the (at most three) transforms, relative to the largest output."""
     import scipy.fft as sf
     x = np.random.default_rng(n).standard_normal((nd, n)).astype(np.float32)
     want = sf.dct(x.astype(np.float64), type=1, axis=-1)
