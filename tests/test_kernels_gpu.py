@@ -552,7 +552,7 @@ def test_f64_rotation(K, nd, n):
     assert (np.abs(got - Al @ Xl) <= nd * 2.0 ** -53 * (np.abs(A) @ np.abs(X))).all()
 
 
-@pytest.mark.parametrize("nd,n", [(52, 65341), (64, 65341), (96, 65341), (48, 130978), (33, 72140)])
+@pytest.mark.parametrize("nd,n", [(52, 65341), (64, 65341), (96, 65341), (48, 130978), (33, 72140), (62, 28162)])
 def test_dct1_f32_one_wave_of_half_size_blocks(K, nd, n):
     """Row counts whose tiles need more blocks than run at once at full size:
     they run with half the threads (smooth lengths and a Bluestein one), with the
