@@ -404,7 +404,7 @@ __device__ __forceinline__ void store_stats(int2 *dst, int mx, float sum, int2 *
   if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = make_int2(mx, __float_as_int(sum));
   __syncthreads();
   if (threadIdx.x == 0) {
-    for (int w = 1; w < NT / 32; w++) {
+    for (int w = 1; w < (int)blockDim.x / 32; w++) {
       mx = max(mx, sh[w].x);
       sum += __int_as_float(sh[w].y);
     }
@@ -439,7 +439,7 @@ template <int R, int FB>
 __device__ __forceinline__ int stage_dit(Z *slot, int Ls, int Ns, float invNs, const W *stw, Shift sh) {
   const int nq = Ls / R;
   int o = 0;
-  for (int q = threadIdx.x / FB; q < nq; q += NT / FB) {
+  for (int q = threadIdx.x / FB; q < nq; q += (int)blockDim.x / FB) {
     const int g = __float2int_rz(((float)q + 0.5f) * invNs);
     const int k = q - g * Ns;
     Z *a = slot + g * Ns * R + k;
@@ -470,7 +470,7 @@ __device__ __forceinline__ int astage_first(Z *sbuf, int pitch, const double *x1
   int o = 0;
   if (b >= nb) return o;
   const int step = p.L1 * nq;
-  for (int q = threadIdx.x / FB; q < nq; q += NT / FB) {
+  for (int q = threadIdx.x / FB; q < nq; q += (int)blockDim.x / FB) {
     const int j = j1_0 + b + p.L1 * __ldg(p.iperm2 + q * R);
     double u[R], w[R];
 #pragma unroll
@@ -505,7 +505,7 @@ __device__ __forceinline__ int astage_last(const Z *sbuf, int pitch, int Ns, con
                                            const Fft4Dev &p, Z *Tp) {
   const int h2 = p.L2 / 2;
   int o = 0;
-  for (int bf = threadIdx.x; bf < FB * Ns; bf += NT) {
+  for (int bf = threadIdx.x; bf < FB * Ns; bf += (int)blockDim.x) {
     const int b = bf / Ns, q = bf - b * Ns;
     if (b >= nb) break;  // b grows with bf
     const Z *a = sbuf + b * pitch + q;
@@ -603,7 +603,7 @@ __global__ void __launch_bounds__(NT, 2) k_i64_a(const double *__restrict__ x, i
     __syncthreads();
     const int k2 = tid & 31, h2 = L2 / 2;
     o = 0;
-    for (int b = tid >> 5; b < nb; b += NT / 32) {
+    for (int b = tid >> 5; b < nb; b += (int)blockDim.x / 32) {
       const int j1 = j1_0 + b;
       if (k2 < L2) {
         const Z v = sbuf[b * pitch + k2];
@@ -685,7 +685,7 @@ __device__ __forceinline__ int bstage_first(Z *slot, int Ls, const TCol &col, co
                                             const PassB &pb, Stats &st) {
   const int nq = Ls / R;
   int o = 0;
-  for (int q = threadIdx.x / FB; q < nq; q += NT / FB) {
+  for (int q = threadIdx.x / FB; q < nq; q += (int)blockDim.x / FB) {
     const int j = __ldg(iperm + q * R);
     Z v[R];
 #pragma unroll
@@ -708,7 +708,7 @@ __device__ __forceinline__ int bstage_first(Z *slot, int Ls, const TCol &col, co
 template <int R, int FB>
 __device__ __forceinline__ void bstage_last(const Z *slot, int Ns, const W *stw, Shift sh, int ex, int epi,
                                             const PassB &pb, Stats &st) {
-  for (int q = threadIdx.x / FB; q < Ns; q += NT / FB) {
+  for (int q = threadIdx.x / FB; q < Ns; q += (int)blockDim.x / FB) {
     const Z *a = slot + q;
     Z v[R];
 #pragma unroll
@@ -766,7 +766,7 @@ __global__ void __launch_bounds__(NT, 2) k_i64_b(const Z *__restrict__ T, int64_
   }
   if (s_ec == NAN_TILE) {
     const double nan = __longlong_as_double(0x7FF8000000000000ll);
-    for (int k1 = tid / FB; on && k1 < L1; k1 += NT / FB) {
+    for (int k1 = tid / FB; on && k1 < L1; k1 += (int)blockDim.x / FB) {
       int kk = pb.k2 + L2 * k1;
       if (pb.self && kk > pb.m) continue;
       kk = min(kk, pb.L - kk);
@@ -777,7 +777,7 @@ __global__ void __launch_bounds__(NT, 2) k_i64_b(const Z *__restrict__ T, int64_
     return;
   }
   const int bsum = texp[pair * MAXT].z, sh0 = stage_shift(s_bits, p.r1[0], bsum, s_ec);
-  for (int i = tid; i < ntile; i += NT) s_shift[i] = min(62, s_ec - texp[pair * MAXT + i].x + sh0);
+  for (int i = tid; i < ntile; i += (int)blockDim.x) s_shift[i] = min(62, s_ec - texp[pair * MAXT + i].x + sh0);
   __syncthreads();
   int ex = s_ec + sh0, o = 0;
   Z *const slot = sbuf + b * pitch_odd(L1);
@@ -869,6 +869,17 @@ int fft4_i64_tfull(const Fft4Dev &d, void *out) {
   return MK_OK;
 }
 
+// threads of a pass of ntile CTAs with smem bytes each: NT, or half of it where
+// CTAs of NT threads (two per SM) would need a second, mostly empty wave and
+// half-size ones (four per SM: the registers are those of 2 NT threads) all run
+// at once.  Larger TODs keep NT (256 x 130,978: 0.97 ms for 1.15).  DCT with NT and
+// with half: 53 x 20,001 (351 tiles a pass) 55.6 and 43.1 us, 64 x 26,245 63.0 and
+// 50.7 us.
+static int threads_for(int64_t ntile, size_t smem) {
+  const int64_t sms = sm_count(), fit = 227 * 1024 / (int64_t)(smem + 2048);
+  return ntile > std::min<int64_t>(2, fit) * sms && ntile <= std::min<int64_t>(4, fit) * sms ? NT / 2 : NT;
+}
+
 int fft4_dct_i64(const Fft4Plan &p, const double *x, int64_t ldx, int64_t nrow, void *scratch, double *out, int64_t ldo,
                  int epi, const double *w, int64_t ldw, bool chained, cudaStream_t st) {
   const Fft4Dev &d = p.d;
@@ -901,14 +912,14 @@ int fft4_dct_i64(const Fft4Plan &p, const double *x, int64_t ldx, int64_t nrow, 
   const int nstat = chained ? tb : PRE;
   const size_t sa = (size_t)d.fba * pitch_odd(d.L2) * sizeof(Z), sb = (size_t)d.fbb * pitch_odd(d.L1) * sizeof(Z);
   if (d.fba == FBH)
-    k_i64_a<FBH><<<dim3(ta, np), NT, sa, st>>>(x, ldx, nrow, T, stat, nstat, texp, d);
+    k_i64_a<FBH><<<dim3(ta, np), threads_for((int64_t)ta * np, sa), sa, st>>>(x, ldx, nrow, T, stat, nstat, texp, d);
   else
-    k_i64_a<FBL><<<dim3(ta, np), NT, sa, st>>>(x, ldx, nrow, T, stat, nstat, texp, d);
+    k_i64_a<FBL><<<dim3(ta, np), threads_for((int64_t)ta * np, sa), sa, st>>>(x, ldx, nrow, T, stat, nstat, texp, d);
   if ((rc = launch_status("fft4 pass A"))) return rc;
   if (d.fbb == FBH)
-    k_i64_b<FBH><<<dim3(tb, np), NT, sb, st>>>(T, nrow, out, ldo, w, ldw, epi, texp, ta, stat, d);
+    k_i64_b<FBH><<<dim3(tb, np), threads_for((int64_t)tb * np, sb), sb, st>>>(T, nrow, out, ldo, w, ldw, epi, texp, ta, stat, d);
   else
-    k_i64_b<FBL><<<dim3(tb, np), NT, sb, st>>>(T, nrow, out, ldo, w, ldw, epi, texp, ta, stat, d);
+    k_i64_b<FBL><<<dim3(tb, np), threads_for((int64_t)tb * np, sb), sb, st>>>(T, nrow, out, ldo, w, ldw, epi, texp, ta, stat, d);
   return launch_status("fft4 pass B");
 }
 

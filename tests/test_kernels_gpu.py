@@ -565,6 +565,19 @@ def test_dct1_f32_one_wave_of_half_size_blocks(K, nd, n):
     assert rel(got, want) < 3 * np.log2(4 * n) * 2.0 ** -24
 
 
+@pytest.mark.parametrize("nd,n", [(47, 20001), (53, 20001), (64, 26245), (92, 20001), (8, 65341)])
+def test_dct1_f64_half_size_blocks_give_the_same_bits(K, nd, n):
+    """FP64 rows whose tiles run in one wave of half-size blocks: the block
+    size changes no value, so every row equals the same row in a call of few
+    rows (full-size blocks), a non-finite row included."""
+    x = dev(np.random.default_rng(n).standard_normal((nd, n)))
+    x[3, 100] = float("inf")
+    whole = K.DCT1(nd, n, torch.float64)(x)
+    few = K.DCT1(4, n, torch.float64)
+    for r in range(0, nd - 3, 4):
+        assert torch.equal(whole[r : r + 4].nan_to_num(7.0), few(x[r : r + 4].contiguous()).nan_to_num(7.0))
+
+
 def test_apply_noise_golden_f64_sliced_rotation(K, gold):
     """The reference's apply_noise (noise.npz) with the sliced FP64 rotation."""
     g = gold("noise.npz")
