@@ -406,8 +406,8 @@ int fft4_init(Fft4Plan *p, int64_t n, void *dev_tables, bool bluestein, bool f64
   for (int64_t j1 = 0; j1 < d.H1 && !d.i64(); j1++) {
     for (int l = 0; l < 32; l++) put(h.data(), t.tlane, 32 * j1 + l, unit(j1 * l, d.L), d.f64);
     for (int i = 0; i < d.nb32; i++) {
-      // the signed k of the block's first entry: e, or e - pad - L2 in the upper half
-      const int64_t e = 32 * i, k = e < d.L2 / 2 + d.pad ? e : e - d.pad - d.L2;
+      // the signed k of the block's first entry
+      const int64_t e = 32 * i, k = e < d.up() ? e : e - d.pad - d.L2;
       put(h.data(), t.tblk, j1 * d.nb32 + i, unit(j1 * k, d.L), d.f64);
     }
   }

@@ -79,6 +79,8 @@ struct Fft4Dev {
   int P, PV;         // row pitch of T (L2 + pad) and of V (L1), rounded up to 16
   int64_t tsz, vsz;  // elements of T and of V per row pair
   int nb32;          // blocks of 32 covering a row of T
+  // entry e of a row of T belongs to column e below up() and to e - pad - L2 from there on (a multiple of 32)
+  __host__ __device__ int up() const { return (L2 + 1) / 2 + pad; }
   int fba, fbb;      // transforms per CTA of pass A (length L2) and pass B (length L1): 8 or 16
   int nr1, nr2;
   int r1[FFT4_MAXR], r2[FFT4_MAXR];

@@ -838,10 +838,10 @@ __device__ W unit_w(int64_t t, int64_t L) {
 
 // the four-step twiddles of every entry of T
 __global__ void k_i64_tfull(W *__restrict__ out, const Fft4Dev p) {
-  const int n = p.H1 * p.P, h = p.L2 / 2;
+  const int n = p.H1 * p.P;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const int j1 = i / p.P, e = i - j1 * p.P;
-    const int k = e < h + p.pad ? e : e - p.pad - p.L2;  // the entry's signed column
+    const int k = e < p.up() ? e : e - p.pad - p.L2;  // the entry's signed column
     out[i] = unit_w((int64_t)j1 * k, p.L);
   }
 }

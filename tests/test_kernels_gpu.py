@@ -357,6 +357,33 @@ def test_dct1_every_short_length(K, dtype, tol, split):
         assert rel(d(dev(x, dtype)).cpu().numpy(), oracle.dct1(x)) < tol, n
 
 
+# n, L2 of its default split: odd L2 with L2 / 2 + 1 a multiple of 32 (the upper entries of a row between the
+# passes follow the lower ones without a gap), one past it (a gap of one), and the even neighbour
+ROW_LAYOUTS = [(1387, 63), (1576, 63), (1702, 63), (1765, 63), (1891, 63), (492076, 1215), (729001, 1215),
+               (7001, 125), (2017, 64)]
+
+
+@pytest.mark.parametrize("dtype,tol", [(torch.float64, 1e-12), (torch.float32, 3e-6)])
+@pytest.mark.parametrize("n,L2", ROW_LAYOUTS)
+def test_dct1_row_layouts(K, dtype, tol, n, L2):
+    """Every layout of a row's lower and upper entries between the passes,
+    against the FP64 oracle at the tolerances of the other smooth lengths."""
+    assert K.dct_describe(n)["L2"] == L2 and K.dct_describe(n)["engine"] == 0
+    x = np.random.default_rng(n).standard_normal((3, n))
+    assert rel(K.DCT1(3, n, dtype)(dev(x, dtype)).cpu().numpy(), oracle.dct1(x)) < tol
+
+
+def test_apply_noise_f64_row_without_gap(K):
+    """The filter's chained transforms at one of those lengths (1891 = 60 x 63 / 2 + 1)."""
+    rng = np.random.default_rng(1891)
+    v = np.linalg.qr(rng.standard_normal((5, 5)))[0]
+    x, w = rng.standard_normal((5, 1891)), rng.random((5, 1891))
+    plan = K.NoisePlan(5, 1891, torch.float64)
+    assert plan.split == (60, 63)
+    got = plan.apply(dev(v), dev(v.T), dev(w), dev(x)).cpu().numpy()
+    assert rel(got, oracle.apply_noise(v, v.T, w, x)) < 1e-12
+
+
 @pytest.mark.parametrize("n", [2, 9, 5001, 65341])
 def test_dct1_f64_ranges_of_values(K, n):
     """The block fixed point of the FP64 DCT-I: rows from 1e-300 to 1e290, an
