@@ -449,6 +449,7 @@ def run_ours(args):
     parallel.barrier()
     with ClockSampler(local) as clk:
         total_ms, per, wall = time_steps(step, args.steps, args.warmup, stream, clk)
+    op.check()
     parallel.barrier()
     rank_ms_step = total_ms / args.steps
     ms_step = max_over_ranks(total_ms) / args.steps
@@ -612,6 +613,7 @@ def pcg_extras(tv, m, dev):
             st.step()
         e1.record()
         torch.cuda.synchronize()
+        op.check()
         ms = e0.elapsed_time(e1) / n
         res[name] = {"ms": ms, "Msamp_per_s": S / (ms * 1e-3) / 1e6, "tod2map_kernel": op.method,
                      "rot_mode": op.rot_mode}
@@ -776,6 +778,7 @@ def solve_c4(dev, tol=1e-6, wall_limit_s=420.0):
     st.step()
     e1.record()
     e1.synchronize()
+    op64.check()
     ms64 = e0.elapsed_time(e1)
     out["jacobi_f64_iter_ms"] = ms64
     del st

@@ -371,9 +371,10 @@ int mk_rotate(mk_noise_plan *plan, const void *A, const void *X, void *R, int ro
               void *stream);
 
 /* Device status of the plan's tensor-core kernels: *code = 1 if one of
- * their bounded waits timed out since the last call (the kernel then stops,
- * frees its tensor memory and leaves its output incomplete), else 0.  Reads
- * and clears the word; synchronises `stream`. */
+ * their bounded waits timed out since the last call, else 0.  The kernel
+ * then stops, frees its tensor memory and fills what it had to write with
+ * NaN, and so does every later tensor-core rotation of the plan until this
+ * call has reported it.  Reads and clears the word; synchronises `stream`. */
 int mk_noise_status(mk_noise_plan *plan, int *code, void *stream);
 
 /* NoiseSmoothedSVD.apply_noise of many TODs in one call, in place on each
@@ -387,7 +388,8 @@ int mk_noise_status(mk_noise_plan *plan, int *code, void *stream);
  * the device job tables; the data pointers, v, vT and mywt must stay valid
  * and unchanged while it is used.  Plans that share a workspace must have
  * their calls ordered on one stream.  mk_noise_group_status reports (and
- * clears) a timed-out wait inside the rotation kernel.  Replaces the
+ * clears) a timed-out wait inside the rotation kernel, whose outputs are NaN
+ * as after mk_noise_status's.  Replaces the
  * per-TOD loop of minkasi/tods/core.py:517-580 (Tod.apply_noise) inside
  * TodVec.dot (core.py:967-1026). */
 typedef struct mk_noise_group mk_noise_group;

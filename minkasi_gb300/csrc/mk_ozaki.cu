@@ -422,6 +422,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
   asm volatile("tcgen05.fence::after_thread_sync;");
   const uint32_t tmem = tmem_base_sh;
   const int ndrain = (nkc + OZ_DRAIN - 1) / OZ_DRAIN;
+  const int prior = tid == 0 ? *(volatile const int *)err : 0;  // an earlier timeout, not yet reported
   uint32_t issued = 0, g_mma = 0;  // chunks whose copies were issued / whose MMAs were committed
 
   if (warp == EPI_WARPS) {
@@ -534,7 +535,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
       }
     }
   }
-  __syncthreads();
+  const bool failed = __syncthreads_or(prior | *abort_flag);
   if (*abort_flag) {
     // after a timeout: bounded waits for the copies and MMAs still in flight
     if (tid == EPI_WARPS * 32)
@@ -547,6 +548,13 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
         (void)mbar_wait(&done[g % XSTG], (g / XSTG) & 1);
     }
   }
+  if (failed)  // no caller takes this CTA's part for a result
+    for (int i = blockIdx.x; i < nitem; i += gridDim.x)
+      for (int e = tid; e < OZ_M * OZ_ND; e += OZ_THREADS) {
+        const int64_t j = j0 + (int64_t)(i / ndb) * OZ_M + e % OZ_M;
+        const int d = (i % ndb) * OZ_ND + e / OZ_M;
+        if (j < ncol && d < nrow) R[(int64_t)d * ldr + j] = __longlong_as_double(0x7FF8000000000000ll);
+      }
   asm volatile("tcgen05.fence::before_thread_sync;");
   __syncthreads();
   if (warp == 0)

@@ -221,6 +221,7 @@ __global__ void __launch_bounds__((8 * MT + 1) * 32, 3 - MT)
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;");
   const uint32_t tmem = tmem_base_sh;
+  const int prior = tid == 0 ? *(volatile const int *)err : 0;  // an earlier timeout, not yet reported
   uint32_t g_copied = 0, g_issued = 0;  // MMA thread: chunks whose image copy / MMAs were issued
 
   if (warp < NSPLIT) {
@@ -362,7 +363,7 @@ __global__ void __launch_bounds__((8 * MT + 1) * 32, 3 - MT)
       mk::mbar_arrive(&acc_empty[ab]);
     }
   }
-  __syncthreads();
+  const bool failed = __syncthreads_or(prior | *abort_flag);
   if (*abort_flag && tid == (NSPLIT + NEPI) * 32) {
     atomicExch(err, 1);
     // bounded waits for the copies and MMAs this thread issued
@@ -370,6 +371,21 @@ __global__ void __launch_bounds__((8 * MT + 1) * 32, 3 - MT)
       (void)mbar_wait(&full_b[g % NSTAGE], (g / NSTAGE) & 1);
     for (uint32_t g = (g_issued > NSTAGE ? g_issued - NSTAGE : 0); g < g_issued; g++)
       (void)mbar_wait(&mma_done[g % NSTAGE], (g / NSTAGE) & 1);
+  }
+  if (failed) {  // no caller takes this CTA's part for a result
+    int cur = 0;
+    for (int64_t item = blockIdx.x; item < nitem; item += gridDim.x) {
+      cur = job_at(jobs, njobs, item, cur);
+      const mk::RotJob &J = jobs[cur];
+      for (int e = tid; e < MT * TILE_M * ndet; e += (int)blockDim.x) {
+        const int64_t my = (item - J.tile0) * MT * TILE_M + e % (MT * TILE_M);
+        float *row = J.R + (int64_t)(e / (MT * TILE_M)) * J.ldr;
+        if (my < J.ncol) {
+          row[my] = __int_as_float(0x7FC00000);
+          if (mirror_n > 0 && my >= 1 && my <= J.ncol - 2) row[mirror_n - my] = __int_as_float(0x7FC00000);
+        }
+      }
+    }
   }
   asm volatile("tcgen05.fence::before_thread_sync;");
   __syncthreads();

@@ -183,6 +183,22 @@ class MapmakingOperator:
         self.project_out(of)
         return out
 
+    def timed_out(self) -> bool:
+        """True if a kernel of this operator stopped on a timed-out wait since
+        the last call: a rotation (its outputs are NaN) or the staged tod2map
+        (its update of the map is incomplete).  Synchronises."""
+        if self._group:
+            bad = self._group.status() != 0
+        else:
+            bad = any([p.status() for p in self.plans.values()]) if self.rot_mode in (2, 4) else False
+        return (self.method == "staged" and K.tod2map_status() != 0) or bad
+
+    def check(self) -> None:
+        """Raises RuntimeError if ``timed_out()``.  The solvers call it before
+        they return or use an FP64 residual."""
+        if self.timed_out():
+            raise RuntimeError("a GPU kernel of the mapmaking operator stopped on a timed-out wait; its results are invalid")
+
     def rhs(self, out: torch.Tensor) -> torch.Tensor:
         """out += sum_tod P^T N d with d = tod.info['dat_calib']."""
         for t, view in zip(self.tods, self.views(self.tmp)):

@@ -507,7 +507,8 @@ class NoisePlan:
         return out
 
     def status(self) -> int:
-        """1 if a tensor-core kernel of this plan timed out since the last call."""
+        """1 if a tensor-core kernel of this plan timed out since the last call
+        (what it and the plan's later ones had to write is NaN then)."""
         code = ctypes.c_int(0)
         check(lib().mk_noise_status(self._h, ctypes.byref(code), _stream()), "noise_status")
         return int(code.value)
@@ -572,7 +573,8 @@ class NoiseGroup:
         check(lib().mk_noise_group_exec(self._h, _stream()), "noise group exec")
 
     def status(self) -> int:
-        """1 if a tensor-core wait of the group timed out since the last call."""
+        """1 if a tensor-core wait of the group timed out since the last call
+        (what it and the group's later ones had to write is NaN then)."""
         code = ctypes.c_int(0)
         check(lib().mk_noise_group_status(self._h, ctypes.byref(code), _stream()), "noise group status")
         return int(code.value)

@@ -79,6 +79,12 @@ class RankSumOp:
         out.add_(part)
         return out
 
+    def check(self) -> None:
+        """The operator's check on every rank: all raise if one has to."""
+        if parallel.allreduce_scalar(float(self.op.timed_out()), "max"):
+            raise RuntimeError("a GPU kernel of the mapmaking operator stopped on a timed-out wait on some rank; "
+                               "the summed results are invalid")
+
 
 def global_op(op):
     """The operator summed over ranks; the local operator itself on one rank."""
@@ -198,6 +204,7 @@ def run_pcg_wprior(b: Mapset, x0: Mapset, tods: TodVec, prior=None, precon=None,
         if need_check or history is not None:
             s = st.scalars()
             if s[MK_S_FLAG]:
+                op.check()
                 raise FloatingPointError(f"PCG breakdown at iteration {i} (p.Ap <= 0 or non-finite)")
             rec = math.sqrt(max(s[MK_S_RR], 0.0)) / bnorm if bnorm else float("nan")
             if history is not None:
@@ -209,6 +216,7 @@ def run_pcg_wprior(b: Mapset, x0: Mapset, tods: TodVec, prior=None, precon=None,
                 if tr <= tol:
                     break
     torch.cuda.synchronize()
+    op.check()
     niter = i + 1
     tave = (time.time() - tloop) / max(niter, 1)
     if verbose:
@@ -260,6 +268,8 @@ def _run_pcg_generic(b, x0, tods, prior, precon, mask, maxiter, outroot, save_it
             history.append({"iter": i, "zr": zr, "alpha": alpha, "beta": beta})
         if i in save_iters:
             x.maps[save_ind].write(outroot + "_" + str(i) + save_tail)
+    if isinstance(tods, TodVec) and tods._fast(b):
+        global_op(tods.engine(b.maps[0])).check()
     x.niter = maxiter
     return x
 
@@ -333,6 +343,8 @@ def run_pcg_mixed(b: Mapset, x0: Mapset, tods: TodVec, precon=None, tol: float =
         # r = b - A64 x; z = M r; zr = r.z  (p kept; the caller restarts it
         # when the recursive residual had drifted)
         op64.apply(xf, ax)
+        op64.check()
+        op32.check()
         K.pcg_init(st.r, st.z, ptmp, bf, ax, st.M, st.s, st.red)
         if st.Mop is not None:
             st.Mop.apply(st.r, st.z)
@@ -354,6 +366,7 @@ def run_pcg_mixed(b: Mapset, x0: Mapset, tods: TodVec, precon=None, tol: float =
             continue
         s = st.scalars()
         if s[MK_S_FLAG]:
+            op32.check()
             raise FloatingPointError(f"mixed PCG breakdown at iteration {k}")
         rec = math.sqrt(max(s[MK_S_RR], 0.0)) / bnorm
         if since >= replace_every or rec <= tol:
@@ -376,6 +389,7 @@ def run_pcg_mixed(b: Mapset, x0: Mapset, tods: TodVec, precon=None, tol: float =
                 on_outer(outer, xf, rel)
             if rel <= tol:
                 break
+    op32.check()
     x.niter = k
     x.outer = outer
     x.restarts = restarts
@@ -409,6 +423,8 @@ def _run_refine(b, x0, tods, precon, tol, inner_iters, max_outer, graph, verbose
     rel = float("inf")
     for outer in range(max_outer):
         op64.apply(xf, ax)
+        op64.check()
+        op32.check()
         r64 = bf - ax
         rel = math.sqrt(red.dot(r64, r64).item()) / bnorm
         if history is not None:

@@ -183,3 +183,27 @@ def test_learned_weight_files_single_and_multilevel(tmp_path):
     assert all(torch.equal(x, y) for a, b in zip(two, b2) for x, y in zip(a.weights, b.weights))
     # the committed weights load
     assert isinstance(L.load(L.weights_path("c1"), "cpu"), L.ConvNet)
+
+
+@pytest.mark.parametrize("plan,group,staged,rot_mode,bad", [
+    (0, None, 0, 4, False), (1, None, 0, 4, True), (1, None, 0, 2, True), (1, None, 0, 1, False),
+    (0, 0, 0, 2, False), (0, 1, 0, 2, True), (0, None, 1, 1, True)])
+def test_operator_reports_timed_out_kernels(monkeypatch, plan, group, staged, rot_mode, bad):
+    """MapmakingOperator.check and RankSumOp.check, host logic: the status of
+    the plans (rotations on the tensor cores), of the group where there is
+    one, and of the staged tod2map."""
+    from types import SimpleNamespace as NS
+    from minkasi_gb300 import kernels as K
+    from minkasi_gb300.engine import MapmakingOperator
+    from minkasi_gb300.pcg import RankSumOp
+    op = MapmakingOperator.__new__(MapmakingOperator)
+    op.plans = {(4, 9): NS(status=lambda: 0), (4, 17): NS(status=lambda: plan)}
+    op._group = False if group is None else NS(status=lambda: group)
+    op.rot_mode, op.method = rot_mode, "staged" if staged else "atomic"
+    monkeypatch.setattr(K, "tod2map_status", lambda: staged)
+    for o in (op, RankSumOp(op)):
+        if bad:
+            with pytest.raises(RuntimeError, match="timed-out"):
+                o.check()
+        else:
+            o.check()

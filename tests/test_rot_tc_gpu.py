@@ -110,3 +110,78 @@ def test_noise_group_equals_per_tod_filter(monkeypatch, dct):
     for (v, vT, w), view, dims in zip(op.ops, op.views(op.tmp), op.dims):
         op.plans[dims].apply(v, vT, w, view, out=view, rot_mode=2)
     assert torch.equal(grouped, op.tmp)
+
+
+@pytest.mark.parametrize("set_word", [0, 1])
+def test_rotations_are_nan_after_an_unreported_timeout(K, set_word):
+    """The kernels' error word, as a timed-out wait leaves it: while it is set
+    every rotation is NaN throughout (FP64 in slices, FP32 with the mirrored
+    extension), and the word stays for the status call; unset, the results
+    are the plan's own bit for bit."""
+    import ctypes
+    h = K.lib()
+    g = torch.Generator(device="cuda").manual_seed(1)
+    vp, i64 = ctypes.c_void_p, ctypes.c_int64
+    err = torch.tensor([set_word], dtype=torch.int32, device=cuda)
+
+    nd, n = 40, 3001  # two detector blocks, a ragged last tile
+    A = torch.randn((nd, nd), generator=g, dtype=torch.float64, device=cuda)
+    X = torch.randn((nd, n), generator=g, dtype=torch.float64, device=cuda)
+    R = torch.zeros((nd, n), dtype=torch.float64, device=cuda)
+    plan = K.NoisePlan(nd, n, torch.float64)
+    want = plan.rotate(A, X, rot_mode=4)
+    rot64 = h._ZN2mk16ozaki_rotate_f64EPKdS1_lPdlllPvmPiP11CUstream_st
+    rot64.argtypes = [vp, vp, i64, vp, i64, i64, i64, vp, ctypes.c_size_t, vp, vp]
+    ws = torch.empty(128 << 20, dtype=torch.uint8, device=cuda)
+    assert rot64(A.data_ptr(), X.data_ptr(), n, R.data_ptr(), n, nd, n, ws.data_ptr(), ws.numel(), err.data_ptr(),
+                 K._stream()) == 0
+    assert R.isnan().all() if set_word else torch.equal(R, want)
+
+    nd = 256
+    A, X = (torch.randn(s, generator=g, device=cuda) for s in ((nd, nd), (nd, n)))
+    plan = K.NoisePlan(nd, n, torch.float32)
+    want = plan.rotate(A, X, rot_mode=2)
+    want = torch.cat([want, want[:, 1:-1].flip(1)], dim=1)
+    R = torch.zeros((nd, 2 * (n - 1)), device=cuda)
+    rot32 = h._ZN2mk10rot_tc_f32EPKfS1_lPflllPvPiP11CUstream_stlli
+    rot32.argtypes = [vp, vp, i64, vp, i64, i64, i64, vp, vp, vp, i64, i64, ctypes.c_int]
+    assert rot32(A.data_ptr(), X.data_ptr(), n, R.data_ptr(), 2 * (n - 1), nd, n, ws.data_ptr(), err.data_ptr(),
+                 K._stream(), 2 * (n - 1), 1, 0) == 0
+    assert R.isnan().all() if set_word else torch.equal(R, want)
+    assert err.item() == set_word
+
+
+def test_solvers_raise_on_a_reported_timeout(K, monkeypatch):
+    """run_pcg, run_pcg_mixed (both modes) and the generic solver end with an
+    error where a plan's or the group's status word says that a wait timed out."""
+    import minkasi_gb300 as mk
+    from minkasi_gb300 import synth
+    monkeypatch.setenv("MINKASI_GB300_TOD2MAP", "atomic")
+    tv, m = synth.make_todvec(synth.CONFIGS["tiny"])
+    tv.rot_mode = 4
+    b = mk.Mapset()
+    b.add_map(m)
+    tv.make_rhs(b, do_clear=True)
+    x0 = b.copy()
+    x0.clear()
+    solve = [lambda: mk.run_pcg(b, x0, tv, maxiter=2, verbose=False),
+             lambda: mk.run_pcg_mixed(b, x0, tv, max_iter=2, replace_every=2),
+             lambda: mk.run_pcg_mixed(b, x0, tv, max_iter=2, mode="refine", max_outer=1),
+             lambda: mk.run_pcg(b, x0, tv, mask=None, maxiter=1, verbose=False, precon=mk.null_precon())]
+    tv.engine(m, torch.float32).rot_mode = 2  # (where the group or the plans would report)
+    tv.engine(m, torch.float32)._group = False
+    monkeypatch.setattr(K.NoisePlan, "apply", _cublas_apply(K))
+    for f in solve[:3]:
+        f()
+    monkeypatch.setattr(K.NoisePlan, "status", lambda self: 1)
+    for f in solve:
+        with pytest.raises(RuntimeError, match="timed-out"):
+            f()
+
+
+def _cublas_apply(K):
+    apply = K.NoisePlan.apply
+
+    def run(self, *a, rot_mode=0, **k):
+        return apply(self, *a, rot_mode=1, **k)
+    return run
