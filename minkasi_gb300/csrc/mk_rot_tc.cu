@@ -398,13 +398,17 @@ int tiles_per_item(int64_t nrow) { return nrow == 256 ? 2 : 1; }
 template <int MT>
 int launch(const mk::RotJob *jobs, int njobs, const mk::RotJob &j0, int64_t nitem, int nd, int *err, cudaStream_t st,
            int64_t mirror_n, int64_t xs, int halve_ends) {
-  const size_t smem = NSTAGE * ((size_t)MT * A_TILE + 3 * (size_t)nd * 64) + 1024;
-  static int attr[64] = {0};
+  const auto bytes = [](int ndet) { return NSTAGE * ((size_t)MT * A_TILE + 3 * (size_t)ndet * 64) + 1024; };
+  const size_t smem = bytes(nd);
+  // the limit of the largest detector count of the instantiation, whatever this
+  // call's: threads that set it at the same time set the same value
+  static bool attr[64] = {false};
   int dev = 0;
   MK_CUDA(cudaGetDevice(&dev));
-  if (dev >= 0 && dev < 64 && attr[dev] < (int)smem) {
-    MK_CUDA(cudaFuncSetAttribute(k_rot_tc<MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    attr[dev] = (int)smem;
+  if (dev >= 0 && dev < 64 && !attr[dev]) {
+    MK_CUDA(cudaFuncSetAttribute(k_rot_tc<MT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)bytes(MT == 1 ? 128 : 256)));
+    attr[dev] = true;
   }
   const int nbuf = MT * nd * 2 <= 512 / (MT == 1 ? 2 : 1) ? 2 : 1;  // accumulators; MT = 1: two CTAs per SM
   const uint32_t tcols = (uint32_t)(MT * nd * nbuf);

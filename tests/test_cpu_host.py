@@ -207,3 +207,86 @@ def test_operator_reports_timed_out_kernels(monkeypatch, plan, group, staged, ro
                 o.check()
         else:
             o.check()
+
+
+FAKE_CUDART = r"""
+#include <stddef.h>
+typedef struct { unsigned x, y, z; } dim3_;
+static struct { const void *f; long limit; } attr[64];
+static int nattr, calls;
+volatile int held, release;
+static __thread size_t pushed;
+/* the first caller stays here, its limit set, until `release` (10 s at most) */
+int cudaFuncSetAttribute(const void *f, int what, int value) {
+  const int first = __atomic_fetch_add(&calls, 1, __ATOMIC_SEQ_CST) == 0;
+  int i = 0;
+  while (i < nattr && attr[i].f != f) i++;
+  attr[i].f = f;
+  attr[i].limit = value;
+  if (i == nattr) nattr++;
+  if (first) {
+    struct timespec { long s, ns; } t = {0, 1000000};
+    int nanosleep(const struct timespec *, struct timespec *);
+    held = 1;
+    for (int k = 0; k < 10000 && !release; k++) nanosleep(&t, 0);
+  }
+  return 0;
+}
+unsigned __cudaPushCallConfiguration(dim3_ g, dim3_ b, size_t smem, void *st) { pushed = smem; return 0; }
+int __cudaPopCallConfiguration(dim3_ *g, dim3_ *b, size_t *smem, void **st) { *smem = pushed; *st = 0; return 0; }
+int __cudaGetKernel(void **k, const void *f) { *k = (void *)f; return 0; }
+static int launch(const void *f, size_t smem) {
+  for (int i = 0; i < nattr; i++)
+    if (attr[i].f == f) return smem <= (size_t)attr[i].limit ? 0 : 1;
+  return smem <= 48 * 1024 ? 0 : 1;
+}
+static __thread int last;
+int __cudaLaunchKernel(void *f, dim3_ g, dim3_ b, void **a, size_t smem, void *st) { return last = launch(f, smem); }
+int cudaLaunchKernel(void *f, dim3_ g, dim3_ b, void **a, size_t smem, void *st) { return last = launch(f, smem); }
+int cudaGetLastError(void) { const int e = last; last = 0; return e; }
+int cudaGetDevice(int *d) { *d = 0; return 0; }
+int cudaDeviceGetAttribute(int *v, int a, int d) { *v = 152; return 0; }
+const char *cudaGetErrorString(int e) { return "fake error"; }
+int cudaOccupancyMaxActiveBlocksPerMultiprocessor(int *n, const void *f, int b, size_t s) { *n = 1; return 0; }
+void **__cudaRegisterFatBinary(void *p) { static void *h; return &h; }
+void __cudaRegisterFatBinaryEnd(void **h) {}
+void __cudaUnregisterFatBinary(void **h) {}
+void __cudaRegisterFunction(void **h, const char *f, char *df, const char *n, int l, void *a, void *b, void *c, void *d, int *e) {}
+"""
+
+
+@pytest.mark.parametrize("first,second", [(128, 32), (32, 128)])
+def test_rotation_launch_limits_of_two_threads(tmp_path, first, second):
+    """Two threads launch the FP32 tensor-core rotation for the first time with
+    different detector counts, the first held inside cudaFuncSetAttribute while
+    the second passes it: every later launch finds its shared memory allowed.
+    The host code of the built object on a fake CUDA runtime (no GPU)."""
+    import subprocess
+    import threading
+    import time
+    from minkasi_gb300 import build
+    objs = [os.path.join(build.BUILD, o) for o in ("mk_rot_tc.o", "mk_common.o")]
+    if not all(map(os.path.exists, objs)):
+        pytest.skip("the objects of the build are not here")
+    (tmp_path / "fake.c").write_text(FAKE_CUDART)
+    subprocess.run(["gcc", "-w", "-fPIC", "-c", "fake.c", "-o", "fake.o"], cwd=tmp_path, check=True)
+    subprocess.run(["g++", "-shared", "-o", "rot.so", *objs, "fake.o", "-Wl,-Bsymbolic", "-lpthread"], cwd=tmp_path,
+                   check=True)
+    h = ctypes.CDLL(str(tmp_path / "rot.so"))
+    group = h._ZN2mk12rot_tc_groupEPKNS_6RotJobEillPiP11CUstream_st
+    group.argtypes = [ctypes.c_void_p, ctypes.c_int, ctypes.c_int64, ctypes.c_int64, ctypes.c_void_p, ctypes.c_void_p]
+    run = lambda nd: group(1, 1, 1, nd, 1, None)  # (nothing runs: the pointers are not read)
+    rc = []
+    t = threading.Thread(target=lambda: rc.append(run(first)))
+    t.start()
+    held = ctypes.c_int.in_dll(h, "held")
+    for _ in range(5000):
+        if held.value:
+            break
+        time.sleep(0.001)
+    assert held.value
+    rc.append(run(second))
+    ctypes.c_int.in_dll(h, "release").value = 1
+    t.join()
+    assert rc == [0, 0]
+    assert [run(nd) for nd in (32, 64, 128, 256)] == [0] * 4
