@@ -90,7 +90,7 @@ def choose_tod2map(op, candidates: Optional[Iterable[str]] = None) -> str:
         candidates = ["atomic", "staged", "fixed"]
         if op.S < (1 << 30) and max(op.sizes) < (1 << 31):
             candidates.append("sorted")  # plan memory 4 B/sample
-    key = workload_key(op, "tod2map")
+    key = workload_key(op, "tod2map2")
     hit = _lookup(key)
     if hit in candidates:
         return hit

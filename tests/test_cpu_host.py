@@ -290,3 +290,27 @@ def test_rotation_launch_limits_of_two_threads(tmp_path, first, second):
     t.join()
     assert rc == [0, 0]
     assert [run(nd) for nd in (32, 64, 128, 256)] == [0] * 4
+
+
+def test_tod2map_choices_of_earlier_kernels_are_not_taken(tmp_path, monkeypatch):
+    """A choice stored before the scatter kernels changed (key "tod2map") is
+    timed again and stored under the present key."""
+    import json
+    import torch
+    from types import SimpleNamespace as NS
+    from minkasi_gb300 import autotune as A
+    cache = tmp_path / "autotune.json"
+    cache.write_text(json.dumps({"tod2map|W": "fixed"}))
+    monkeypatch.setenv("MINKASI_GB300_AUTOTUNE", str(cache))
+    monkeypatch.delenv("MINKASI_GB300_TOD2MAP", raising=False)
+    monkeypatch.setattr(A, "_MEM", {})
+    monkeypatch.setattr(A, "workload_key", lambda op, what: f"{what}|W")
+    asked = []
+    ms = {"atomic": 1.0, "staged": 2.0, "fixed": 3.0}
+    monkeypatch.setattr(A, "time_ms", lambda fn: ms[fn()])
+    op = NS(tmp=torch.zeros(4), npix=3, dtype=torch.float64, device="cpu", _pixplans=None,
+            project_out=lambda out, m: asked.append(m) or m)
+    assert A.choose_tod2map(op, list(ms)) == "atomic" and sorted(asked) == sorted(ms)
+    asked.clear()
+    A._MEM.clear()
+    assert A.choose_tod2map(op, list(ms)) == "atomic" and not asked  # from the file
