@@ -44,7 +44,7 @@ void factor(int64_t L, std::vector<int> &f) {
 }
 
 // radices of a transform of length Ls (a product of 2, 3, 5, 7, 11): the
-// fewest stages over the radices 2 .. 16 held in registers (ties broken by
+// fewest stages over the radices 2 .. rmax, 7 and 11 (ties broken by
 // an estimate of the arithmetic), odd ones first (the stride-1 first stage
 // is then free of bank conflicts), each group in decreasing order.
 // MINKASI_GB300_FFT4_RADIX=basic keeps the prime radices with 3 x 3 as 9
@@ -76,7 +76,7 @@ static const RadixPlan &best_plan(const int *e, int rmax, std::vector<RadixPlan>
     best.stages = 0;
   } else {
     for (size_t i = 0; i < sizeof(kRadix) / sizeof(int); i++) {
-      if (kRadix[i] > rmax) continue;
+      if (kRadix[i] > rmax && kRadix[i] != 7 && kRadix[i] != 11) continue;  // (no smaller radix holds these)
       int f[5];
       radix_exps(kRadix[i], f);
       bool fits = true;
@@ -239,6 +239,21 @@ static std::atomic<int> g_split_rank{0};
 void fft4_set_split_rank(int r) { g_split_rank.store(r < 0 ? 0 : r); }
 int fft4_split_rank() { return g_split_rank.load(); }
 
+// largest radix of a pass of length Ls.  A fixed-point butterfly is some
+// 40 R .. 100 R instructions, and a short pass has few of them per SM (all of 3,001
+// samples' second pass: 5 of radix 16 or 20 of radix 4 per transform), which
+// then run one after the other: up to 128 points more and smaller stages are
+// faster at every row count.  DCT-I with radices to 16 and to 6: 2 x 1,025 26.9 and
+// 22.8 us, 16 x 2,049 28.9 and 24.8, 16 x 3,001 37.1 and 25.5, 16 x 5,001 37.1 and
+// 26.8, 256 x 5,001 74.1 and 61.8 (the FP64 passes before the fixed-point ones:
+// 22.8, 24.8, 33.0, 28.9 for the first four).  Longer passes fill their CTA with
+// butterflies of any radix, and fewer stages win: 256 x 262,145 (512 x 1,024)
+// 1317 and 1604 us.
+static int rmax_for(int Ls, bool f64, bool bluestein) {
+  if (!f64) return MK_FFT4_RMAX;
+  return !bluestein && Ls <= 128 ? 6 : MK_FFT4_RMAX64;
+}
+
 // L1 x L2 split of a transform of length L (by g_split_rank among the
 // divisor pairs with both parts <= LMAX and L1 > 1, ordered by closeness to
 // sqrt(L)), radices and stage constants.  Bluestein's last pass runs the
@@ -271,8 +286,9 @@ static bool split_len(int64_t L, Fft4Dev *t, bool bluestein) {
   t->L = L;
   t->L1 = (int)best;
   t->L2 = (int)(L / best);
-  const int rmax = t->f64 ? MK_FFT4_RMAX64 : MK_FFT4_RMAX;
-  if (!radices(t->L1, t->r1, &t->nr1, rmax) || !radices(t->L2, t->r2, &t->nr2, rmax)) return false;
+  if (!radices(t->L1, t->r1, &t->nr1, rmax_for(t->L1, t->f64, bluestein)) ||
+      !radices(t->L2, t->r2, &t->nr2, rmax_for(t->L2, t->f64, bluestein)))
+    return false;
   t->H1 = t->L1 / 2 + 1;
   t->H2 = t->L2 / 2 + 1;
   t->pad = (t->H2 + 31) / 32 * 32 - (t->L2 + 1) / 2;
