@@ -201,12 +201,45 @@ void put(char *base, size_t off, int64_t i, Cd v, bool f64) {
   }
 }
 
-// a fixed-point twiddle: 2^62 (x, y), each as a high and a signed low word
-void put_i64(char *base, size_t off, int64_t i, Cd v) {
+// exp(-2 pi i t / L) for L <= FFT4_LMAX with 62 fraction bits, off by a unit or
+// two: the angle in integers, cosine and sine by their series.  (Rounded to
+// double first, each stage's twiddles would add 2^-54 to the values, as much as
+// the result's own rounding: radices up to 6 instead of 16 took the error of a DCT-I
+// of 2,049 points from 8.1e-17 to 1.0e-16.)
+void unit_q62(int64_t t, int64_t L, int64_t *q) {
+  typedef unsigned __int128 u128;
+  t %= L;
+  if (t < 0) t += L;
+  const bool neg = 2 * t > L;
+  if (neg) t = L - t;
+  const bool half = 4 * t > L;
+  const int64_t u = half ? L - 2 * t : 2 * t;  // angle = pi u / L, u <= L / 2
+  const bool swap = 4 * u > L;
+  // a = pi v / (2 L) <= pi / 4 and its square with 64 fraction bits, from pi 2^112
+  const int64_t v = swap ? L - 2 * u : 2 * u;
+  const u128 pi = (u128)0x3243F6A8885A3ull << 64 | 0x08D313198A2E0370ull;
+  const uint64_t a = (uint64_t)(pi * (u128)v / (u128)(2 * L) >> 48);
+  const auto mul = [](uint64_t x, uint64_t y) { return (uint64_t)((u128)x * y >> 64); };
+  const uint64_t y = mul(a, a);
+  // 1 - cos a = y / 2 (1 - y / 12 (1 - ...)), 1 - sin a / a = y / 6 (1 - y / 20 (1 - ...))
+  uint64_t zc = 0, zs = 0;
+  for (int k = 10; k >= 1; k--) {
+    zc = (y - mul(y, zc)) / (uint64_t)(2 * k * (2 * k - 1));
+    zs = (y - mul(y, zs)) / (uint64_t)(2 * k * (2 * k + 1));
+  }
+  int64_t c = (1ll << 62) - (int64_t)((zc + 2) >> 2), s = (int64_t)((a - mul(a, zs) + 2) >> 2);
+  if (swap) std::swap(c, s);
+  q[0] = half ? -c : c;
+  q[1] = neg ? s : -s;
+}
+
+// a fixed-point twiddle: exp(-2 pi i t / L), each part as a high and a signed low word
+void put_i64(char *base, size_t off, int64_t i, int64_t t, int64_t L) {
   int *w = reinterpret_cast<int *>(base + off) + 4 * i;
-  const double c[2] = {v.x, v.y};
+  int64_t c[2];
+  unit_q62(t, L, c);
   for (int k = 0; k < 2; k++) {
-    const int64_t q = (int64_t)std::llrint(c[k] * 0x1p62);
+    const int64_t q = c[k];
     const int32_t l = (int32_t)(uint32_t)(uint64_t)q;
     w[2 * k] = (int)((q - l) >> 32);
     w[2 * k + 1] = l;
@@ -239,19 +272,20 @@ static std::atomic<int> g_split_rank{0};
 void fft4_set_split_rank(int r) { g_split_rank.store(r < 0 ? 0 : r); }
 int fft4_split_rank() { return g_split_rank.load(); }
 
-// largest radix of a pass of length Ls.  A fixed-point butterfly is some
-// 40 R .. 100 R instructions, and a short pass has few of them per SM (all of 3,001
+// largest radix of a pass of length Ls.  A fixed-point butterfly is some 40 R ..
+// 100 R instructions, and a short pass has few of them per SM (all of 3,001
 // samples' second pass: 5 of radix 16 or 20 of radix 4 per transform), which
-// then run one after the other: up to 128 points more and smaller stages are
-// faster at every row count.  DCT-I with radices to 16 and to 6: 2 x 1,025 26.9 and
-// 22.8 us, 16 x 2,049 28.9 and 24.8, 16 x 3,001 37.1 and 25.5, 16 x 5,001 37.1 and
-// 26.8, 256 x 5,001 74.1 and 61.8 (the FP64 passes before the fixed-point ones:
-// 22.8, 24.8, 33.0, 28.9 for the first four).  Longer passes fill their CTA with
-// butterflies of any radix, and fewer stages win: 256 x 262,145 (512 x 1,024)
-// 1317 and 1604 us.
+// then run one after the other: up to 176 points more and smaller stages are
+// faster.  Longer passes fill their CTA with butterflies of any radix, and fewer
+// stages win.  DCT-I with radices to 16 and to 6, us: 2 x 1,025 26.9 and 20.8, 16 x
+// 3,001 37.1 and 25.5, 16 x 5,001 37.1 and 26.8 (the FP64 passes before the
+// fixed point: 22.8, 33.0, 28.9), 256 x 9,073 (126 x 144) 120 and 92, 128 x 10,001
+// (125 x 160) 53.6 and 55.7, 96 x 20,001 (200 x 200) 78 and 84, 256 x 262,145 (512 x
+// 1,024) 1317 and 1604.  Bluestein's FP64 passes gain too (16 x 3,000 61 and 47), but
+// each stage's twiddles add to their error (6.00e-16 and 6.10e-16): they keep 16.
 static int rmax_for(int Ls, bool f64, bool bluestein) {
   if (!f64) return MK_FFT4_RMAX;
-  return !bluestein && Ls <= 128 ? 6 : MK_FFT4_RMAX64;
+  return !bluestein && Ls <= 176 ? 6 : MK_FFT4_RMAX64;
 }
 
 // L1 x L2 split of a transform of length L (by g_split_rank among the
@@ -405,9 +439,9 @@ int fft4_init(Fft4Plan *p, int64_t n, void *dev_tables, bool bluestein, bool f64
       for (int rr = 1; rr < r[s]; rr++)
         for (int k = 0; k < ns[s]; k++) {
           const int64_t i = to[s] + (rr - 1) * ns[s] + k;
-          const Cd v = unit((int64_t)rr * k, (int64_t)ns[s] * r[s]);
-          if (d.i64()) put_i64(h.data(), so, i, v);
-          else put(h.data(), so, i, v, d.f64);
+          const int64_t num = (int64_t)rr * k, den = (int64_t)ns[s] * r[s];
+          if (d.i64()) put_i64(h.data(), so, i, num, den);
+          else put(h.data(), so, i, unit(num, den), d.f64);
         }
   }
   {

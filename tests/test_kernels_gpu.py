@@ -373,6 +373,20 @@ def test_dct1_row_layouts(K, dtype, tol, n, L2):
     assert rel(K.DCT1(3, n, dtype)(dev(x, dtype)).cpu().numpy(), oracle.dct1(x)) < tol
 
 
+@pytest.mark.parametrize("n", [1387, 2049, 3001, 8641, 9073, 11665, 15001])
+def test_dct1_f64_error_of_short_rows(K, n):
+    """FP64 DCT-I in passes of up to 176 points (small radices) and just above,
+    white noise, against extended precision.  In rms, relative: the result's
+    rounding at most 2^-53 / sqrt(3), the four-step twiddle's (both parts and its
+    angle, 2^-54 each) at most 2 x 2^-54 / sqrt(3), everything else 2^-57 a stage:
+    below 1e-16; 1.5e-16 allowed."""
+    import scipy.fft
+    x = np.random.default_rng(n).standard_normal((6, n))
+    ref = scipy.fft.dct(x.astype(np.longdouble), type=1, axis=-1)
+    err = (K.DCT1(6, n, torch.float64)(dev(x)).cpu().numpy() - ref).astype(np.float64)
+    assert np.linalg.norm(err) < 1.5e-16 * np.linalg.norm(ref.astype(np.float64))
+
+
 def test_apply_noise_f64_row_without_gap(K):
     """The filter's chained transforms at one of those lengths (1891 = 60 x 63 / 2 + 1)."""
     rng = np.random.default_rng(1891)
