@@ -424,11 +424,11 @@ struct Cfg {
 // run at once.  Beyond one wave the larger CTAs hide latency better (256 x
 // 130,978 FP32: 165 us for 198).  DCT with NT and with half, FP32: 64 x 65,341
 // (384 tiles a pass; 304 CTAs of 512 threads run at once) 29.4 and 24.1 us, 96 x
-// 65,341 34.0 and 29.8, 48 x 130,978 41.6 and 35.6.
+// 65,341 34.0 and 29.8, 48 x 130,978 41.6 and 35.6; FP64 (Bluestein) 53 x 2,340
+// 90.6 and 76.2, 64 x 2,000 107 and 79.
 template <int FB>
 int threads_for(int64_t ntile, size_t smem) {
   constexpr int NT = Cfg<FB>::NT, HALF = NT / 2;
-  if (HALF < 256) return NT;
   const int64_t sms = sm_count(), fit = 227 * 1024 / (int64_t)(smem + 1024);
   const int64_t full = std::min<int64_t>(Cfg<FB>::MINB, fit), half = std::min<int64_t>(2 * Cfg<FB>::MINB, fit);
   return ntile > full * sms && ntile <= half * sms ? HALF : NT;
