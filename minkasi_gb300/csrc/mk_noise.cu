@@ -593,8 +593,8 @@ struct mk_noise_group {
     float *data;
   };
   struct Class {  // the TODs with one detector count
-    int64_t ndet = 0, ntile = 0;
-    int njobs = 0;
+    int64_t ndet = 0, nitem = 0;
+    int njobs = 0, mt = 1;  // mt: tiles per work item
     mk::RotJob *jobs_v = nullptr, *jobs_vT = nullptr;  // device tables
   };
   std::vector<Tod> tods;
@@ -662,14 +662,17 @@ extern "C" int mk_noise_group_create(mk_noise_group **group, int ntod, mk_noise_
   for (size_t k = 0; k < nds.size() && !rc; k++) {
     mk_noise_group::Class cl;
     cl.ndet = nds[k];
+    int64_t ntile = 0;
+    for (int t = 0; t < ntod; t++)
+      if (plans[t]->core.nrow == cl.ndet) ntile += mk::rot_tc_tiles(plans[t]->core.n);
+    cl.mt = mk::rot_tc_tiles_per_item(cl.ndet, ntile);
     std::vector<mk::RotJob> jv, jvT;
     for (int t = 0; t < ntod; t++) {
       const DctCore &c = plans[t]->core;
       if (c.nrow != cl.ndet) continue;
-      const int64_t tiles = mk::rot_tc_items(c.nrow, c.n);
-      jv.push_back({data[t], data[t], img_v[t], c.n, c.n, c.n, cl.ntile});
-      jvT.push_back({data[t], data[t], img_vT[t], c.n, c.n, c.n, cl.ntile});
-      cl.ntile += tiles;
+      jv.push_back({data[t], data[t], img_v[t], c.n, c.n, c.n, cl.nitem});
+      jvT.push_back({data[t], data[t], img_vT[t], c.n, c.n, c.n, cl.nitem});
+      cl.nitem += mk::rot_tc_items(c.n, cl.mt);
     }
     cl.njobs = (int)jv.size();
     const size_t tb = align_up((size_t)ntod * sizeof(mk::RotJob));
@@ -700,7 +703,7 @@ extern "C" int mk_noise_group_exec(mk_noise_group *g, void *stream) {
   cudaStream_t st = mk::as_stream(stream);
   int rc;
   for (const auto &cl : g->classes)
-    if ((rc = mk::rot_tc_group(cl.jobs_v, cl.njobs, cl.ntile, cl.ndet, g->err, st))) return rc;
+    if ((rc = mk::rot_tc_group(cl.jobs_v, cl.njobs, cl.nitem, cl.mt, cl.ndet, g->err, st))) return rc;
   for (const auto &t : g->tods) {
     DctCore *c = t.core;
     if (c->own) {
@@ -723,7 +726,7 @@ extern "C" int mk_noise_group_exec(mk_noise_group *g, void *stream) {
     if ((rc = mk::launch_status("noise group/halve"))) return rc;
   }
   for (const auto &cl : g->classes)
-    if ((rc = mk::rot_tc_group(cl.jobs_vT, cl.njobs, cl.ntile, cl.ndet, g->err, st))) return rc;
+    if ((rc = mk::rot_tc_group(cl.jobs_vT, cl.njobs, cl.nitem, cl.mt, cl.ndet, g->err, st))) return rc;
   return MK_OK;
 }
 

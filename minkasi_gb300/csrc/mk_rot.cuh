@@ -22,7 +22,7 @@ int rot_tc_f32(const float *A, const float *X, int64_t ldx, float *R, int64_t ld
                int64_t x_stride = 1, int halve_ends = 0);
 
 // One TOD of a grouped rotation: R = A . X with A given by its operand image
-// bimg (rot_tc_bprep); tile0 = the first of its rot_tc_items(nrow, ncol) work
+// bimg (rot_tc_bprep); tile0 = the first of its rot_tc_items(ncol, mt) work
 // items in the launch (jobs sorted by tile0, contiguous).  R may equal X (in
 // place): the kernel reads all of a tile's inputs before it writes that tile.
 struct RotJob {
@@ -31,9 +31,14 @@ struct RotJob {
   const char *bimg;
   int64_t ldx, ldr, ncol, tile0;
 };
-int64_t rot_tc_items(int64_t nrow, int64_t ncol);
+// tiles of ncol samples, tiles per work item of a launch with ntile of them over
+// all its jobs, and work items of a job
+int64_t rot_tc_tiles(int64_t ncol);
+int rot_tc_tiles_per_item(int64_t nrow, int64_t ntile);
+int64_t rot_tc_items(int64_t ncol, int mt);
 // the operand image of A (rot_tc_bimg_bytes(nrow) bytes)
 int rot_tc_bprep(const float *A, int64_t nrow, void *bimg, cudaStream_t st);
 // every job of the (device) table in one launch; all jobs have nrow detectors
-int rot_tc_group(const RotJob *jobs_dev, int njobs, int64_t nitem, int64_t nrow, int *err, cudaStream_t st);
+// and items of mt tiles
+int rot_tc_group(const RotJob *jobs_dev, int njobs, int64_t nitem, int mt, int64_t nrow, int *err, cudaStream_t st);
 }  // namespace mk

@@ -25,8 +25,10 @@
 // detectors one tile per pass reads three times as much of A's image from L2
 // as of X from memory, which is what bounded the kernel (with the 8 B TF32
 // image: 0.156 ms on 256 x 130,978).  MT = 2 there (one CTA per SM: two
-// accumulators of 256 columns fill tensor memory); MT = 1 below, where two
-// CTAs fit an SM and each has two accumulators.
+// accumulators of 256 columns fill tensor memory) once there are more tiles than
+// SMs; MT = 1 for fewer, which an item of two would put on half as many SMs
+// (256 x 1,000 .. 19,000: 30.9 us with MT = 2, 22.7 with 1), and MT = 1 below 256
+// detectors, where two CTAs fit an SM and each has two accumulators.
 //
 // Roles: MT x 4 split warps; MT x 4 epilogue warps (warp w reads TMEM lanes
 // 32 (w % 4) .. of its tile and stores per detector 32 consecutive samples);
@@ -393,8 +395,6 @@ __global__ void __launch_bounds__((8 * MT + 1) * 32, 3 - MT)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(tcols));
 }
 
-int tiles_per_item(int64_t nrow) { return nrow == 256 ? 2 : 1; }
-
 template <int MT>
 int launch(const mk::RotJob *jobs, int njobs, const mk::RotJob &j0, int64_t nitem, int nd, int *err, cudaStream_t st,
            int64_t mirror_n, int64_t xs, int halve_ends) {
@@ -407,7 +407,7 @@ int launch(const mk::RotJob *jobs, int njobs, const mk::RotJob &j0, int64_t nite
   MK_CUDA(cudaGetDevice(&dev));
   if (dev >= 0 && dev < 64 && !attr[dev]) {
     MK_CUDA(cudaFuncSetAttribute(k_rot_tc<MT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)bytes(MT == 1 ? 128 : 256)));
+                                 (int)bytes(256)));
     attr[dev] = true;
   }
   const int nbuf = MT * nd * 2 <= 512 / (MT == 1 ? 2 : 1) ? 2 : 1;  // accumulators; MT = 1: two CTAs per SM
@@ -419,9 +419,9 @@ int launch(const mk::RotJob *jobs, int njobs, const mk::RotJob &j0, int64_t nite
   return mk::launch_status("rot_tc");
 }
 
-int launch_nd(const mk::RotJob *jobs, int njobs, const mk::RotJob &j0, int64_t nitem, int nd, int *err,
+int launch_mt(int mt, const mk::RotJob *jobs, int njobs, const mk::RotJob &j0, int64_t nitem, int nd, int *err,
               cudaStream_t st, int64_t mirror_n, int64_t xs, int halve_ends) {
-  if (tiles_per_item(nd) == 2) return launch<2>(jobs, njobs, j0, nitem, nd, err, st, mirror_n, xs, halve_ends);
+  if (mt == 2) return launch<2>(jobs, njobs, j0, nitem, nd, err, st, mirror_n, xs, halve_ends);
   return launch<1>(jobs, njobs, j0, nitem, nd, err, st, mirror_n, xs, halve_ends);
 }
 
@@ -435,10 +435,11 @@ bool rot_tc_supported(int64_t nrow) {
 
 size_t rot_tc_bimg_bytes(int64_t nrow) { return (size_t)nrow * (size_t)nrow * 6; }
 
-int64_t rot_tc_items(int64_t nrow, int64_t ncol) {
-  const int64_t per = (int64_t)TILE_M * tiles_per_item(nrow);
-  return (ncol + per - 1) / per;
-}
+int64_t rot_tc_tiles(int64_t ncol) { return (ncol + TILE_M - 1) / TILE_M; }
+
+int rot_tc_tiles_per_item(int64_t nrow, int64_t ntile) { return nrow == 256 && ntile > sm_count() ? 2 : 1; }
+
+int64_t rot_tc_items(int64_t ncol, int mt) { return (rot_tc_tiles(ncol) + mt - 1) / mt; }
 
 int rot_tc_f32(const float *A, const float *X, int64_t ldx, float *R, int64_t ldr, int64_t nrow,
                int64_t ncol, void *bimg, int *err, cudaStream_t st, int64_t mirror_n, int64_t x_stride,
@@ -451,7 +452,8 @@ int rot_tc_f32(const float *A, const float *X, int64_t ldx, float *R, int64_t ld
   const int rc = rot_tc_bprep(A, nrow, bimg, st);
   if (rc) return rc;
   const RotJob j0{X, R, (const char *)bimg, ldx, ldr, ncol, 0};
-  return launch_nd(nullptr, 1, j0, rot_tc_items(nrow, ncol), (int)nrow, err, st, mirror_n, x_stride, halve_ends);
+  const int mt = rot_tc_tiles_per_item(nrow, rot_tc_tiles(ncol));
+  return launch_mt(mt, nullptr, 1, j0, rot_tc_items(ncol, mt), (int)nrow, err, st, mirror_n, x_stride, halve_ends);
 }
 
 int rot_tc_bprep(const float *A, int64_t nrow, void *bimg, cudaStream_t st) {
@@ -463,12 +465,12 @@ int rot_tc_bprep(const float *A, int64_t nrow, void *bimg, cudaStream_t st) {
   return launch_status("rot_tc_bprep");
 }
 
-int rot_tc_group(const RotJob *jobs_dev, int njobs, int64_t nitem, int64_t nrow, int *err, cudaStream_t st) {
+int rot_tc_group(const RotJob *jobs_dev, int njobs, int64_t nitem, int mt, int64_t nrow, int *err, cudaStream_t st) {
   MK_CHECK_ARG(rot_tc_supported(nrow), "tensor-core rotation supports ndet in {32,64,128,256}, got %lld",
                (long long)nrow);
   MK_CHECK_ARG(jobs_dev && njobs >= 1 && err, "tensor-core rotation group: bad arguments");
   if (nitem <= 0) return MK_OK;
-  return launch_nd(jobs_dev, njobs, RotJob{}, nitem, (int)nrow, err, st, 0, 1, 0);
+  return launch_mt(mt, jobs_dev, njobs, RotJob{}, nitem, (int)nrow, err, st, 0, 1, 0);
 }
 
 }  // namespace mk

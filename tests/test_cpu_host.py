@@ -273,9 +273,10 @@ def test_rotation_launch_limits_of_two_threads(tmp_path, first, second):
     subprocess.run(["g++", "-shared", "-o", "rot.so", *objs, "fake.o", "-Wl,-Bsymbolic", "-lpthread"], cwd=tmp_path,
                    check=True)
     h = ctypes.CDLL(str(tmp_path / "rot.so"))
-    group = h._ZN2mk12rot_tc_groupEPKNS_6RotJobEillPiP11CUstream_st
-    group.argtypes = [ctypes.c_void_p, ctypes.c_int, ctypes.c_int64, ctypes.c_int64, ctypes.c_void_p, ctypes.c_void_p]
-    run = lambda nd: group(1, 1, 1, nd, 1, None)  # (nothing runs: the pointers are not read)
+    group = h._ZN2mk12rot_tc_groupEPKNS_6RotJobEililPiP11CUstream_st
+    group.argtypes = [ctypes.c_void_p, ctypes.c_int, ctypes.c_int64, ctypes.c_int, ctypes.c_int64, ctypes.c_void_p,
+                      ctypes.c_void_p]
+    run = lambda nd, mt=1: group(1, 1, 1, mt, nd, 1, None)  # (nothing runs: the pointers are not read)
     rc = []
     t = threading.Thread(target=lambda: rc.append(run(first)))
     t.start()
@@ -289,7 +290,7 @@ def test_rotation_launch_limits_of_two_threads(tmp_path, first, second):
     ctypes.c_int.in_dll(h, "release").value = 1
     t.join()
     assert rc == [0, 0]
-    assert [run(nd) for nd in (32, 64, 128, 256)] == [0] * 4
+    assert [run(nd) for nd in (32, 64, 128, 256)] + [run(256, 2)] == [0] * 5
 
 
 def test_tod2map_choices_of_earlier_kernels_are_not_taken(tmp_path, monkeypatch):

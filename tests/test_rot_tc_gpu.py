@@ -62,6 +62,37 @@ def test_tc_rotation_tile_edges_and_nonfinite(K, ndet, ncol):
     assert plan.status() == 0
 
 
+@pytest.mark.parametrize("ncol", [19_456, 19_457, 19_584, 19_585])
+def test_tc_rotation_around_one_tile_per_sm(K, ncol):
+    """256 detectors: 152 tiles of 128 samples (one tile per item on 152 SMs), a
+    ragged 153rd, 153 and a ragged 154th (two tiles per item, the last one half
+    empty or ragged), at the bound of test_tc_rotation_tile_edges_and_nonfinite."""
+    rng = np.random.default_rng(ncol)
+    A = rng.standard_normal((256, 256)).astype(np.float32)
+    X = rng.standard_normal((256, ncol)).astype(np.float32)
+    ref = A.astype(np.float64) @ X.astype(np.float64)
+    plan = K.NoisePlan(256, ncol, torch.float32)
+    R = plan.rotate(torch.from_numpy(A).to(cuda), torch.from_numpy(X).to(cuda), rot_mode=2).cpu().numpy()
+    assert (np.abs(R - ref).max(0) <= 2.3e-5 * np.abs(ref).max(0)).all()
+    assert plan.status() == 0
+
+
+def test_noise_group_of_more_tiles_than_its_tods(K):
+    """Three 256-detector TODs of one tile per item each, two as a group: as
+    each TOD's own filter gives, bit for bit."""
+    g = torch.Generator(device="cuda").manual_seed(4)
+    r = lambda *s: torch.randn(s, generator=g, device=cuda)
+    ns = [9001, 300, 12_001]
+    plans = [K.NoisePlan(256, n, torch.float32) for n in ns]
+    ops = [(r(256, 256), r(256, 256), r(256, n).abs()) for n in ns]
+    data = [r(256, n) for n in ns]
+    want = [p.apply(*o, d, rot_mode=2) for p, o, d in zip(plans, ops, data)]
+    grp = K.NoiseGroup(plans, ops, data)
+    grp.apply()
+    assert grp.status() == 0
+    assert all(torch.equal(a, b) for a, b in zip(data, want))
+
+
 def test_tc_apply_noise_matches_golden(K, gold):
     g = gold("noise.npz")
     x = g["x"]
