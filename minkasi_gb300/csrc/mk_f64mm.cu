@@ -63,11 +63,21 @@ int rot_launch(const double *A, const double *X, int64_t ldx, double *R, int64_t
 int rot_f64(const double *A, const double *X, int64_t ldx, double *R, int64_t ldr, int64_t nrow, int64_t ncol,
             cudaStream_t st) {
   if (ncol <= 0) return MK_OK;
-  // detectors per thread: 8, or fewer where that pads less
+  // detectors per thread: 8, or fewer where that pads less, or where it leaves the
+  // SM with the most CTAs at least a tenth less to do (a few CTAs per SM and a
+  // nearly empty last wave; a quarter of a multiply-add more for a thread's loads).
+  // 96 x 1,000 with 8 and 6: 37.8 and 30.1 us, 128 x 1,000 with 8 and 7: 48.5 and
+  // 45.7 (DGEMM 35.7 and 44.8), 300 x 1,000 with 6 and 8: 176 and 159; for less than
+  // a tenth 200 x 3,000 lost (8 and 7: 213 and 223).
   const int nd = (int)nrow;
+  const int64_t cols = (ncol + RT - 1) / RT, sms = sm_count();
+  const auto cost = [&](int c) { return (cols * ((nd + c - 1) / c) + sms - 1) / sms * (4 * c + 1); };
   int ob = 8;
   for (int c = 7; c >= 5; c--)
     if ((nd + c - 1) / c * c < (nd + ob - 1) / ob * ob) ob = c;
+  const int64_t enough = cost(ob) * 9 / 10;
+  for (int c = 8, base = ob; c >= 5; c--)
+    if (cost(c) <= enough && (ob == base || cost(c) < cost(ob))) ob = c;
   switch (ob) {
     case 5: return rot_launch<5>(A, X, ldx, R, ldr, nd, ncol, st);
     case 6: return rot_launch<6>(A, X, ldx, R, ldr, nd, ncol, st);

@@ -593,6 +593,13 @@ def test_f64_rotation(K, nd, n):
     assert (np.abs(got - Al @ Xl) <= nd * 2.0 ** -53 * (np.abs(A) @ np.abs(X))).all()
 
 
+@pytest.mark.parametrize("nd,n", [(32, 1000), (33, 960), (96, 1001), (128, 1023), (300, 1000)])
+def test_f64_rotation_of_few_blocks(K, nd, n):
+    """The FP64-pipe rotation where the block heights follow the number of SMs
+    (5 to 8 detectors, the last block ragged), at the bound of test_f64_rotation."""
+    test_f64_rotation(K, nd, n)
+
+
 @pytest.mark.parametrize("nd,n", [(52, 65341), (64, 65341), (96, 65341), (48, 130978), (33, 72140), (62, 28162)])
 def test_dct1_f32_one_wave_of_half_size_blocks(K, nd, n):
     """Row counts whose tiles need more blocks than run at once at full size:
