@@ -491,6 +491,24 @@ def test_noise_plans_sharing_one_workspace(K, dtype):
         assert p_s.status() == 0
 
 
+@pytest.mark.parametrize("mode", [0, 4])
+def test_f64_filters_sharing_one_workspace(K, mode):
+    """FP64 plans on one workspace, used alternately with the sliced rotation
+    (its slices and exponents) and the FP64-pipe one, through fixed-point
+    transforms (their exponents and statistics) and Bluestein's: each gives what
+    it gives on a workspace of its own."""
+    shapes = [(16, 3529), (257, 500), (32, 4097), (9, 1000), (64, 1891)]
+    ws = torch.empty(max(K.noise_workspace_bytes(nd, n) for nd, n in shapes), dtype=torch.uint8, device="cuda")
+    g = torch.Generator(device="cuda").manual_seed(2)
+    r = lambda *s: torch.randn(s, generator=g, dtype=torch.float64, device=cuda)
+    cases = [(r(nd, nd), r(nd, nd), r(nd, n).abs(), r(nd, n)) for nd, n in shapes]
+    alone = [K.NoisePlan(nd, n).apply(*c, rot_mode=mode) for (nd, n), c in zip(shapes, cases)]
+    shared = [K.NoisePlan(nd, n, workspace=ws) for nd, n in shapes]
+    for _ in range(2):
+        for p, c, want in zip(shared, cases, alone):
+            assert torch.equal(p.apply(*c, rot_mode=mode), want)
+
+
 def test_apply_noise_golden_f64(K, gold):
     g = gold("noise.npz")
     v, vT, w = dev(g["v"]), dev(g["vT"]), dev(g["mywt"])
