@@ -371,10 +371,10 @@ int mk_rotate(mk_noise_plan *plan, const void *A, const void *X, void *R, int ro
               void *stream);
 
 /* Device status of the plan's tensor-core kernels: *code = 1 if one of
- * their bounded waits timed out since the last call, else 0.  The kernel
- * then stops, frees its tensor memory and fills what it had to write with
- * NaN, and so does every later tensor-core rotation of the plan until this
- * call has reported it.  Reads and clears the word; synchronises `stream`. */
+ * their bounded waits timed out since the last call, else 0.  The kernel's
+ * block then stops, frees its tensor memory and fills what it had to write
+ * with NaN (so that the filtered timestream, which mixes all of them, is NaN
+ * too).  Reads and clears the word; synchronises `stream`. */
 int mk_noise_status(mk_noise_plan *plan, int *code, void *stream);
 
 /* NoiseSmoothedSVD.apply_noise of many TODs in one call, in place on each

@@ -8,6 +8,13 @@ namespace mk {
 // iterations of mbarrier.try_wait (each may suspend briefly) before a wait
 // is declared timed out
 constexpr uint32_t SPIN_LIMIT = 1u << 24;
+// the same for the waits between the roles of a tensor-core kernel, after which
+// its CTA stops and writes NaN (a compile-time constant: as a kernel argument it
+// cost the sliced FP64 rotation 2 %)
+#ifndef MK_ROLE_SPIN_LIMIT
+#define MK_ROLE_SPIN_LIMIT SPIN_LIMIT
+#endif
+constexpr uint32_t ROLE_SPIN_LIMIT = MK_ROLE_SPIN_LIMIT;
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) {
   return (uint32_t)__cvta_generic_to_shared(p);

@@ -302,7 +302,7 @@ __device__ __forceinline__ void tmem_wait(uint32_t (&r)[N][8]) {
 
 // bounded wait that also polls the CTA's abort flag (set on a timeout)
 __device__ __forceinline__ bool oz_wait(uint64_t *bar, uint32_t parity, volatile int *abort_flag) {
-  for (uint32_t i = 0; i < SPIN_LIMIT; i++) {
+  for (uint32_t i = 0; i < ROLE_SPIN_LIMIT; i++) {
     if (mbar_try_wait(bar, parity)) return true;
     if ((i & 31u) == 31u && *abort_flag) return false;
   }
@@ -382,6 +382,17 @@ __device__ __forceinline__ double combine(long long hi, long long lo, int e) {
   return __hiloint2double((int)rh, (int)rl);
 }
 
+// NaN where this CTA writes R (not inlined: the kernel around it keeps its code
+// and its time; inlined, 256 x 130,978 took 643 us for 628)
+__device__ __noinline__ void fill_nan(double *R, int64_t ldr, int nrow, int ndb, int nitem, int64_t j0, int64_t ncol) {
+  for (int i = blockIdx.x; i < nitem; i += gridDim.x)
+    for (int e = threadIdx.x; e < OZ_M * OZ_ND; e += OZ_THREADS) {
+      const int64_t j = j0 + (int64_t)(i / ndb) * OZ_M + e % OZ_M;
+      const int d = (i % ndb) * OZ_ND + e / OZ_M;
+      if (j < ncol && d < nrow) R[(int64_t)d * ldr + j] = __longlong_as_double(0x7FF8000000000000ll);
+    }
+}
+
 // R for ntile tiles of OZ_M samples (the first at column j0) and ndb blocks of
 // OZ_ND detectors; item i = (tile i / ndb, block i % ndb), so the CTAs that
 // run together share X chunks in L2
@@ -422,7 +433,6 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
   asm volatile("tcgen05.fence::after_thread_sync;");
   const uint32_t tmem = tmem_base_sh;
   const int ndrain = (nkc + OZ_DRAIN - 1) / OZ_DRAIN;
-  const int prior = tid == 0 ? *(volatile const int *)err : 0;  // an earlier timeout, not yet reported
   uint32_t issued = 0, g_mma = 0;  // chunks whose copies were issued / whose MMAs were committed
 
   if (warp == EPI_WARPS) {
@@ -535,8 +545,9 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
       }
     }
   }
-  const bool failed = __syncthreads_or(prior | *abort_flag);
-  if (*abort_flag) {
+  __syncthreads();
+  const bool failed = *abort_flag;
+  if (failed) {
     // after a timeout: bounded waits for the copies and MMAs still in flight
     if (tid == EPI_WARPS * 32)
       for (uint32_t g = issued > XSTG ? issued - XSTG : 0; g < issued; g++) {
@@ -548,13 +559,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
         (void)mbar_wait(&done[g % XSTG], (g / XSTG) & 1);
     }
   }
-  if (failed)  // no caller takes this CTA's part for a result
-    for (int i = blockIdx.x; i < nitem; i += gridDim.x)
-      for (int e = tid; e < OZ_M * OZ_ND; e += OZ_THREADS) {
-        const int64_t j = j0 + (int64_t)(i / ndb) * OZ_M + e % OZ_M;
-        const int d = (i % ndb) * OZ_ND + e / OZ_M;
-        if (j < ncol && d < nrow) R[(int64_t)d * ldr + j] = __longlong_as_double(0x7FF8000000000000ll);
-      }
+  if (failed) fill_nan(R, ldr, nrow, ndb, nitem, j0, ncol);  // no caller takes this CTA's part for a result
   asm volatile("tcgen05.fence::before_thread_sync;");
   __syncthreads();
   if (warp == 0)

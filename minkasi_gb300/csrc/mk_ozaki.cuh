@@ -13,8 +13,8 @@ bool ozaki_supported(int64_t nrow);
 // blocks, so it does not grow with ncol)
 size_t ozaki_ws_bytes(int64_t nrow);
 // stream-ordered on st; R must not overlap X.  `err` is a device int set to 1
-// if a bounded wait inside the kernel timed out; R becomes NaN where that
-// happened, and everywhere while the word stays set.
+// if a bounded wait inside the kernel timed out; what the kernel's block had to
+// write is NaN then.
 int ozaki_rotate_f64(const double *A, const double *X, int64_t ldx, double *R, int64_t ldr, int64_t nrow,
                      int64_t ncol, void *ws, size_t ws_bytes, int *err, cudaStream_t st);
 }  // namespace mk

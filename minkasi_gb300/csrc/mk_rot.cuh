@@ -12,7 +12,8 @@ namespace mk {
 bool rot_tc_supported(int64_t nrow);
 // bytes of the operand image the kernel stages A from (16-byte aligned buffer)
 size_t rot_tc_bimg_bytes(int64_t nrow);
-// `err` is a device int set to 1 if a bounded wait inside the kernel timed out.
+// `err` is a device int set to 1 if a bounded wait inside the kernel timed out;
+// what the kernel's block had to write is NaN then.
 // mirror_n > 0 (= 2(ncol-1), with ldr >= mirror_n) also writes the even
 // extension R[., mirror_n - j] = R[., j], 1 <= j <= ncol-2, for a DCT-I.
 // x_stride 2 reads X[r][j] at X + r*ldx + 2j (the real parts of an

@@ -153,7 +153,7 @@ __global__ void k_bprep(const float *__restrict__ A, int ndet, char *__restrict_
 }
 
 __device__ __forceinline__ bool ws_wait(uint64_t *bar, uint32_t parity, volatile int *abort_flag) {
-  for (uint32_t i = 0; i < mk::SPIN_LIMIT; i++) {
+  for (uint32_t i = 0; i < mk::ROLE_SPIN_LIMIT; i++) {
     if (mk::mbar_try_wait(bar, parity)) return true;
     if ((i & 31u) == 31u && *abort_flag) return false;
   }
@@ -177,6 +177,25 @@ __device__ __forceinline__ int job_at(const mk::RotJob *jobs, int njobs, int64_t
 
 // plain (R may be X) streaming load; zero past the TOD's end
 __device__ __forceinline__ float load1(const float *p, bool ok) { return ok ? __ldcs(p) : 0.f; }
+
+// NaN where this CTA writes its jobs' R (not inlined: the kernel around it keeps
+// its code)
+template <int MT>
+__device__ __noinline__ void fill_nan(const mk::RotJob *jobs, int njobs, int64_t nitem, int ndet, int64_t mirror_n) {
+  const float nan = __int_as_float(0x7FC00000);
+  int cur = 0;
+  for (int64_t item = blockIdx.x; item < nitem; item += gridDim.x) {
+    cur = job_at(jobs, njobs, item, cur);
+    const mk::RotJob &J = jobs[cur];
+    for (int e = threadIdx.x; e < MT * TILE_M * ndet; e += (int)blockDim.x) {
+      const int64_t my = (item - J.tile0) * MT * TILE_M + e % (MT * TILE_M);
+      float *row = J.R + (int64_t)(e / (MT * TILE_M)) * J.ldr;
+      if (my >= J.ncol) continue;
+      row[my] = nan;
+      if (mirror_n > 0 && my >= 1 && my <= J.ncol - 2) row[mirror_n - my] = nan;
+    }
+  }
+}
 
 // One item = MT tiles of 128 samples of one job (RotJob::tile0 counts items).
 // `jobs` (device memory, sorted by tile0) lists the TODs of a grouped launch,
@@ -223,7 +242,6 @@ __global__ void __launch_bounds__((8 * MT + 1) * 32, 3 - MT)
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;");
   const uint32_t tmem = tmem_base_sh;
-  const int prior = tid == 0 ? *(volatile const int *)err : 0;  // an earlier timeout, not yet reported
   uint32_t g_copied = 0, g_issued = 0;  // MMA thread: chunks whose image copy / MMAs were issued
 
   if (warp < NSPLIT) {
@@ -365,8 +383,9 @@ __global__ void __launch_bounds__((8 * MT + 1) * 32, 3 - MT)
       mk::mbar_arrive(&acc_empty[ab]);
     }
   }
-  const bool failed = __syncthreads_or(prior | *abort_flag);
-  if (*abort_flag && tid == (NSPLIT + NEPI) * 32) {
+  __syncthreads();
+  const bool failed = *abort_flag;
+  if (failed && tid == (NSPLIT + NEPI) * 32) {
     atomicExch(err, 1);
     // bounded waits for the copies and MMAs this thread issued
     for (uint32_t g = (g_copied > NSTAGE ? g_copied - NSTAGE : 0); g < g_copied; g++)
@@ -374,21 +393,7 @@ __global__ void __launch_bounds__((8 * MT + 1) * 32, 3 - MT)
     for (uint32_t g = (g_issued > NSTAGE ? g_issued - NSTAGE : 0); g < g_issued; g++)
       (void)mbar_wait(&mma_done[g % NSTAGE], (g / NSTAGE) & 1);
   }
-  if (failed) {  // no caller takes this CTA's part for a result
-    int cur = 0;
-    for (int64_t item = blockIdx.x; item < nitem; item += gridDim.x) {
-      cur = job_at(jobs, njobs, item, cur);
-      const mk::RotJob &J = jobs[cur];
-      for (int e = tid; e < MT * TILE_M * ndet; e += (int)blockDim.x) {
-        const int64_t my = (item - J.tile0) * MT * TILE_M + e % (MT * TILE_M);
-        float *row = J.R + (int64_t)(e / (MT * TILE_M)) * J.ldr;
-        if (my < J.ncol) {
-          row[my] = __int_as_float(0x7FC00000);
-          if (mirror_n > 0 && my >= 1 && my <= J.ncol - 2) row[mirror_n - my] = __int_as_float(0x7FC00000);
-        }
-      }
-    }
-  }
+  if (failed) fill_nan<MT>(jobs, njobs, nitem, ndet, mirror_n);  // no caller takes this CTA's part for a result
   asm volatile("tcgen05.fence::before_thread_sync;");
   __syncthreads();
   if (warp == 0)

@@ -185,7 +185,7 @@ class MapmakingOperator:
 
     def timed_out(self) -> bool:
         """True if a kernel of this operator stopped on a timed-out wait since
-        the last call: a rotation (its outputs are NaN) or the staged tod2map
+        the last call: a rotation (its outputs hold NaN) or the staged tod2map
         (its update of the map is incomplete).  Synchronises."""
         if self._group:
             bad = self._group.status() != 0

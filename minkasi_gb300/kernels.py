@@ -508,7 +508,7 @@ class NoisePlan:
 
     def status(self) -> int:
         """1 if a tensor-core kernel of this plan timed out since the last call
-        (what it and the plan's later ones had to write is NaN then)."""
+        (its outputs hold NaN then)."""
         code = ctypes.c_int(0)
         check(lib().mk_noise_status(self._h, ctypes.byref(code), _stream()), "noise_status")
         return int(code.value)
@@ -574,7 +574,7 @@ class NoiseGroup:
 
     def status(self) -> int:
         """1 if a tensor-core wait of the group timed out since the last call
-        (what it and the group's later ones had to write is NaN then)."""
+        (the timestreams hold NaN then)."""
         code = ctypes.c_int(0)
         check(lib().mk_noise_group_status(self._h, ctypes.byref(code), _stream()), "noise group status")
         return int(code.value)

@@ -143,43 +143,46 @@ def test_noise_group_equals_per_tod_filter(monkeypatch, dct):
     assert torch.equal(grouped, op.tmp)
 
 
-@pytest.mark.parametrize("set_word", [0, 1])
-def test_rotations_are_nan_after_an_unreported_timeout(K, set_word):
-    """The kernels' error word, as a timed-out wait leaves it: while it is set
-    every rotation is NaN throughout (FP64 in slices, FP32 with the mirrored
-    extension), and the word stays for the status call; unset, the results
-    are the plan's own bit for bit."""
+def test_rotations_that_time_out_are_nan(K, tmp_path):
+    """The rotations built with a limit of no tries on every wait between their
+    roles, so that each block stops at its first one: the error word is set and
+    every output is NaN (FP64 in slices; FP32 with the mirrored extension, one
+    tile and two per item); nothing is left in flight: the library's own
+    kernels run on afterwards."""
     import ctypes
-    h = K.lib()
+    import os
+    import subprocess
+    from minkasi_gb300 import build
+    objs = []
+    for f in ("mk_ozaki", "mk_rot_tc", "mk_common"):
+        objs.append((f, subprocess.Popen(
+            [build._nvcc(), "-O1", "-std=c++17", "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr", *build.ARCH,
+             "-DMK_ROLE_SPIN_LIMIT=0", "-c", os.path.join(build.CSRC, f + ".cu"), "-o", f + ".o"], cwd=tmp_path)))
+    assert all(p.wait() == 0 for _, p in objs)
+    subprocess.run([build._nvcc(), "-shared", *build.ARCH, "-o", "quick.so", *[f + ".o" for f, _ in objs]],
+                   cwd=tmp_path, check=True)
+    h = ctypes.CDLL(str(tmp_path / "quick.so"))
     g = torch.Generator(device="cuda").manual_seed(1)
     vp, i64 = ctypes.c_void_p, ctypes.c_int64
-    err = torch.tensor([set_word], dtype=torch.int32, device=cuda)
-
-    nd, n = 40, 3001  # two detector blocks, a ragged last tile
-    A = torch.randn((nd, nd), generator=g, dtype=torch.float64, device=cuda)
-    X = torch.randn((nd, n), generator=g, dtype=torch.float64, device=cuda)
-    R = torch.zeros((nd, n), dtype=torch.float64, device=cuda)
-    plan = K.NoisePlan(nd, n, torch.float64)
-    want = plan.rotate(A, X, rot_mode=4)
+    ws = torch.empty(128 << 20, dtype=torch.uint8, device=cuda)
     rot64 = h._ZN2mk16ozaki_rotate_f64EPKdS1_lPdlllPvmPiP11CUstream_st
     rot64.argtypes = [vp, vp, i64, vp, i64, i64, i64, vp, ctypes.c_size_t, vp, vp]
-    ws = torch.empty(128 << 20, dtype=torch.uint8, device=cuda)
-    assert rot64(A.data_ptr(), X.data_ptr(), n, R.data_ptr(), n, nd, n, ws.data_ptr(), ws.numel(), err.data_ptr(),
-                 K._stream()) == 0
-    assert R.isnan().all() if set_word else torch.equal(R, want)
-
-    nd = 256
-    A, X = (torch.randn(s, generator=g, device=cuda) for s in ((nd, nd), (nd, n)))
-    plan = K.NoisePlan(nd, n, torch.float32)
-    want = plan.rotate(A, X, rot_mode=2)
-    want = torch.cat([want, want[:, 1:-1].flip(1)], dim=1)
-    R = torch.zeros((nd, 2 * (n - 1)), device=cuda)
     rot32 = h._ZN2mk10rot_tc_f32EPKfS1_lPflllPvPiP11CUstream_stlli
     rot32.argtypes = [vp, vp, i64, vp, i64, i64, i64, vp, vp, vp, i64, i64, ctypes.c_int]
-    assert rot32(A.data_ptr(), X.data_ptr(), n, R.data_ptr(), 2 * (n - 1), nd, n, ws.data_ptr(), err.data_ptr(),
-                 K._stream(), 2 * (n - 1), 1, 0) == 0
-    assert R.isnan().all() if set_word else torch.equal(R, want)
-    assert err.item() == set_word
+    # 40: two detector blocks; 3001: a ragged last tile; 256 x 20,001: two tiles per item
+    for nd, n, dt in ((40, 3001, torch.float64), (64, 3001, torch.float32), (256, 20_001, torch.float32)):
+        err = torch.zeros(1, dtype=torch.int32, device=cuda)
+        A, X = (torch.randn(s, generator=g, dtype=dt, device=cuda) for s in ((nd, nd), (nd, n)))
+        N = n if dt == torch.float64 else 2 * (n - 1)
+        R = torch.zeros((nd, N), dtype=dt, device=cuda)
+        args = [A.data_ptr(), X.data_ptr(), n, R.data_ptr(), N, nd, n, ws.data_ptr()]
+        if dt == torch.float64:
+            assert rot64(*args, ws.numel(), err.data_ptr(), K._stream()) == 0
+        else:
+            assert rot32(*args, err.data_ptr(), K._stream(), N, 1, 0) == 0
+        assert err.item() == 1 and R.isnan().all()
+        plan = K.NoisePlan(nd, n, dt)
+        assert plan.rotate(A, X, rot_mode=4 if dt == torch.float64 else 2).isfinite().all() and plan.status() == 0
 
 
 def test_solvers_raise_on_a_reported_timeout(K, monkeypatch):
