@@ -412,9 +412,10 @@ int blas_rotate(int dtype, const void *A, const void *X, int64_t ldx, void *R, i
 }
 
 // mode 0 (automatic): FP32 cuBLAS, FP64 this library's kernel on the FP64 pipe
-// (FP64 arithmetic throughout, as DGEMM; faster at every size tried, 2 to 300
-// detectors: see mk_f64mm.cu); the host autotuner picks another mode per workload
-// after checking its accuracy against cuBLAS.
+// (FP64 arithmetic throughout, as DGEMM, and faster at 2 to 1,000 detectors of
+// 1,000 to 65,341 samples but for 128 x 1,000, 46 us for 45: see mk_f64mm.cu);
+// the host autotuner picks another mode per workload after checking its accuracy
+// against cuBLAS.
 // mirror_n: see rot_tc_f32 (only the tensor-core kernel fuses the extension;
 // the caller runs k_mirror otherwise).
 int rotate(DctCore *c, int mode, const void *A, const void *X, int64_t ldx, void *R, int64_t ldr,
@@ -574,8 +575,8 @@ extern "C" int mk_noise_status(mk_noise_plan *plan, int *code, void *stream) {
   if (!plan->core.tc_err) return MK_OK;
   cudaStream_t st = mk::as_stream(stream);
   MK_CUDA(cudaMemcpyAsync(code, plan->core.tc_err, sizeof(int), cudaMemcpyDeviceToHost, st));
-  MK_CUDA(cudaMemsetAsync(plan->core.tc_err, 0, sizeof(int), st));
   MK_CUDA(cudaStreamSynchronize(st));
+  if (*code) MK_CUDA(cudaMemsetAsync(plan->core.tc_err, 0, sizeof(int), st));
   return MK_OK;
 }
 
@@ -734,8 +735,8 @@ extern "C" int mk_noise_group_status(mk_noise_group *g, int *code, void *stream)
   MK_CHECK_ARG(g && code, "mk_noise_group_status: null pointer");
   cudaStream_t st = mk::as_stream(stream);
   MK_CUDA(cudaMemcpyAsync(code, g->err, sizeof(int), cudaMemcpyDeviceToHost, st));
-  MK_CUDA(cudaMemsetAsync(g->err, 0, sizeof(int), st));
   MK_CUDA(cudaStreamSynchronize(st));
+  if (*code) MK_CUDA(cudaMemsetAsync(g->err, 0, sizeof(int), st));
   return MK_OK;
 }
 
