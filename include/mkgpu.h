@@ -352,7 +352,7 @@ int mk_get_fft4_split(void);
  * power-of-two row / column scaling, their products on the bf16 tensor cores
  * with FP32 accumulation (exact: every sum stays below 2^24), combined in
  * integers and rounded to FP64 once (ndet <= 1040; the plan's workspace holds
- * its scratch, at most 90 MB). */
+ * its scratch, at most 92 MB). */
 typedef struct mk_noise_plan mk_noise_plan;
 int mk_noise_workspace_bytes(int64_t ndet, int64_t ndata, int dtype, size_t *bytes);
 int mk_noise_plan_create(mk_noise_plan **plan, int64_t ndet, int64_t ndata, int dtype,
@@ -384,7 +384,7 @@ int mk_noise_status(mk_noise_plan *plan, int *code, void *stream);
  * and each TOD's two DCT-I run on its plan (plans[t]: FP32, any DCT engine,
  * ndet in {32, 64, 128, 256}).  Same arithmetic as mk_apply_noise with
  * rot_mode 2 on each TOD, bit for bit.  The group keeps the rotation
- * operand images of v and vT (built at creation: 8 ndet^2 bytes each) and
+ * operand images of v and vT (built at creation: 6 ndet^2 bytes each) and
  * the device job tables; the data pointers, v, vT and mywt must stay valid
  * and unchanged while it is used.  Plans that share a workspace must have
  * their calls ordered on one stream.  mk_noise_group_status reports (and

@@ -15,7 +15,7 @@
 // form, FP64) or read from a cos/sin pair computed once per TOD by
 // mk_pol_sincos (the pointing is fixed across PCG iterations, so this trades
 // 8 more bytes per sample for no FP64 transcendental work on GB300's narrow
-// FP64 pipe).  tod2map sums runs of equal pixels over windows of 128 samples
+// FP64 pipe).  tod2map sums runs of equal pixels over windows of 256 samples
 // per warp and issues one atomic per Stokes component per run.
 #include <math.h>
 

@@ -2,8 +2,11 @@
 // FP32 out: the apply_noise rotations np.dot(v, dat), np.dot(vT, .) of
 // minkasi/mapmaking/noise.py:704,709.
 //
-// Split: every FP32 value is the exact sum of three bf16 values, x = h + m + l
-// (8 significant bits each, every part rounded to nearest), and
+// Split: an FP32 value is the exact sum of three bf16 values, x = h + m + l (8
+// significant bits each, every part rounded to nearest) for 2^-110 <= |x| <
+// 2^128 (1 - 2^-9); below, the low part loses bits to bf16's smallest denormal
+// (2^-133: an absolute error of at most 2^-134), above, h rounds to infinity and
+// the sample becomes NaN.  Then
 //   R ~= h h + h m + m h + m m + h l + l h   (tcgen05.mma kind::f16, FP32
 // accumulation in tensor memory); the dropped products are below 2^-25
 // relative.  (Two TF32 parts need 8 B per value where three bf16 parts need

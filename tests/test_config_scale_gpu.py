@@ -11,7 +11,7 @@ minkasi/mapmaking/tod2map.py:343-400):
 
 TodVec.dot, make_rhs and make_hits run through the public API in FP64 and
 are held to 1e-12 relative (max error over max value; hits exactly).  The
-FP32 operator (FP32 projections and DCT-I, 3xTF32 tensor-core or FP32 cuBLAS
+FP32 operator (FP32 projections and DCT-I, tensor-core or FP32 cuBLAS
 rotation) is held to 1e-5 relative L2 against the FP64 oracle, with each
 FP32 DCT engine (four-step FFT with Bluestein, cuFFT).  GPU only."""
 import os

@@ -1,7 +1,7 @@
-"""The tcgen05 3xTF32 tensor-core rotation against an FP64 reference product
+"""The tcgen05 tensor-core rotation (three bf16 parts per value) against an FP64 reference product
 and against the cuBLAS FP32 rotation, alone and inside apply_noise.  GPU only.
 
-Tolerance: 3xTF32 keeps FP32-level accuracy; max |R - R64| / max |R64| <= 5e-6.
+Tolerance: the split keeps FP32-level accuracy; max |R - R64| / max |R64| <= 5e-6.
 """
 import numpy as np
 import pytest
