@@ -19,9 +19,9 @@
 // value where FP64 rounds at 2^-53 of each value.  Both spread over all
 // outputs in the stages that follow; relative error (2-norm) of a DCT-I of
 // 130,978 points against extended precision, FP64 passes in brackets: white
-// noise 1.3e-16 (7.0e-16), 1/f noise 1.3e-16 (5.7e-16), noise on an offset of
+// noise 7.4e-17 (7.0e-16), 1/f noise 1.0e-16 (5.7e-16), noise on an offset of
 // 1e4 1.2e-16 (3.5e-16; its upper spectrum 1.3e-12, 3.6e-12), one sample 1e6
-// times the others 4.5e-16 (6.9e-16), a 1/f power spectrum 7.6e-16 (7.9e-16).
+// times the others 4.3e-16 (6.9e-16), a 1/f power spectrum 7.6e-16 (7.9e-16).
 // A pair with a NaN or infinity becomes NaN throughout, as its FP64 transform
 // (which mixes the two rows in every product) does.
 //

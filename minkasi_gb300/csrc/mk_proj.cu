@@ -619,9 +619,8 @@ __device__ __forceinline__ void warp_runs(T *__restrict__ map, const int32_t (&p
   __syncwarp();
 }
 
-// WIDE: ipix and dat 32-byte aligned (else 16).  The L1's tag stage bounds the
-// kernel (91 % busy with 16-byte loads, FP64), so half the load instructions
-// count: 256 x 130,978 FP64 on a 1024^2 map 84.7 -> 79.8 us (5.0 TB/s),
+// WIDE: ipix and dat 32-byte aligned (else 16).  The L1 bounds the kernel
+// (81 % of its active cycles, FP64), so half the load instructions count: 256 x 130,978 FP64 on a 1024^2 map 84.7 -> 79.8 us (5.0 TB/s),
 // 128 x 383,329 on 2048^2 157 -> 142 us, 64 x 65,341 15.2 -> 14.7 us; FP32
 // unchanged (67.0 us).  Two groups of 4 samples a lane (coalesced 16-byte
 // loads, two prefix sums) took 89.8, 142 and 18.8 us.
