@@ -57,6 +57,13 @@ class null_precon:
         return val
 
 
+def _check_ranks(timed_out: bool, device) -> None:
+    """Raises on every rank if ``timed_out`` holds on one (called by all)."""
+    if parallel.allreduce_(torch.tensor([float(timed_out)], device=device)).item():
+        raise RuntimeError("a GPU kernel of the mapmaking operator stopped on a timed-out wait on some rank; "
+                           "the summed results are invalid")
+
+
 class RankSumOp:
     """A rank's operator followed by the sum of the map over ranks: the one
     exchange per operator application of the reference's TodVec.dot
@@ -81,9 +88,7 @@ class RankSumOp:
 
     def check(self) -> None:
         """The operator's check on every rank: all raise if one has to."""
-        if parallel.allreduce_scalar(float(self.op.timed_out()), "max"):
-            raise RuntimeError("a GPU kernel of the mapmaking operator stopped on a timed-out wait on some rank; "
-                               "the summed results are invalid")
+        _check_ranks(self.op.timed_out(), self.op.device)
 
 
 def global_op(op):
@@ -268,8 +273,10 @@ def _run_pcg_generic(b, x0, tods, prior, precon, mask, maxiter, outroot, save_it
             history.append({"iter": i, "zr": zr, "alpha": alpha, "beta": beta})
         if i in save_iters:
             x.maps[save_ind].write(outroot + "_" + str(i) + save_tail)
-    if isinstance(tods, TodVec) and tods._fast(b):
-        global_op(tods.engine(b.maps[0])).check()
+    if isinstance(tods, TodVec):  # (a rank without TODs has no engine, but takes part)
+        op = tods.engine(b.maps[0]) if tods._fast(b) else None
+        if op is not None or parallel.have_mpi():
+            _check_ranks(op is not None and op.timed_out(), "cuda")
     x.niter = maxiter
     return x
 

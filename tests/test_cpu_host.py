@@ -199,7 +199,7 @@ def test_operator_reports_timed_out_kernels(monkeypatch, plan, group, staged, ro
     op = MapmakingOperator.__new__(MapmakingOperator)
     op.plans = {(4, 9): NS(status=lambda: 0), (4, 17): NS(status=lambda: plan)}
     op._group = False if group is None else NS(status=lambda: group)
-    op.rot_mode, op.method = rot_mode, "staged" if staged else "atomic"
+    op.rot_mode, op.method, op.device = rot_mode, "staged" if staged else "atomic", "cpu"
     monkeypatch.setattr(K, "tod2map_status", lambda: staged)
     for o in (op, RankSumOp(op)):
         if bad:

@@ -175,3 +175,36 @@ def test_rank_sum_operator_sums_the_shares():
     assert sorted(own0 + own1) == list(range(40)) and not set(own0) & set(own1)
     assert x0 == x1
     assert res0 < 1e-8
+
+
+def _check_worker(rank, world, port, q, fail_rank):
+    import datetime
+    from types import SimpleNamespace
+    os.environ.update(MASTER_ADDR="127.0.0.1", MASTER_PORT=str(port))
+    torch.distributed.init_process_group("gloo", rank=rank, world_size=world,
+                                         timeout=datetime.timedelta(seconds=20))
+    from minkasi_gb300 import parallel
+    from minkasi_gb300.pcg import RankSumOp
+
+    def scalar(*_):  # as a process group without CPU tensors (NCCL) answers
+        raise RuntimeError("No backend type associated with device type cpu")
+    parallel.allreduce_scalar = scalar
+    out = []
+    try:
+        for bad in (-1, fail_rank):
+            op = RankSumOp(SimpleNamespace(device=torch.device("cpu"), timed_out=lambda: rank == bad))
+            try:
+                op.check()
+                out.append("ok")
+            except RuntimeError as e:
+                out.append("timed-out" if "timed-out" in str(e) else str(e))
+        q.put((rank, out))
+    finally:
+        torch.distributed.destroy_process_group()
+
+
+def test_one_ranks_timed_out_kernel_stops_every_rank():
+    """RankSumOp.check: every rank raises when one rank's operator has a
+    timed-out kernel, none otherwise; the flags are summed as a tensor on the
+    operator's device, so that NCCL groups (no CPU tensors) can."""
+    assert _run(2, fail_rank=1, target=_check_worker) == [(r, ["ok", "timed-out"]) for r in range(2)]
